@@ -138,6 +138,7 @@ _SIGS = {
     "epsr_atogen_last_pair_updates": (I64, []),
     "epsr_atogen_noalloc": (C.c_int, [C.POINTER(Box), I32, F32, F32, P, P, P, P, P, I32, P, P, P, I32, P, P]),
     "epsr_timing_enable": (C.c_int, [I32]),
+    "epsr_check_pair_math": (C.c_int, [I32, C.c_uint32, C.c_uint32, F32, P, P]),
     "epsr_umma_gemm_f32": (C.c_int, [P, I32, P, I32, I32, I32, P, I32, I32, P, P]),
     "epsr_bmc_begin_sweep": (C.c_int, [P, P]),
     "epsr_bmc_propose": (C.c_int, [P, I32, P, P]),

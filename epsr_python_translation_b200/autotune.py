@@ -20,6 +20,8 @@ import os
 
 import torch
 
+from .batch import CELL_MOL
+
 THREADS = (64, 128, 256)
 TILES = (256, 512, 1024, 2048, 4096)
 _CACHE = {}
@@ -63,7 +65,7 @@ def tune(bb, mode="plain", net=None, path=None, hist=True):
             pass
     if key in _CACHE:
         ch = _CACHE[key]
-        bb.c.threads = int(ch["threads"])
+        bb.c.threads = int(ch["threads"]) | CELL_MOL
         if hist:
             bb._hist = None
             bb.hist_tile = int(ch["tile"])
@@ -71,11 +73,11 @@ def tune(bb, mode="plain", net=None, path=None, hist=True):
     st = _state(bb)
     times = {"threads": {}, "tile": {}}
     for t in THREADS:
-        bb.c.threads = t
+        bb.c.threads = t | CELL_MOL
         times["threads"][t] = _time(lambda: bb.sweep(mode, net), reps=2)
         _restore(bb, st)
     best_t = min(times["threads"], key=times["threads"].get)
-    bb.c.threads = best_t
+    bb.c.threads = best_t | CELL_MOL
     best_tile = 1024
     if hist:
         for tl in TILES:

@@ -60,7 +60,10 @@ class Bmc(C.Structure):
                 ("mol_cell", C.c_void_p), ("slot_mol", C.c_void_p), ("slot_new", C.c_void_p),
                 ("slot_off", C.c_void_p), ("slot_centre", C.c_void_p), ("energy", C.c_void_p),
                 ("emol", C.c_void_p), ("counters", C.c_void_p), ("sweep_counter", C.c_void_p),
-                ("status", C.c_void_p)]
+                ("status", C.c_void_p), ("cell_mol", C.c_void_p)]
+
+
+CELL_MOL = 0x10000      # EPSR_BMC_CELL_MOL
 
 
 class BmcHist(C.Structure):
@@ -232,12 +235,15 @@ class BatchBoxes:
         self.counters = z(self.nbox * 4, torch.int64)
         self.sweep_counter = z(1, torch.int64)
         self.status = z(1, torch.int32)
+        self.cell_mol = z(4 * self.nmol, torch.float32)
         c = Bmc()
         c.nbox, c.nmol, c.natom, c.ncell, c.nslot = self.nbox, self.nmol, self.natom, self.ncell, self.nslot
-        c.threads = 256
+        # at least 256 threads a move: the library widens a move's CTA while every move stays resident
+        c.threads = 256 | CELL_MOL
         for k in ("slot_box", "mol_box", "naf", "nato", "fclass", "xa", "ya", "za", "xadd", "yadd", "zadd", "pos",
                   "tab", "xstar", "npairref", "cell_start", "cell_mols", "mol_cell", "slot_mol", "slot_new",
-                  "slot_off", "slot_centre", "energy", "emol", "counters", "sweep_counter", "status"):
+                  "slot_off", "slot_centre", "energy", "emol", "counters", "sweep_counter", "status",
+                  "cell_mol"):
             setattr(c, k, _p(getattr(self, k)))
         c.box = _p(self.box_t)
         self.c = c

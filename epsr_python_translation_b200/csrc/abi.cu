@@ -134,3 +134,33 @@ extern "C" int epsr_timing_read(const char *kernel, double *total_ms, int64_t *l
     *launches = n;
     return EPSR_OK;
 }
+
+// ----------------------------------------------------------------- the pair arithmetic's own check
+namespace epsr {
+// differences between the branch-free forms of common.cuh and the operations they stand for, over
+// the floats of bit patterns lo .. hi - 1
+__global__ void check_pair_math_kernel(int what, uint32_t lo, uint32_t hi, float par, unsigned long long *bad) {
+    unsigned long long n = 0;
+    const float rcp = step_rcp(par, 4000);
+    for (uint64_t i = lo + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < hi; i += (uint64_t)gridDim.x * blockDim.x) {
+        const float x = __uint_as_float((uint32_t)i);
+        if (what == 0) n += __float_as_uint(sqrt_unit(x)) != __float_as_uint(__fsqrt_rn(x));
+        else if (what == 1) n += bin_index(x, par, rcp) != ifix(__fdiv_rn(x, par));
+        else n += __float_as_uint(wrap_sq_small(x)) != __float_as_uint(wrap_sq(x));
+    }
+    if (n) atomicAdd(bad, n);
+}
+}  // namespace epsr
+
+extern "C" int epsr_check_pair_math(int32_t what, uint32_t lo, uint32_t hi, float par, unsigned long long *bad,
+                                    void *stream) {
+    if (what < 0 || what > 2 || hi < lo || !bad) {
+        epsr_set_error("epsr_check_pair_math: bad arguments");
+        return EPSR_ERR_ARG;
+    }
+    cudaStream_t s = (cudaStream_t)stream;
+    EPSR_CUDA(cudaMemsetAsync(bad, 0, sizeof(unsigned long long), s));
+    epsr::check_pair_math_kernel<<<1184, 256, 0, s>>>(what, lo, hi, par, bad);
+    EPSR_CUDA(cudaGetLastError());
+    return EPSR_OK;
+}

@@ -176,6 +176,49 @@ __device__ __forceinline__ float wrap_sq(float x) {
     return __fmul_rn(r, r);
 }
 
+// wrap_sq on the FP32 adder.  Adding and subtracting 1.5 * 2^23 rounds a float of magnitude up
+// to 2^22 to the nearest integer, ties to even, which is rintf there; every caller's argument is a
+// difference of box-fraction coordinates.  The rounding instruction rintf compiles to runs on the
+// conversion unit at an eighth of the adder's rate; two additions do not.
+__device__ __forceinline__ float rint_small(float x) { return __fsub_rn(__fadd_rn(x, 12582912.0f), 12582912.0f); }
+__device__ __forceinline__ float wrap_sq_small(float x) {
+    const float r = __fsub_rn(x, rint_small(x));
+    return __fmul_rn(r, r);
+}
+
+// The squared minimum-image distance of a cubic box, as dist_f forms it before its square root.
+__device__ __forceinline__ float dsq_cubic(float4 a, float4 b) {
+    return __fadd_rn(__fadd_rn(wrap_sq_small(__fsub_rn(b.x, a.x)), wrap_sq_small(__fsub_rn(b.y, a.y))),
+                     wrap_sq_small(__fsub_rn(b.z, a.z)));
+}
+
+// ifix(d / stepcl) without a table of edges: the product with the rounded reciprocal is within
+// 7.3e-4 of the rounded quotient while that is at most 4096, so its integer part is the index
+// unless it lies within 1e-3 of an integer; there (and for a NaN) the division decides.
+// rcp = step_rcp(stepcl, largest index asked for) is NaN, which always divides, beyond 4000.
+__host__ __device__ inline float step_rcp(float stepcl, int izmax) {
+    return izmax <= 4000 ? 1.0f / stepcl : nanf("");
+}
+__device__ __forceinline__ int bin_index(float d, float stepcl, float rcp) {
+    const float q = __fmul_rn(d, rcp);
+    const float big = __fadd_rz(q, 8388608.0f);          // 2^23 + trunc(q), 0 <= q < 2^23
+    const float fr = __fsub_rn(q, __fsub_rn(big, 8388608.0f));
+    int n = __float_as_int(big) - 0x4b000000;
+    if (!(fabsf(__fsub_rn(fr, 0.5f)) < 0.499f)) n = ifix(__fdiv_rn(d, stepcl));
+    return n;
+}
+
+// The IEEE square root without its range checks: one Newton step from the reciprocal square
+// root's approximation, the residual exact by the fused product.  Equal to __fsqrt_rn for zero and
+// for every float from 2^-60 to 2^4 (tests/test_pair_math_gpu.py compares all of them); squared
+// distances in box units lie there.
+__device__ __forceinline__ float sqrt_unit(float x) {
+    float s;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(s) : "f"(fmaxf(x, 1e-37f)));
+    const float d = __fmul_rn(x, s);
+    return __fmaf_rn(__fmaf_rn(-d, d, x), __fmul_rn(0.5f, s), d);
+}
+
 // pair_energy for a cubic box, bit for bit: the same distance, index, table entry and sum
 __device__ __forceinline__ float pair_energy_cubic_bins(const Bins &B, float4 p1, float4 p2, int icref) {
     const float d = __fsqrt_rn(__fadd_rn(__fadd_rn(wrap_sq(__fsub_rn(p2.x, p1.x)), wrap_sq(__fsub_rn(p2.y, p1.y))),

@@ -296,7 +296,7 @@ typedef struct {
 
 typedef struct {
     int32_t nbox, nmol, natom, ncell, nslot;
-    int32_t threads;              /* threads per move's CTA in propose and decide: 64, 128 or 256 */
+    int32_t threads;              /* least threads per move's CTA in propose and decide: 64, 128 or 256 */
     epsr_bmc_box_t *box;          /* [nbox] */
     const int32_t *slot_box;      /* [nslot] box of each slot */
     const int32_t *mol_box;       /* [nmol] box of each molecule */
@@ -321,7 +321,10 @@ typedef struct {
     long long *counters;          /* [nbox*4] attempts, first-stage accepts, accepts, left-cell */
     int64_t *sweep_counter;       /* [1] sweeps begun */
     int32_t *status;
+    float *cell_mol;              /* [4*nmol] read only when threads carries EPSR_BMC_CELL_MOL: the molecules in
+                                     cell order, centre and packed atoms (written by the binning and commits) */
 } epsr_bmc_t;
+#define EPSR_BMC_CELL_MOL 0x10000 /* added to threads: the structure ends with cell_mol */
 
 /* Partial g(r) histograms of every box over all atom pairs (atogen ato_manipulation_rev4.py:
  * 3640-3899 with every molecule an origin: intramolecular pairs once each (nint bin, weight 2
@@ -385,6 +388,11 @@ typedef struct {
  * k range split over kslices CTAs. */
 int epsr_umma_gemm_f32(const void *a, int32_t m, const void *b, int32_t n, int32_t k, int32_t kslices, float *out,
                        int32_t ldo, int32_t accumulate, int32_t *status, void *stream);
+
+/* Differences, over the floats of bit patterns lo .. hi - 1, between the kernels' branch-free pair
+ * arithmetic and the operations it stands for, counted into *bad (device): what 0 the square root
+ * (IEEE), 1 the table index ifix(x / par) (par the table step), 2 the squared minimum image. */
+int epsr_check_pair_math(int32_t what, uint32_t lo, uint32_t hi, float par, unsigned long long *bad, void *stream);
 /* device bytes of the work area for `rows` rows (forward or one training step) */
 int64_t epsr_mlp_work_bytes(int32_t rows);
 int epsr_mlp_sync_weights(const epsr_mlp_t *net, void *stream);
