@@ -101,6 +101,8 @@ struct SpecDev {
     float4 *edge_w;                        // [nedge] written by the propose pass
     int nedge;                             // 0: the energy pass divides (triclinic box, or too many bins)
     int ev;                                // the energy pass's staged values per chunk (>= 2 maxat^2)
+    const int32_t *ngrot;                  // [N] rotational groups of each molecule, or NULL
+    int32_t *ninter;                       // [2*nmoltype] zeroed by a cycle without internal rotations, or NULL
 };
 
 // ----------------------------------------------------------------- plan
@@ -141,6 +143,7 @@ __global__ void spec_plan_kernel(SpecDev S) {
                 istr = true;
             }
             nd += 1;
+            if (S.ngrot && S.ngrot[m] == 0) S.internrot[t] = 0.0f;
         }
         // per-type counts, one atomic per type present in the warp (integers: any order)
         {
@@ -194,9 +197,9 @@ __global__ void spec_plan_kernel(SpecDev S) {
     // per-type first-visit initialisation (molfit.py:377-394): a type whose molecules rotate
     // starts at rotstepmin if its step is not positive; otherwise its step is set to 0
     for (int t = tid; t < S.nmoltype; t += blockDim.x) {
-        // no molecule of this path has rotational groups: every visited type's internrot is
-        // set to 0 (molfit.py:358-360)
-        if (S.cnt_type[t] > 0) S.internrot[t] = 0.0f;
+        // a visited type's internrot is set to 0 (molfit.py:358-360); with groups in the box, by
+        // its molecules without any (above)
+        if (S.cnt_type[t] > 0 && !S.ngrot) S.internrot[t] = 0.0f;
         if (S.tries_rot[t] > 0) {
             if (S.rotstep[t] <= 0.0f) S.rotstep[t] = 1.0e-5f;
         }
@@ -879,6 +882,209 @@ __global__ void __launch_bounds__(SP_RT, 1) spec_resolve_kernel(SpecDev S) {
     }
 }
 
+// ----------------------------------------------------------------- walk (exact sums)
+// The cycles whose sums are the sequential kernel's: the reference's float sum in list order
+// (strict), or the sum in double rounded once to float (a box with rotational groups in a cycle
+// without internal rotations).  Both need every partner's term in full, decided or not, so the
+// running float sums of the resolver do not serve.
+//
+// One CTA; a warp takes every WK_NW-th move.  It waits for the decisions up to the WK_W-th move
+// before its own, resolves every other partner's terms with them, and its 32 lanes form the sum
+// for the 32 outcomes of the WK_W moves just before: the accept test of every lane is one
+// ballot, a table of the move's decision by theirs.  When their decisions are known, looking one
+// bit up decides the move, so the sums of WK_W + 1 moves run side by side and only a poll, a shift
+// and the running total of accepted changes lie between one decision and the next.
+//
+// Bound by the strict sum's chain: two dependent additions a partner, about 300 partners a
+// move, 2,800 cycles, of which six run at once.  The sequential kernel took 31 us a move
+// (24.4 ms a cycle of 259 DMSO + 518 water); with the energies evaluated side by side the cycle
+// takes 0.64 ms, draws included.
+constexpr int WK_W = 5;            // moves whose outcomes the lanes enumerate
+constexpr int WK_NW = 12;          // warps (moves in flight, most of them waiting or loading)
+constexpr int WK_CH = 256;         // partners resolved at a time
+constexpr int WK_MAXN = 65536;     // molecules whose decisions fit beside the staging
+
+struct WalkShared {
+    float2 t[WK_NW][WK_CH];        // {new, old} energy of each partner of the chunk
+    float2 c1[WK_NW][WK_W];        // an undecided partner's terms if it accepted
+    double d0[WK_NW][WK_W], d1[WK_NW][WK_W];   // the same in the double form, rejected and accepted
+    int cpos[WK_NW][WK_W];         // its place in the list
+    float fadd;
+    int abort_flag;
+    unsigned char dec[1];          // [N] 0 open, 1 rejected, 2 accepted
+};
+
+// Per move: each partner's visit position (-1: visited later) and the two stored energies its new
+// energy is compared with, {as the cycle began, after the partner's own move}.
+__global__ void __launch_bounds__(128) spec_terms_kernel(SpecDev S) {
+    if (S.flags[0]) return;
+    const int k = blockIdx.x;
+    const int m = S.visit[k];
+    const int nn = S.nergpairm[m];
+    const size_t row = (size_t)m * S.M, krow = (size_t)k * S.M;
+    for (int s = 1 + threadIdx.x; s < nn; s += blockDim.x) {
+        const size_t e = row + s;
+        const int kp = S.vpos[S.molergpair[e]];
+        const float sv = S.ergpair[S.ergpairref[e] - 1];
+        float after = sv;
+        if (kp < k) {
+            const int e2 = S.mirror[e];
+            if (e2 % S.M >= 1) after = S.A[e2];
+        }
+        S.farkp[krow + s - 1] = kp < k ? kp : -1;
+        S.fart[krow + s - 1] = make_float2(sv, after);
+    }
+    if (threadIdx.x == 0) S.nnk[k] = max(nn - 1, 0);
+}
+
+template <bool STRICT>
+__global__ void __launch_bounds__(32 * WK_NW, 1) spec_walk_kernel(SpecDev S) {
+    extern __shared__ __align__(16) unsigned char wk_smem[];
+    WalkShared &W = *reinterpret_cast<WalkShared *>(wk_smem);
+    volatile unsigned char *dec = W.dec;
+    volatile int *vabort = &W.abort_flag;
+    if (S.flags[0]) return;
+    const int N = S.N, M = S.M;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int i = threadIdx.x; i < N; i += blockDim.x) W.dec[i] = 0;
+    if (threadIdx.x == 0) {
+        W.fadd = 0.0f;
+        W.abort_flag = 0;
+    }
+    __syncthreads();
+    const float temp = __fdiv_rn(1.0f, S.simt);
+    float2 *t = W.t[w];
+    // move k is decided (by then so is every move before it); false when the wait gave up
+    auto decided = [&](int k) -> bool {
+        long long it = 0;
+        bool ok = true;
+        if (k >= 0)
+            while (dec[k] == 0) {
+                if (++it > SP_SPIN_LIMIT || *vabort) {
+                    ok = false;
+                    break;
+                }
+            }
+        __syncwarp();
+        return __all_sync(0xffffffffu, ok);
+    };
+    bool ok = true;
+    for (int k = w; k < N && ok; k += WK_NW) {
+        const int m = S.visit[k];
+        const int n = S.nnk[k];
+        const float thr = S.thr[k];
+        const float *A = S.A + (size_t)m * M + 1, *B = S.B + (size_t)m * M + 1;
+        const size_t krow = (size_t)k * M;
+        float f = 0.0f;
+        double sum = 0.0;
+        float a[WK_CH / 32], b[WK_CH / 32];
+        float2 o[WK_CH / 32];
+        int kp[WK_CH / 32];
+        auto load = [&](int c0) {
+#pragma unroll
+            for (int j = 0; j < WK_CH / 32; ++j) {
+                const int i = c0 + 32 * j + lane;
+                kp[j] = -2;
+                if (i < n) {
+                    kp[j] = S.farkp[krow + i];
+                    a[j] = A[i];
+                    o[j] = S.fart[krow + i];
+                    b[j] = kp[j] >= 0 ? B[i] : 0.0f;
+                }
+            }
+        };
+        load(0);
+        if (lane < WK_W) {
+            W.cpos[w][lane] = 0x7fffffff;
+            W.d0[w][lane] = W.d1[w][lane] = 0.0;
+        }
+        ok = decided(k - 1 - WK_W);
+        if (!ok) break;
+        for (int c0 = 0; c0 < n; c0 += WK_CH) {
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < WK_CH / 32; ++j) {
+                if (kp[j] == -2) continue;
+                const int i = 32 * j + lane;
+                const bool open = kp[j] >= max(k - WK_W, 0);   // one of the WK_W moves before
+                const bool acc = kp[j] >= 0 && !open && dec[kp[j]] == 2;
+                if (open) {
+                    const int q = k - 1 - kp[j];
+                    if (STRICT) {
+                        W.cpos[w][q] = c0 + i;
+                        W.c1[w][q] = make_float2(b[j], o[j].y);
+                    } else {
+                        W.d0[w][q] = (double)a[j] - (double)o[j].x;
+                        W.d1[w][q] = (double)b[j] - (double)o[j].y;
+                    }
+                }
+                if (STRICT) t[i] = acc ? make_float2(b[j], o[j].y) : make_float2(a[j], o[j].x);
+                else if (!open) sum += acc ? (double)b[j] - (double)o[j].y : (double)a[j] - (double)o[j].x;
+            }
+            __syncwarp();
+            const int nc = min(n - c0, WK_CH);
+            if (c0 + WK_CH < n) load(c0 + WK_CH);
+            if (STRICT) {
+                int cp[WK_W];
+#pragma unroll
+                for (int q = 0; q < WK_W; ++q) cp[q] = W.cpos[w][q];
+                for (int i = 0; i < nc;) {
+                    // up to the next undecided partner: the same terms in every lane
+                    int stop = c0 + nc, who = -1;
+#pragma unroll
+                    for (int q = 0; q < WK_W; ++q)
+                        if (cp[q] >= c0 + i && cp[q] < stop) {
+                            stop = cp[q];
+                            who = q;
+                        }
+                    const int e = stop - c0;
+                    for (; i < e && (i & 1); ++i) f = __fsub_rn(__fadd_rn(f, t[i].x), t[i].y);
+                    const float4 *t4 = reinterpret_cast<const float4 *>(t);
+#pragma unroll 4
+                    for (; i + 1 < e; i += 2) {
+                        const float4 v = t4[i >> 1];
+                        f = __fsub_rn(__fadd_rn(f, v.x), v.y);
+                        f = __fsub_rn(__fadd_rn(f, v.z), v.w);
+                    }
+                    for (; i < e; ++i) f = __fsub_rn(__fadd_rn(f, t[i].x), t[i].y);
+                    if (who >= 0) {
+                        const float2 v = (lane >> who) & 1 ? W.c1[w][who] : t[i];
+                        f = __fsub_rn(__fadd_rn(f, v.x), v.y);
+                        ++i;
+                    }
+                }
+            }
+        }
+        __syncwarp();
+        if (!STRICT) {
+            double tot = warp_sum_d(sum);
+#pragma unroll
+            for (int q = 0; q < WK_W; ++q) tot += (lane >> q) & 1 ? W.d1[w][q] : W.d0[w][q];
+            f = (float)tot;
+        }
+        const float e = __fmul_rn(__fadd_rn(f, 0.0f), temp);
+        const unsigned table = __ballot_sync(0xffffffffu, e < thr);
+        ok = decided(k - 1);
+        if (!ok) break;
+        const int q = k - 1 - lane;
+        const unsigned h = __ballot_sync(0xffffffffu, lane < WK_W && q >= 0 && dec[max(q, 0)] == 2);
+        const bool acc = (table >> h) & 1u;
+        const float fd = __shfl_sync(0xffffffffu, f, h);
+        if (lane == 0) {
+            if (acc) *(volatile float *)&W.fadd = __fadd_rn(*(volatile float *)&W.fadd, fd);
+            __threadfence_block();
+            dec[k] = acc ? 2 : 1;
+            S.acc[k] = acc ? 1 : 0;
+            S.fdiff[k] = fd;
+            if (k == N - 1) *S.fadd_acc = (double)*(volatile float *)&W.fadd;
+        }
+    }
+    if (!ok && lane == 0) {
+        *vabort = 1;
+        S.flags[1] = 1;
+    }
+}
+
 // ----------------------------------------------------------------- commit
 // The cycle's commits in one pass, one warp per molecule m (visited at position km), four
 // molecules a CTA: if its move was accepted, its stored energies (the later accepted writer of a
@@ -954,6 +1160,8 @@ __device__ void spec_epilogue(const SpecDev &S) {
     if (S.flags[0]) return;  // the sequential kernel runs this cycle
     const int nmt = S.nmoltype;
     const float rotstepmin = 1.0e-5f, rotstepmax = 1.0f;
+    if (S.ninter)
+        for (int t = 0; t < 2 * nmt; ++t) S.ninter[t] = 0;
     for (int t = 0; t < nmt; ++t) {
         // step values as the cycle leaves them: first-visit initialisation, or zero for a
         // visited type that does not rotate / translate (molfit.py:377-396)
@@ -1084,7 +1292,7 @@ static int ahead_stream(AheadStream **out) {
     return EPSR_OK;
 }
 int molfit_seq_launch(const epsr_box_t *box, const epsr_cells_t *cells, epsr_store_t *store, epsr_mc_t *mc,
-                      void *scratch, int64_t scratch_bytes, cudaStream_t s, const int32_t *run_if);
+                      void *scratch, int64_t scratch_bytes, cudaStream_t s, const int32_t *run_if, bool strict);
 }  // namespace epsr
 
 using namespace epsr;
@@ -1114,8 +1322,10 @@ extern "C" int64_t epsr_molfit_spec_scratch_bytes(int32_t nmol, int32_t natom, i
     return (int64_t)spec_bytes(nmol, natom, M, nmoltype);
 }
 
+// mode 0: the fast cycle; 1: the reference's float sums (spec_walk_kernel<true>); 2: sums in double
+// rounded once (spec_walk_kernel<false>).
 int epsr_molfit_spec(const epsr_box_t *box, const epsr_cells_t *cells, epsr_store_t *store, epsr_mc_t *mc,
-                     void *scratch, int64_t scratch_bytes, void *stream) {
+                     void *scratch, int64_t scratch_bytes, void *stream, int mode) {
     const int N = box->nmol, M = store->nnbrefmax, nmt = box->nmoltype, natom = box->natom;
     if (!store->mirror) {
         epsr_set_error("epsr_molfit: the fast path needs the store's mirror index (built by epsr_fmolec1)");
@@ -1125,7 +1335,7 @@ int epsr_molfit_spec(const epsr_box_t *box, const epsr_cells_t *cells, epsr_stor
         int dev = 0, optin = 0;
         EPSR_CUDA(cudaGetDevice(&dev));
         EPSR_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-        if (spec_resolve_smem(N) > (size_t)optin) {
+        if (mode == 0 && spec_resolve_smem(N) > (size_t)optin) {
             epsr_set_error("epsr_molfit: %d molecules need %zu bytes of shared memory in the resolver (at most %d)", N,
                            spec_resolve_smem(N), optin);
             return EPSR_ERR_CAPACITY;
@@ -1138,6 +1348,10 @@ int epsr_molfit_spec(const epsr_box_t *box, const epsr_cells_t *cells, epsr_stor
     cudaStream_t s = (cudaStream_t)stream;
     SpecDev S;
     memset(&S, 0, sizeof(S));
+    if (mc->intra) {
+        S.ngrot = ((const epsr_intra_t *)mc->intra)->ngrot;
+        S.ninter = mc->ninter;
+    }
     S.L.cubic = box->cubic;
     S.L.alatx = box->lat[0];
     S.L.blatx = box->lat[1];
@@ -1285,23 +1499,46 @@ int epsr_molfit_spec(const epsr_box_t *box, const epsr_cells_t *cells, epsr_stor
         EPSR_SMEM_OPTIN(spec_energy_kernel<false>);
         EPSR_TIMED("spec_energy_kernel", s, spec_energy_kernel<false><<<N, SP_ET, en_bytes, s>>>(S));
     }
-    EPSR_CUDA(cudaMemsetAsync(S.nearT, 0, sizeof(float2) * npad * SP_W, s));
-    EPSR_TIMED("spec_corr_kernel", s, spec_corr_kernel<<<N, 128, 0, s>>>(S));
-    // the walk is latency-bound on its scheduler: the CTA asks for all the shared memory a CTA
-    // may have (its own need, spec_resolve_smem(N), is checked above), so no other kernel's CTA
-    // shares the SM and takes issue slots from it
-    size_t rsmem = spec_resolve_smem(N);
-    {
+    if (mode != 0) {
+        spec_terms_kernel<<<N, 128, 0, s>>>(S);
         int dev = 0, optin = 0;
         EPSR_CUDA(cudaGetDevice(&dev));
         EPSR_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-        rsmem = max(rsmem, (size_t)optin - 1024);
+        const size_t wsmem = (size_t)optin - 1024;   // no other kernel's CTA shares the walk's SM
+        if (mode == 1) {
+            EPSR_SMEM_OPTIN(spec_walk_kernel<true>);
+            EPSR_TIMED("spec_walk_kernel", s, spec_walk_kernel<true><<<1, 32 * WK_NW, wsmem, s>>>(S));
+        } else {
+            EPSR_SMEM_OPTIN(spec_walk_kernel<false>);
+            EPSR_TIMED("spec_walk_kernel", s, spec_walk_kernel<false><<<1, 32 * WK_NW, wsmem, s>>>(S));
+        }
+    } else {
+        EPSR_CUDA(cudaMemsetAsync(S.nearT, 0, sizeof(float2) * npad * SP_W, s));
+        EPSR_TIMED("spec_corr_kernel", s, spec_corr_kernel<<<N, 128, 0, s>>>(S));
+        // the walk is latency-bound on its scheduler: the CTA asks for all the shared memory a CTA
+        // may have (its own need, spec_resolve_smem(N), is checked above), so no other kernel's CTA
+        // shares the SM and takes issue slots from it
+        size_t rsmem = spec_resolve_smem(N);
+        {
+            int dev = 0, optin = 0;
+            EPSR_CUDA(cudaGetDevice(&dev));
+            EPSR_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+            rsmem = max(rsmem, (size_t)optin - 1024);
+        }
+        EPSR_SMEM_OPTIN(spec_resolve_kernel);
+        EPSR_TIMED("spec_resolve_kernel", s, spec_resolve_kernel<<<1, SP_RT, rsmem, s>>>(S));
     }
-    EPSR_SMEM_OPTIN(spec_resolve_kernel);
-    EPSR_TIMED("spec_resolve_kernel", s, spec_resolve_kernel<<<1, SP_RT, rsmem, s>>>(S));
     EPSR_TIMED("spec_commit_kernel", s, spec_commit_kernel<<<(N + SP_CW - 1) / SP_CW, 32 * SP_CW, 0, s>>>(S));
     EPSR_CUDA(cudaGetLastError());
     if (ahead) EPSR_CUDA(cudaStreamWaitEvent(s, as->join, 0));
     // a cycle with a translation retry runs on the sequential kernel (no-op otherwise)
-    return molfit_seq_launch(box, cells, store, mc, nullptr, 0, s, S.flags);
+    return molfit_seq_launch(box, cells, store, mc, nullptr, 0, s, S.flags, mode == 1);
+}
+
+// Whether the walk takes a cycle of this box: its decisions fit, the store has its mirror index
+// and the scratch is the fast path's (a caller of the strict cycle may have given none).
+bool epsr_molfit_walk_fits(const epsr_box_t *box, const epsr_store_t *store, const void *scratch, int64_t scratch_bytes) {
+    return box->nmol <= WK_MAXN && store->mirror && scratch && box->maxat <= SP_MAXAT &&
+           (int64_t)spec_bytes(box->nmol, box->natom, store->nnbrefmax, box->nmoltype) <= scratch_bytes &&
+           sizeof(float) * 2 * (size_t)store->nnbrefmax <= 160 * 1024;
 }

@@ -1,0 +1,66 @@
+"""The cycles whose sums are exact (strict float sums in list order; double sums of a box with
+rotational groups in a cycle without rotations) on the walk against the sequential kernel, which a
+store without its mirror index selects: the same moves of the same stream.  Strict cycles agree
+bit for bit; the double sums add the same doubles in another order, so a change may differ where
+their rounding to float does (one unit in the last place)."""
+
+import numpy as np
+import pytest
+import torch
+
+from epsr_python_translation_b200 import configs
+from epsr_python_translation_b200.box import BoxArrays, Ran1State, trsteps
+
+pytestmark = pytest.mark.gpu
+f32 = np.float32
+
+
+def _box(s, groups):
+    from epsr_python_translation_b200.device import DeviceBox
+    from epsr_python_translation_b200.intra import IntraModel
+    box = BoxArrays.from_system(s)
+    d = DeviceBox(box)
+    d.cell_list(10, box.sepmax)
+    d.fmolec1(configs.intra_energies(s), strict=True)
+    tmax, tmin = trsteps(box.natomr)
+    d.mc_setup(rejrate=0.75, stepr=1.0, stepm=1.0, wholerot=np.full(s.nmoltype, f32(0.05), f32),
+               wholetrans=np.full(s.nmoltype, f32(0.3) / s.dmax, f32), ran1=Ran1State(idum=-77), trstepmax=tmax,
+               trstepmin=tmin)
+    if groups:
+        r = configs.rotations(s)
+        d.set_rotations(IntraModel(d, **configs.intra_model(s), ngrot=r["ngrot"]), r["nrf"], r["nrl"], r["axis"],
+                        r["first"], r["last"], r["atoms"])
+        d.m_internrot.copy_(torch.tensor([0.05, 0.02]))
+    return d
+
+
+SYSTEMS = {
+    # fewer molecules than the enumerated window, than the warps, one list chunk, several chunks
+    "water_4": lambda: configs.c1_water(seed=3, nmol=4), "water_9": lambda: configs.c1_water(seed=4, nmol=9),
+    "water_100": lambda: configs.c1_water(seed=5), "water_1200": lambda: configs.c1_water(seed=6, nmol=1200),
+    "mixture_45": lambda: configs.c2_mixture(seed=7, ndmso=15, nwater=30),
+    "silica_301": lambda: configs.silica(seed=8, natom=301),
+}
+
+
+@pytest.mark.parametrize("name,groups", [(k, False) for k in SYSTEMS] + [("mixture_45", True)])
+def test_walk_matches_sequential_kernel(name, groups):
+    s = SYSTEMS[name]()
+    a, b = _box(s, groups), _box(s, groups)
+    b.store.mirror = None            # the sequential kernel
+    for _ in range(3):
+        for d in (a, b):
+            d.molfit(strict=not groups, rotcycle=False)
+            d.check_status()
+        x, y = a.download_mc(), b.download_mc()
+        if groups:
+            assert np.all(np.abs(x["den"] - y["den"]) <= np.spacing(np.abs(y["den"])))
+        else:
+            assert np.array_equal(x["den"].view(np.uint32), y["den"].view(np.uint32))
+            assert x["fadds"] == y["fadds"]
+        for k in ("acc", "wholerot", "wholetrans", "internrot", "interntrans", "nwhole", "nmovem", "nstepreject"):
+            assert np.array_equal(x[k], y[k]), k
+        assert np.array_equal(x["ran1"].as_array(), y["ran1"].as_array())
+        ca, cb = a.download_coords(), b.download_coords()
+        assert all(np.array_equal(ca[k].view(np.uint32), cb[k].view(np.uint32)) for k in ca)
+        assert np.array_equal(a.download_store()["ergpair"], b.download_store()["ergpair"])
