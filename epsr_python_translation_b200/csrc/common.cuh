@@ -238,6 +238,19 @@ __device__ __forceinline__ float pair_energy_cubic_bins(const Bins &B, float4 p1
     return in ? sume : 0.0f;
 }
 
+// pair_energy for a cubic box in box units, bit for bit, with the branch-free root, wrap and
+// index above; rcp = step_rcp(T.stepcl, T.izcut)
+__device__ __forceinline__ float pair_energy_unit(const Tables &T, float rcp, float4 p1, float4 p2, int icref) {
+    const float d = sqrt_unit(dsq_cubic(p1, p2));
+    const int iz = bin_index(d, T.stepcl, rcp) + 2;
+    const int izc = min(max(iz, 2), T.izcut);
+    const float4 t = __ldg(T.tab + (size_t)icref * T.ld + izc);
+    const float dt = __fsub_rn(d, __ldg(T.xstar + izc));
+    float sume = __fadd_rn(t.x, __fmul_rn(t.y, dt));
+    sume = __fadd_rn(__fadd_rn(sume, t.z), __fmul_rn(t.w, dt));
+    return iz == izc ? sume : 0.0f;
+}
+
 // ----------------------------------------------------------------- ran1 (device, one lane)
 // auxiliary_routines.py:324-391 with state {idum, iy, mcall, iv[32]}.
 struct Ran1 {

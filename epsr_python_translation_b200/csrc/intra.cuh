@@ -222,4 +222,29 @@ static __device__ float en_mole_intra_d(const IntraDev &I, int im, const float *
     return e;
 }
 
+// en_mole_intra by one warp: the pair values side by side into `vals` (n (n - 1) / 2 of shared
+// memory), then their sum in the reference's order; the same value in every lane.
+static __device__ float en_mole_intra_warp(const IntraDev &I, int im, const float *x, const float *y, const float *z,
+                                           float *vals) {
+    const int lane = threadIdx.x & 31;
+    const int a0 = I.naf[im], n = I.nato[im];
+    const int np = n * (n - 1) / 2;
+    int i = 0, r = lane;   // pair `lane` is (i, i + 1 + r)
+    for (int p = lane; p < np; p += 32) {
+        while (r >= n - 1 - i) {
+            r -= n - 1 - i;
+            ++i;
+        }
+        const int ia = a0 + i, ja = ia + 1 + r;
+        vals[p] = en_atom_intra_d(I, im, ia, ja, x[ia], y[ia], z[ia], x[ja], y[ja], z[ja]);
+        r += 32;
+    }
+    __syncwarp();
+    float e = 0.0f;
+    for (int p = 0; p < np; ++p) e = __fadd_rn(e, vals[p]);
+    if (has_dihedral_term(I, im)) e = __fadd_rn(e, dihedral_term_d(I, im, x, y, z));
+    __syncwarp();
+    return e;
+}
+
 }  // namespace epsr

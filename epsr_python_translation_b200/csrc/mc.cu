@@ -2,11 +2,16 @@
 //
 // Sequential kernel: one CTA walks the molecules in cell-visit order exactly as the
 // reference (the ran1 stream and the accept decisions chain every move to the previous
-// one).  Per move: one thread draws the rotation (rotatm :672) and translation (movem :733,
-// including the step-doubling retry); all threads evaluate the moved molecule against its
-// stored neighbours, one neighbour per thread in the reference's (ia, ja) order so each
-// neighbour energy is bit-identical (en_change :806); then the Metropolis test (:401-408),
-// the store update (save_energies/save_erg_pairs) and the coordinate commit or restore.
+// one).  Per move: the first warp draws the rotation (rotatm :672) and translation (movem :733,
+// including the step-doubling retry); all threads evaluate the moved molecule against the
+// atoms of its stored neighbours, and each neighbour's pair energies are added in the
+// reference's (ia, ja) order so its energy is bit-identical (en_change :806); then the Metropolis
+// test (:401-408), the store update (save_energies/save_erg_pairs) and the coordinate commit.
+//
+// Bound by the chain of one move after another.  A neighbour per thread (up to a hundred pair
+// evaluations one behind the other), the proposal and the intramolecular energy (forty-five
+// pairs of dependent list look-ups for DMSO) on one thread took 31 us a move, and 25-32 ms for
+// a cycle of 200 DMSO + 400 water with rotating methyl groups; about 10 ms a cycle now.
 #include <string.h>
 
 #include "common.cuh"
@@ -14,8 +19,9 @@
 
 namespace epsr {
 
-constexpr int MC_THREADS = 512;
+constexpr int MC_THREADS = 1024;
 constexpr int MC_MAXAT = 64;  // atoms per molecule handled by the kernel
+constexpr int MC_RING = 512;  // draws held ahead (batches of 32)
 
 struct McDev {
     Lattice L;
@@ -38,6 +44,8 @@ struct McDev {
     int32_t *trace_acc;
     float *ergnew_g;   // [M] global fallback when M is large
     int use_smem;
+    int ev;            // pair values staged at a time (>= 64 x 64)
+    float rcp;         // step_rcp of the tables (cubic boxes)
     int32_t *status;
     const int32_t *run_if;  // when set, the kernel runs only if *run_if != 0
     // internal rotations of rotational groups (molfit.py:295-360), when has_rot
@@ -84,150 +92,282 @@ __device__ __forceinline__ void rotati_d(const McDev &D, int a0, int ig, float c
     }
 }
 
-__device__ __forceinline__ float next_cos(const McDev &D, int &kcos, float phi) {
-    if (D.cos_override) return D.cos_override[kcos++];
-    ++kcos;
-    return cos_r(phi);
-}
+// The ran1 stream of a cycle, drawn by one warp in batches of 32 into a ring; any lane may read
+// draws the warp has asked for.  finish() leaves the state after exactly the draws taken: the
+// state before the batch that holds the next draw, walked on.
+struct DrawRing {
+    float v[MC_RING];
+    int32_t tab[34];
+    int32_t state[MC_RING / 32][34];   // idum, iy, iv[32] before each batch
+    long long start[MC_RING / 32];
+};
+struct Draws {
+    Ran1Warp g;
+    DrawRing *r;
+    long long gen, used, batch;
+    int32_t mcall;
+    __device__ __forceinline__ void begin(DrawRing *ring, const int32_t *state) {
+        r = ring;
+        g.load(state);
+        mcall = state[2];
+        gen = used = batch = 0;
+    }
+    // the next n (at most 256) draws are in the ring; returns the position of the first
+    __device__ __forceinline__ long long take(int n) {
+        const int lane = threadIdx.x & 31;
+        while (gen - used < n) {
+            const int slot = (int)(batch & (MC_RING / 32 - 1));
+            r->state[slot][2 + lane] = g.iv;
+            if (lane == 0) {
+                r->state[slot][0] = g.idum;
+                r->state[slot][1] = g.iy;
+                r->start[slot] = gen;
+            }
+            int32_t mine;
+            const int cnt = g.next(32, mine, r->tab);
+            if (lane < cnt) r->v[(gen + lane) & (MC_RING - 1)] = ran1_out(mine);
+            gen += cnt;
+            ++batch;
+            __syncwarp();
+        }
+        const long long at = used;
+        used += n;
+        return at;
+    }
+    __device__ __forceinline__ float get(long long i) const { return r->v[i & (MC_RING - 1)]; }
+    __device__ void finish(int32_t *out) const {   // one lane
+        Ran1 s;
+        s.idum = g.idum;
+        s.iy = g.iy;
+        for (int i = 0; i < 32; ++i) s.iv[i] = 0;
+        long long from = -1;
+        for (long long b = batch - 1; b >= 0 && b > batch - MC_RING / 32; --b) {
+            const int slot = (int)(b & (MC_RING / 32 - 1));
+            if (r->start[slot] <= used) {
+                from = r->start[slot];
+                s.idum = r->state[slot][0];
+                s.iy = r->state[slot][1];
+                for (int i = 0; i < 32; ++i) s.iv[i] = r->state[slot][2 + i];
+                break;
+            }
+        }
+        if (from < 0) return;   // no draw was made: the state stays
+        for (long long i = from; i < used; ++i) ran1_next(s);
+        s.mcall = (int32_t)((uint32_t)mcall + (uint32_t)used);
+        ran1_store(s, out);
+    }
+};
 
-__global__ void __launch_bounds__(MC_THREADS) molfit_seq_kernel(McDev D) {
-    extern __shared__ float dyn[];  // ergnew[M], ergold[M] when use_smem
-    __shared__ Ran1 R;
+__global__ void __launch_bounds__(MC_THREADS, 1) molfit_seq_kernel(McDev D) {
+    extern __shared__ __align__(16) float dyn[];   // vals[ev], items[ev] (16 bits), ergnew[M], ergold[M] when use_smem
+    __shared__ DrawRing ring;
     __shared__ float4 mv[MC_MAXAT];
     __shared__ float nx[MC_MAXAT], ny[MC_MAXAT], nz[MC_MAXAT];
-    __shared__ float sx[MC_MAXAT], sy[MC_MAXAT], sz[MC_MAXAT];
-    __shared__ int sh_im, sh_n, sh_acc, sh_bad, sh_rot;
-    __shared__ float sh_cx, sh_cy, sh_cz, sh_fdiff;
+    __shared__ float intra_vals[MC_MAXAT * (MC_MAXAT - 1) / 2];
+    __shared__ int c_b0[MC_THREADS];
+    __shared__ unsigned short c_voff[MC_THREADS];
+    __shared__ unsigned char c_nb[MC_THREADS];
+    __shared__ int ws_v[MC_THREADS / 32], ws_i[MC_THREADS / 32];
+    __shared__ int sh_im, sh_n, sh_acc, sh_rot, sh_items, sh_take;
+    __shared__ float sh_cx, sh_cy, sh_cz, sh_intra;
     __shared__ double red[MC_THREADS / 32];
     if (D.run_if && *D.run_if == 0) return;
-    float *ergnew = D.use_smem ? dyn : D.ergnew_g;
-    float *ergold = D.use_smem ? dyn + D.M : D.ergnew_g + D.M;
-    const int tid = threadIdx.x;
+    float *vals = dyn;
+    unsigned short *items = (unsigned short *)(dyn + D.ev);
+    float *ergnew = D.use_smem ? dyn + D.ev + D.ev / 2 : D.ergnew_g;
+    float *ergold = ergnew + D.M;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int nmt = D.nmoltype;
     const float pi = 3.14159265358979323846f;
     const float rotstepmin = 1.0e-5f, rotstepmax = 1.0f;
+    // the state of the chain, the same in every lane of warp 0
+    Draws R;
     int kcos = 0;
     float fadd = 0.0f, faddb = 0.0f;
     // the reference's ergold(1) (molfit's work array): the first stored energy of the last
     // molecule whose list was loaded, as updated by that molecule's accepted moves
     float eold0 = 0.0f, p0 = 0.0f;
-    if (tid == 0) {
-        ran1_load(R, D.ran1);
-        for (int k = 0; k < 2 * nmt; ++k) {
-            D.nwhole[k] = 0;
-            D.nmovem[k] = 0;
-            if (D.ninter) D.ninter[k] = 0;
-            if (D.nmovei) D.nmovei[k] = 0;
-        }
+    if (wid == 0) R.begin(&ring, D.ran1);
+    for (int k = tid; k < 2 * nmt; k += MC_THREADS) {
+        D.nwhole[k] = 0;
+        D.nmovem[k] = 0;
+        if (D.ninter) D.ninter[k] = 0;
+        if (D.nmovei) D.nmovei[k] = 0;
     }
     const float temp = __fdiv_rn(1.0f, D.simt);
     __syncthreads();
-    // en_change (molfit.py:806-919) of molecule sh_im at positions mv[] over its stored list:
-    // ergnew/ergold filled for slots 1.., the change summed in list order (strict) or in double
-    auto en_change_mv = [&](int im, int n) -> float {
+    // Metropolis (:401-408): exp(-x) against the draw
+    auto accepts = [&](float ediff, float u) -> int {
+        float etest;
+        if (ediff <= 0.0f) etest = 10.0f;
+        else if (ediff < 20.0f) etest = exp_r(-ediff);
+        else etest = 0.0f;
+        return u < etest;
+    };
+    // `n` cosines (molfit's angles in draw order), lane q's angle phi: cosine and signed sine
+    auto cosines = [&](int n, float phi, float &c, float &s) {
+        c = 1.0f;
+        if (lane < n) c = D.cos_override ? D.cos_override[kcos + lane] : cos_r(phi);
+        kcos += n;
+        s = fsign(__fsqrt_rn(__fsub_rn(1.0f, __fmul_rn(c, c))), phi);
+    };
+    // en_change (molfit.py:806-919) of molecule im at positions mv[] over its stored list:
+    // ergnew/ergold filled for slots 1.., the change summed in list order (strict) or in double;
+    // the value is warp 0's.  `fresh`: the list's items are not those of the call before.  The last
+    // warp adds the trial's intramolecular energy (`intra`) meanwhile.
+    auto en_change_mv = [&](int im, int n, bool fresh, bool intra) -> float {
         const size_t row = (size_t)im * D.M;
         const int nn = D.nergpairm[im];
+        auto trial_intra = [&]() {
+            const int a0 = D.naf[im];
+            const float e = en_mole_intra_warp(D.I, im, nx - a0, ny - a0, nz - a0, intra_vals);
+            if (lane == 0) sh_intra = e;
+        };
+        bool todo = intra;   // the trial's intramolecular energy is still to be formed
+        if (todo && nn <= 1) {
+            if (wid == MC_THREADS / 32 - 1) trial_intra();
+            todo = false;
+        }
         double part = 0.0;
-        for (int inn = 1 + tid; inn < nn; inn += MC_THREADS) {
-            const int jm = D.molergpair[row + inn];
-            const int b0 = D.naf[jm], b1 = b0 + D.nato[jm];
-            float sume = 0.0f;
-            for (int ia = 0; ia < n; ++ia) {
-                const float4 p1 = mv[ia];
-                const int it = __float_as_int(p1.w);
-                for (int ja = b0; ja < b1; ++ja) {
-                    const float4 p2 = D.pos[ja];
-                    const int icref = __ldg(D.npairref + it * D.ntype + __float_as_int(p2.w));
-                    sume = __fadd_rn(sume, pair_energy(D.L, D.T, p1, p2, icref));
+        bool kept = !fresh;
+        for (int s0 = 1; s0 < nn;) {
+            // a chunk: partners from s0 (one a thread) whose pair values fit the staging
+            const int inn = s0 + tid;
+            int ntake;
+            if (kept && s0 == 1 && sh_take >= nn - 1) {
+                ntake = sh_take;
+            } else {
+                int b0 = 0, nb = 0;
+                if (inn < nn) {
+                    const int jm = D.molergpair[row + inn];
+                    b0 = D.naf[jm];
+                    nb = D.nato[jm];
+                }
+                int ii = nb;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int u = __shfl_up_sync(0xffffffffu, ii, o);
+                    if (lane >= o) ii += u;
+                }
+                if (lane == 31) ws_i[wid] = ii;
+                __syncthreads();
+                ii += __reduce_add_sync(0xffffffffu, lane < wid ? ws_i[lane] : 0);
+                const bool take = inn < nn && ii * n <= D.ev;
+                if (take) {
+                    c_b0[tid] = b0;
+                    c_nb[tid] = (unsigned char)nb;
+                    c_voff[tid] = (unsigned short)(ii - nb);
+                    for (int j = 0; j < nb; ++j) items[ii - nb + j] = (unsigned short)((tid << 6) | j);
+                }
+                ntake = __syncthreads_count(take);
+                if (take && tid == ntake - 1) {
+                    sh_items = ii;
+                    sh_take = ntake;
+                }
+                __syncthreads();
+            }
+            const bool mine = tid < ntake;
+            float eo = 0.0f;
+            if (mine) eo = D.ergpair[D.ergpairref[row + inn] - 1];
+            // items: a partner's atom against every atom of the moved molecule
+            const int nit = sh_items, nthr = todo ? MC_THREADS - 32 : MC_THREADS;
+            if (tid >= nthr) trial_intra();
+            for (int it = tid; it < nit && tid < nthr; it += nthr) {
+                const int code = items[it], t = code >> 6, ja = code & 63, nb = c_nb[t];
+                const float4 p2 = D.pos[c_b0[t] + ja];
+                const int *col = D.npairref + __float_as_int(p2.w);
+                float *v = vals + (int)c_voff[t] * n + ja;
+                if (D.L.cubic) {
+#pragma unroll 2
+                    for (int ia = 0; ia < n; ++ia) {
+                        const float4 p1 = mv[ia];
+                        v[ia * nb] = pair_energy_unit(D.T, D.rcp, p1, p2, __ldg(col + __float_as_int(p1.w) * D.ntype));
+                    }
+                } else {
+                    for (int ia = 0; ia < n; ++ia) {
+                        const float4 p1 = mv[ia];
+                        v[ia * nb] = pair_energy(D.L, D.T, p1, p2, __ldg(col + __float_as_int(p1.w) * D.ntype));
+                    }
                 }
             }
-            const float en = __fadd_rn(0.0f, sume);
-            const float eo = D.ergpair[D.ergpairref[row + inn] - 1];
-            ergnew[inn] = en;
-            ergold[inn] = eo;
-            part += (double)en - (double)eo;
-        }
-        float fdiff;
-        if (D.strict) {
             __syncthreads();
-            if (tid == 0) {
-                float f = 0.0f;
-                for (int inn = 1; inn < nn; ++inn) f = __fsub_rn(__fadd_rn(f, ergnew[inn]), ergold[inn]);
-                red[0] = (double)f;
+            if (mine) {
+                const float *v = vals + (int)c_voff[tid] * n;
+                const int nv = n * c_nb[tid];
+                float sume = 0.0f;
+                for (int q = 0; q < nv; ++q) sume = __fadd_rn(sume, v[q]);
+                const float en = __fadd_rn(0.0f, sume);
+                ergnew[inn] = en;
+                ergold[inn] = eo;
+                part += (double)en - (double)eo;
             }
-            __syncthreads();
-            fdiff = (float)red[0];
-        } else {
+            s0 += ntake;
+            if (s0 < nn) __syncthreads();   // the staging is rewritten
+            kept = todo = false;
+        }
+        if (!D.strict) {
             part = warp_sum_d(part);
-            if ((tid & 31) == 0) red[tid >> 5] = part;
-            __syncthreads();
-            double t = 0.0;
-            for (int w = 0; w < MC_THREADS / 32; ++w) t += red[w];
-            fdiff = (float)t;
+            if (lane == 0) red[wid] = part;
         }
         __syncthreads();
+        float fdiff = 0.0f;
+        if (wid == 0) {
+            if (D.strict) {
+#pragma unroll 4
+                for (int inn = 1; inn < nn; ++inn) fdiff = __fsub_rn(__fadd_rn(fdiff, ergnew[inn]), ergold[inn]);
+            } else {
+                fdiff = (float)warp_sum_d(red[lane]);
+            }
+        }
         return fdiff;
     };
-    for (int v = 0; v < D.nmol; ++v) {
-        if (tid == 0) {
-            const int im = D.shake ? v : D.visit[v];
-            const int n = D.nato[im];
-            sh_bad = n > MC_MAXAT;
-        }
-        __syncthreads();
-        if (sh_bad) {
+    {   // a box with a molecule larger than the kernel's arrays: nothing is moved
+        bool bad = false;
+        for (int m = tid; m < D.nmol; m += MC_THREADS) bad = bad || D.nato[m] > MC_MAXAT;
+        if (__syncthreads_or(bad)) {
             if (tid == 0 && D.status) D.status[0] = 1;
             return;
         }
+    }
+    for (int v = 0; v < D.nmol; ++v) {
         // ---- internal rotations of the molecule's rotational groups (molfit.py:295-360), in
         // the intramolecular cycle after the molecule's atom moves (:141-267)
-        if (tid == 0) {
+        if (wid == 0) {
             const int im = D.shake ? v : D.visit[v];
-            const int n = D.nato[im];
+            const int n = D.nato[im], a0 = D.naf[im];
             const int mt = D.mtype[im];
             const size_t row = (size_t)im * D.M;
-            if (D.nergpairm[im] >= 1) eold0 = D.ergpair[D.ergpairref[row] - 1];   // make_neighbour_list_from_mols
+            const int nn = D.nergpairm[im];
+            if (nn >= 1) eold0 = D.ergpair[D.ergpairref[row] - 1];   // make_neighbour_list_from_mols
+            const float cx = D.xadd[im], cy = D.yadd[im], cz = D.zadd[im];
             if (D.shake && n > 1 && D.stepmi > 0.0f) {
                 // movei/movea (:545-567) on the offsets, en_change_intra against ergold(1), the
                 // Metropolis test; on acceptance the store's first slot (save_energies,
                 // save_erg_pairs) and the centre of mass put back (centreofmassi)
                 float step = D.interntrans[mt];
                 if (step == 0.0f) step = D.trstepmin;
-                D.interntrans[mt] = step;
-                const int a0 = D.naf[im];
-                for (int k = 0; k < n; ++k) {
-                    sx[k] = D.xa[a0 + k];
-                    sy[k] = D.ya[a0 + k];
-                    sz[k] = D.za[a0 + k];
-                }
-                D.nmovei[mt]++;
-                for (int k = 0; k < n; ++k) {
+                const long long at = R.take(3 * n + 1);
+                for (int k = lane; k < n; k += 32) {
                     const int a = a0 + k;
-                    D.za[a] = __fadd_rn(D.za[a], __fmul_rn(step, __fsub_rn(__fmul_rn(2.0f, ran1_next(R)), 1.0f)));
-                    D.ya[a] = __fadd_rn(D.ya[a], __fmul_rn(step, __fsub_rn(__fmul_rn(2.0f, ran1_next(R)), 1.0f)));
-                    D.xa[a] = __fadd_rn(D.xa[a], __fmul_rn(step, __fsub_rn(__fmul_rn(2.0f, ran1_next(R)), 1.0f)));
+                    nz[k] = __fadd_rn(D.za[a], __fmul_rn(step, __fsub_rn(__fmul_rn(2.0f, R.get(at + 3 * k)), 1.0f)));
+                    ny[k] = __fadd_rn(D.ya[a], __fmul_rn(step, __fsub_rn(__fmul_rn(2.0f, R.get(at + 3 * k + 1)), 1.0f)));
+                    nx[k] = __fadd_rn(D.xa[a], __fmul_rn(step, __fsub_rn(__fmul_rn(2.0f, R.get(at + 3 * k + 2)), 1.0f)));
                 }
-                const float enew = en_mole_intra_d(D.I, im, D.xa, D.ya, D.za);
+                __syncwarp();
+                const float enew = en_mole_intra_warp(D.I, im, nx - a0, ny - a0, nz - a0, intra_vals);
                 const float fdiffb = __fsub_rn(enew, eold0);
-                const float ediff = __fmul_rn(fdiffb, temp);
-                float etest;
-                if (ediff <= 0.0f) etest = 10.0f;
-                else if (ediff < 20.0f) etest = exp_r(-ediff);
-                else etest = 0.0f;
-                if (ran1_next(R) < etest) {
+                const int acc = accepts(__fmul_rn(fdiffb, temp), R.get(at + 3 * n));
+                if (acc) {
                     faddb = __fadd_rn(faddb, fdiffb);
-                    if (D.nergpairm[im] >= 1) {
-                        eold0 = enew;
-                        D.ergpair[D.ergpairref[row] - 1] = enew;
-                    }
+                    if (nn >= 1) eold0 = enew;
                     float x1 = 0.0f, y1 = 0.0f, z1 = 0.0f, summass = 0.0f;
                     for (int k = 0; k < n; ++k) {
                         const int a = a0 + k;
                         if (D.I.qtype[a] == 0) {
                             const float am = D.I.amassa[D.I.itype[a]];
-                            x1 = __fadd_rn(x1, __fmul_rn(D.xa[a], am));
-                            y1 = __fadd_rn(y1, __fmul_rn(D.ya[a], am));
-                            z1 = __fadd_rn(z1, __fmul_rn(D.za[a], am));
+                            x1 = __fadd_rn(x1, __fmul_rn(nx[k], am));
+                            y1 = __fadd_rn(y1, __fmul_rn(ny[k], am));
+                            z1 = __fadd_rn(z1, __fmul_rn(nz[k], am));
                             summass = __fadd_rn(summass, am);
                         }
                     }
@@ -236,201 +376,204 @@ __global__ void __launch_bounds__(MC_THREADS) molfit_seq_kernel(McDev D) {
                         y1 = __fdiv_rn(y1, summass);
                         z1 = __fdiv_rn(z1, summass);
                     }
-                    const float cx = D.xadd[im], cy = D.yadd[im], cz = D.zadd[im];
-                    for (int k = 0; k < n; ++k) {
+                    for (int k = lane; k < n; k += 32) {
                         const int a = a0 + k;
-                        D.xa[a] = __fsub_rn(D.xa[a], x1);
-                        D.ya[a] = __fsub_rn(D.ya[a], y1);
-                        D.za[a] = __fsub_rn(D.za[a], z1);
-                        D.pos[a] = make_float4(__fadd_rn(D.xa[a], cx), __fadd_rn(D.ya[a], cy), __fadd_rn(D.za[a], cz),
-                                               D.pos[a].w);
-                    }
-                } else {
-                    D.nmovei[nmt + mt]++;
-                    for (int k = 0; k < n; ++k) {
-                        D.xa[a0 + k] = sx[k];
-                        D.ya[a0 + k] = sy[k];
-                        D.za[a0 + k] = sz[k];
+                        const float xk = __fsub_rn(nx[k], x1), yk = __fsub_rn(ny[k], y1), zk = __fsub_rn(nz[k], z1);
+                        D.xa[a] = xk;
+                        D.ya[a] = yk;
+                        D.za[a] = zk;
+                        D.pos[a] = make_float4(__fadd_rn(xk, cx), __fadd_rn(yk, cy), __fadd_rn(zk, cz), D.pos[a].w);
                     }
                 }
+                if (lane == 0) {
+                    D.interntrans[mt] = step;
+                    D.nmovei[mt]++;
+                    if (!acc) D.nmovei[nmt + mt]++;
+                    else if (nn >= 1) D.ergpair[D.ergpairref[row] - 1] = enew;
+                }
+                __syncwarp();
             }
             const int ng = D.ngrot ? D.ngrot[im] : 0;
-            sh_rot = D.has_rot && D.stepri > 0.0f && ng > 0 && (D.rotcycle || D.shake);
-            sh_im = im;
-            sh_n = n;
-            if (sh_rot) {
-                if (D.internrot[mt] == 0.0f) D.internrot[mt] = rotstepmin;
-                D.ninter[mt]++;
-                const int a0 = D.naf[im];
-                for (int k = 0; k < n; ++k) {
-                    sx[k] = D.xa[a0 + k];
-                    sy[k] = D.ya[a0 + k];
-                    sz[k] = D.za[a0 + k];
-                    nx[k] = sx[k];
-                    ny[k] = sy[k];
-                    nz[k] = sz[k];
+            const bool rot = D.has_rot && D.stepri > 0.0f && ng > 0 && (D.rotcycle || D.shake);
+            if (lane == 0) {
+                sh_rot = rot;
+                sh_im = im;
+                sh_n = n;
+            }
+            if (rot) {
+                float step = D.internrot[mt];
+                if (step == 0.0f) step = rotstepmin;
+                for (int k = lane; k < n; k += 32) {
+                    nx[k] = D.xa[a0 + k];
+                    ny[k] = D.ya[a0 + k];
+                    nz[k] = D.za[a0 + k];
                 }
-                const float step = D.internrot[mt];
-                for (int ig = D.rot_nrf[im]; ig <= D.rot_nrl[im]; ++ig) {
-                    const float phi = __fmul_rn(__fmul_rn(pi, step), __fsub_rn(__fmul_rn(2.0f, ran1_next(R)), 1.0f));
-                    const float c = next_cos(D, kcos, phi);
-                    const float sp = fsign(__fsqrt_rn(__fsub_rn(1.0f, __fmul_rn(c, c))), phi);
-                    rotati_d(D, a0, ig, c, sp, nx, ny, nz);
+                __syncwarp();
+                const int g0 = D.rot_nrf[im], g1 = D.rot_nrl[im];
+                for (int ig = g0; ig <= g1; ig += 32) {   // up to 32 groups' angles at a time
+                    const int m = min(32, g1 - ig + 1);
+                    const long long at = R.take(m);
+                    const float phi = __fmul_rn(
+                        __fmul_rn(pi, step), __fsub_rn(__fmul_rn(2.0f, R.get(at + min(lane, m - 1))), 1.0f));
+                    float c, sp;
+                    cosines(m, phi, c, sp);
+                    for (int q = 0; q < m; ++q) {
+                        const float cq = __shfl_sync(0xffffffffu, c, q), sq = __shfl_sync(0xffffffffu, sp, q);
+                        if (lane == 0) rotati_d(D, a0, ig + q, cq, sq, nx, ny, nz);
+                    }
                 }
-                const float cx = D.xadd[im], cy = D.yadd[im], cz = D.zadd[im];
-                for (int k = 0; k < n; ++k) {
-                    D.xa[a0 + k] = nx[k];   // the trial lives in the offsets, as the reference's
-                    D.ya[a0 + k] = ny[k];
-                    D.za[a0 + k] = nz[k];
+                __syncwarp();
+                for (int k = lane; k < n; k += 32)
                     mv[k] = make_float4(__fadd_rn(nx[k], cx), __fadd_rn(ny[k], cy), __fadd_rn(nz[k], cz),
                                         D.pos[a0 + k].w);
+                if (lane == 0) {
+                    D.internrot[mt] = step;
+                    D.ninter[mt]++;
                 }
-            } else if (!D.ngrot || D.ngrot[im] == 0) {
+            } else if (lane == 0 && (!D.ngrot || ng == 0)) {
                 D.internrot[mt] = 0.0f;
             }
         }
         __syncthreads();
         if (sh_rot) {
             const int im = sh_im, n = sh_n;
-            const float fdiff = en_change_mv(im, n);
-            if (tid == 0) {
+            const size_t row = (size_t)im * D.M;
+            const float fdiff = en_change_mv(im, n, true, true);
+            if (wid == 0) {
                 const int mt = D.mtype[im];
-                const int a0 = D.naf[im];
                 // en_change_intra: the new intramolecular energy against ergold(1)
-                const float enew0 = en_mole_intra_d(D.I, im, D.xa, D.ya, D.za);
+                const float enew0 = sh_intra;
                 const float fdiffb = __fsub_rn(enew0, eold0);
                 p0 = enew0;
-                const float ediff = __fmul_rn(__fadd_rn(fdiff, fdiffb), temp);
-                float etest;
-                if (ediff <= 0.0f) etest = 10.0f;
-                else if (ediff < 20.0f) etest = exp_r(-ediff);
-                else etest = 0.0f;
-                const int acc = ran1_next(R) < etest;
-                const size_t row = (size_t)im * D.M;
-                const int nn = D.nergpairm[im];
+                const int acc = accepts(__fmul_rn(__fadd_rn(fdiff, fdiffb), temp), R.get(R.take(1)));
                 if (acc) {
-                    D.nstepreject[im] = 0;
                     fadd = __fadd_rn(fadd, fdiff);
                     faddb = __fadd_rn(faddb, fdiffb);
                     eold0 = enew0;
-                    if (nn >= 1) D.ergpair[D.ergpairref[row] - 1] = enew0;
-                    for (int k = 0; k < n; ++k) D.pos[a0 + k] = mv[k];
-                } else {
-                    D.nstepreject[im]++;
-                    for (int k = 0; k < n; ++k) {
-                        D.xa[a0 + k] = sx[k];
-                        D.ya[a0 + k] = sy[k];
-                        D.za[a0 + k] = sz[k];
-                    }
-                    D.ninter[nmt + mt]++;
                 }
-                sh_acc = acc;
+                if (lane == 0) {
+                    if (acc) {
+                        D.nstepreject[im] = 0;
+                        if (D.nergpairm[im] >= 1) D.ergpair[D.ergpairref[row] - 1] = enew0;
+                    } else {
+                        D.nstepreject[im]++;
+                        D.ninter[nmt + mt]++;
+                    }
+                    sh_acc = acc;
+                }
             }
             __syncthreads();
             if (sh_acc) {
-                const size_t row = (size_t)im * D.M;
-                const int nn = D.nergpairm[im];
+                const int nn = D.nergpairm[im], a0 = D.naf[im];
                 for (int inn = 1 + tid; inn < nn; inn += MC_THREADS) D.ergpair[D.ergpairref[row + inn] - 1] = ergnew[inn];
+                for (int k = tid; k < n; k += MC_THREADS) {
+                    D.xa[a0 + k] = nx[k];
+                    D.ya[a0 + k] = ny[k];
+                    D.za[a0 + k] = nz[k];
+                    D.pos[a0 + k] = mv[k];
+                }
             }
             __syncthreads();
         }
         if (D.shake) continue;   // the intramolecular cycle moves no molecule whole (uniform branch)
         // ---- whole-molecule rotation and translation (molfit.py:362-448)
-        if (tid == 0) {
+        if (wid == 0) {
             const int im = sh_im;
             const int n = sh_n;
             const int a0 = D.naf[im];
             const int mt = D.mtype[im];
-            for (int k = 0; k < n; ++k) {
-                nx[k] = D.xa[a0 + k];
-                ny[k] = D.ya[a0 + k];
-                nz[k] = D.za[a0 + k];
-            }
-            if (D.stepr > 0.0f && n > 1) {
-                if (D.wholerot[mt] <= 0.0f) D.wholerot[mt] = rotstepmin;
-                D.nwhole[mt]++;
-                const float step = D.wholerot[mt];
-                // rotatm: about z, then y, then x (molfit.py:683-710)
-                for (int ax = 0; ax < 3; ++ax) {
-                    float phi = __fmul_rn(__fmul_rn(pi, step), __fsub_rn(__fmul_rn(2.0f, ran1_next(R)), 1.0f));
-                    float c = next_cos(D, kcos, phi);
-                    float sgn = fsign(__fsqrt_rn(__fsub_rn(1.0f, __fmul_rn(c, c))), phi);
-                    for (int k = 0; k < n; ++k) {
-                        if (ax == 0) {
-                            float xs = __fsub_rn(__fmul_rn(nx[k], c), __fmul_rn(ny[k], sgn));
-                            ny[k] = __fadd_rn(__fmul_rn(nx[k], sgn), __fmul_rn(ny[k], c));
-                            nx[k] = xs;
-                        } else if (ax == 1) {
-                            float zs = __fsub_rn(__fmul_rn(nz[k], c), __fmul_rn(nx[k], sgn));
-                            nx[k] = __fadd_rn(__fmul_rn(nz[k], sgn), __fmul_rn(nx[k], c));
-                            nz[k] = zs;
-                        } else {
-                            float ys = __fsub_rn(__fmul_rn(ny[k], c), __fmul_rn(nz[k], sgn));
-                            nz[k] = __fadd_rn(__fmul_rn(ny[k], sgn), __fmul_rn(nz[k], c));
-                            ny[k] = ys;
-                        }
-                    }
-                }
-            } else {
-                D.wholerot[mt] = 0.0f;
-            }
             float cx = D.xadd[im], cy = D.yadd[im], cz = D.zadd[im];
-            if (D.stepm > 0.0f) {
-                if (D.wholetrans[mt] <= 0.0f) D.wholetrans[mt] = D.trstepmin;
-                D.nmovem[mt]++;
-                float st = D.wholetrans[mt];
-                const float xs = cx, ys = cy, zs = cz;
-                cz = __fadd_rn(cz, __fmul_rn(st, __fsub_rn(__fmul_rn(2.0f, ran1_next(R)), 1.0f)));
-                cy = __fadd_rn(cy, __fmul_rn(st, __fsub_rn(__fmul_rn(2.0f, ran1_next(R)), 1.0f)));
-                cx = __fadd_rn(cx, __fmul_rn(st, __fsub_rn(__fmul_rn(2.0f, ran1_next(R)), 1.0f)));
-                while (xs == cx && ys == cy && zs == cz) {
-                    st = __fmul_rn(st, 2.0f);
-                    cz = __fadd_rn(cz, __fmul_rn(st, __fsub_rn(__fmul_rn(2.0f, ran1_next(R)), 1.0f)));
-                    cy = __fadd_rn(cy, __fmul_rn(st, __fsub_rn(__fmul_rn(2.0f, ran1_next(R)), 1.0f)));
-                    cx = __fadd_rn(cx, __fmul_rn(st, __fsub_rn(__fmul_rn(2.0f, ran1_next(R)), 1.0f)));
-                }
-                D.wholetrans[mt] = st;
-            } else {
-                D.wholetrans[mt] = 0.0f;
+            const bool turns = D.stepr > 0.0f && n > 1;
+            float rstep = D.wholerot[mt], tstep = D.wholetrans[mt];
+            float c = 1.0f, sgn = 0.0f;
+            if (turns) {
+                // rotatm: about z, then y, then x (molfit.py:683-710)
+                if (rstep <= 0.0f) rstep = rotstepmin;
+                const long long at = R.take(3);
+                const float phi = __fmul_rn(__fmul_rn(pi, rstep),
+                                            __fsub_rn(__fmul_rn(2.0f, R.get(at + min(lane, 2))), 1.0f));
+                cosines(3, phi, c, sgn);
             }
-            for (int k = 0; k < n; ++k)
-                mv[k] = make_float4(__fadd_rn(nx[k], cx), __fadd_rn(ny[k], cy), __fadd_rn(nz[k], cz),
-                                    D.pos[a0 + k].w);
-            sh_cx = cx;
-            sh_cy = cy;
-            sh_cz = cz;
+            const float c0 = __shfl_sync(0xffffffffu, c, 0), c1 = __shfl_sync(0xffffffffu, c, 1),
+                        c2 = __shfl_sync(0xffffffffu, c, 2), s0 = __shfl_sync(0xffffffffu, sgn, 0),
+                        s1 = __shfl_sync(0xffffffffu, sgn, 1), s2 = __shfl_sync(0xffffffffu, sgn, 2);
+            if (D.stepm > 0.0f) {
+                if (tstep <= 0.0f) tstep = D.trstepmin;
+                const float xs = cx, ys = cy, zs = cz;
+                bool again = false;
+                do {
+                    if (again) tstep = __fmul_rn(tstep, 2.0f);
+                    const long long at = R.take(3);
+                    cz = __fadd_rn(cz, __fmul_rn(tstep, __fsub_rn(__fmul_rn(2.0f, R.get(at)), 1.0f)));
+                    cy = __fadd_rn(cy, __fmul_rn(tstep, __fsub_rn(__fmul_rn(2.0f, R.get(at + 1)), 1.0f)));
+                    cx = __fadd_rn(cx, __fmul_rn(tstep, __fsub_rn(__fmul_rn(2.0f, R.get(at + 2)), 1.0f)));
+                    again = true;
+                } while (xs == cx && ys == cy && zs == cz);
+            }
+            for (int k = lane; k < n; k += 32) {
+                float x = D.xa[a0 + k], y = D.ya[a0 + k], z = D.za[a0 + k];
+                if (turns) {
+                    const float xr = __fsub_rn(__fmul_rn(x, c0), __fmul_rn(y, s0));
+                    y = __fadd_rn(__fmul_rn(x, s0), __fmul_rn(y, c0));
+                    x = xr;
+                    const float zr = __fsub_rn(__fmul_rn(z, c1), __fmul_rn(x, s1));
+                    x = __fadd_rn(__fmul_rn(z, s1), __fmul_rn(x, c1));
+                    z = zr;
+                    const float yr = __fsub_rn(__fmul_rn(y, c2), __fmul_rn(z, s2));
+                    z = __fadd_rn(__fmul_rn(y, s2), __fmul_rn(z, c2));
+                    y = yr;
+                }
+                nx[k] = x;
+                ny[k] = y;
+                nz[k] = z;
+                mv[k] = make_float4(__fadd_rn(x, cx), __fadd_rn(y, cy), __fadd_rn(z, cz), D.pos[a0 + k].w);
+            }
+            if (lane == 0) {
+                if (turns) {
+                    D.wholerot[mt] = rstep;
+                    D.nwhole[mt]++;
+                } else {
+                    D.wholerot[mt] = 0.0f;
+                }
+                if (D.stepm > 0.0f) {
+                    D.wholetrans[mt] = tstep;
+                    D.nmovem[mt]++;
+                } else {
+                    D.wholetrans[mt] = 0.0f;
+                }
+                sh_cx = cx;
+                sh_cy = cy;
+                sh_cz = cz;
+            }
         }
         __syncthreads();
         const int im = sh_im, n = sh_n;
         const size_t row = (size_t)im * D.M;
         const int nn = D.nergpairm[im];
-        const float fdiff = en_change_mv(im, n);
-        if (tid == 0) {
+        const float fdiff = en_change_mv(im, n, !sh_rot, false);
+        if (wid == 0) {
             const int mt = D.mtype[im];
-            const float ediff = __fmul_rn(__fadd_rn(fdiff, 0.0f), temp);
-            float etest;
-            if (ediff <= 0.0f) etest = 10.0f;
-            else if (ediff < 20.0f) etest = exp_r(-ediff);
-            else etest = 0.0f;
-            const int acc = ran1_next(R) < etest;
+            const int acc = accepts(__fmul_rn(__fadd_rn(fdiff, 0.0f), temp), R.get(R.take(1)));
             if (acc) {
-                D.nstepreject[im] = 0;
                 fadd = __fadd_rn(fadd, fdiff);
-                // save_energies copies every slot, the first one included: after an internal
-                // rotation of this visit it holds the rotation's intramolecular energy even when
-                // that rotation was rejected (molfit.py:215, :419; ergpairreference.py:192-210)
-                if (sh_rot) {
-                    eold0 = p0;
-                    if (nn >= 1) D.ergpair[D.ergpairref[row] - 1] = p0;
-                }
-            } else {
-                D.nstepreject[im]++;
-                if (D.stepr > 0.0f) D.nwhole[nmt + mt]++;
-                if (D.stepm > 0.0f) D.nmovem[nmt + mt]++;
+                if (sh_rot) eold0 = p0;
             }
-            if (D.trace_den) D.trace_den[v] = fdiff;
-            if (D.trace_acc) D.trace_acc[v] = acc;
-            sh_acc = acc;
+            if (lane == 0) {
+                if (acc) {
+                    D.nstepreject[im] = 0;
+                    // save_energies copies every slot, the first one included: after an internal
+                    // rotation of this visit it holds the rotation's intramolecular energy even when
+                    // that rotation was rejected (molfit.py:215, :419; ergpairreference.py:192-210)
+                    if (sh_rot && nn >= 1) D.ergpair[D.ergpairref[row] - 1] = p0;
+                } else {
+                    D.nstepreject[im]++;
+                    if (D.stepr > 0.0f) D.nwhole[nmt + mt]++;
+                    if (D.stepm > 0.0f) D.nmovem[nmt + mt]++;
+                }
+                if (D.trace_den) D.trace_den[v] = fdiff;
+                if (D.trace_acc) D.trace_acc[v] = acc;
+                sh_acc = acc;
+            }
         }
         __syncthreads();
         if (sh_acc) {
@@ -506,9 +649,8 @@ __global__ void __launch_bounds__(MC_THREADS) molfit_seq_kernel(McDev D) {
         }
         D.fadds[0] = __fadd_rn(D.fadds[0], __fdiv_rn(fadd, (float)D.nmol));
         if (D.faddbs) D.faddbs[0] = __fadd_rn(D.faddbs[0], __fdiv_rn(faddb, (float)D.nmol));
-        ran1_store(R, D.ran1);
+        R.finish(D.ran1);
     }
-    (void)sh_fdiff;
 }
 
 // en_change for one molecule at its current coordinates (no move)
@@ -709,10 +851,15 @@ static int seq_launch(const epsr_box_t *box, const epsr_cells_t *cells, epsr_sto
         D.visit = nullptr;
     }
     const size_t need = sizeof(float) * 2 * (size_t)(D.M > 0 ? D.M : 1);
+    D.rcp = step_rcp(D.T.stepcl, D.T.izcut);
+    // the staging takes what the list's energies leave of 190 KB: four bytes a pair value and two
+    // an item, 64 x 64 values at least
     size_t shm = 0;
     if (need <= 160 * 1024) {
         D.use_smem = 1;
-        shm = need;
+        D.ev = (int)((190 * 1024 - need) / 6) & ~1023;
+        D.ev = D.ev > 24576 ? 24576 : D.ev;
+        shm = need + 6 * (size_t)D.ev;
     } else {
         if (!scratch || scratch_bytes < (int64_t)need) {
             epsr_set_error("epsr_molfit: scratch needs %zu bytes", need);
@@ -720,9 +867,10 @@ static int seq_launch(const epsr_box_t *box, const epsr_cells_t *cells, epsr_sto
         }
         D.use_smem = 0;
         D.ergnew_g = (float *)scratch;
+        D.ev = 24576;
+        shm = 6 * (size_t)D.ev;
     }
-    if (shm > 48 * 1024)
-        EPSR_SMEM_OPTIN(molfit_seq_kernel);
+    EPSR_SMEM_OPTIN(molfit_seq_kernel);
     EPSR_TIMED("molfit_seq_kernel", s, molfit_seq_kernel<<<1, MC_THREADS, shm, s>>>(D));
     EPSR_CUDA(cudaGetLastError());
     return EPSR_OK;
