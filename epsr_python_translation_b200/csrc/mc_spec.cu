@@ -34,7 +34,7 @@
 // mc.cu).  The rare translation retry of movem (a move that leaves the centre unchanged
 // doubles the step and draws again, molfit.py:752-758) shifts every later draw; the cycle is
 // then discarded and the sequential kernel runs it instead, from the unchanged state.
-#include "common.cuh"
+#include "ran1_pair.cuh"
 #include "umma.cuh"
 
 namespace epsr {
@@ -82,8 +82,6 @@ struct SpecDev {
     int32_t *ran1_next;                    // [35]
     float *draws;
     int32_t *ahead;                        // the draws-ahead buffer (AH_* words), or NULL
-    const float *ahead_vals;               // the draws-ahead values, or NULL
-    const int32_t *use_ahead;              // [1] 1: this cycle reads ahead_vals (NULL: never)
     float *nx, *ny, *nz;                   // [natom] proposed offsets
     float4 *nc;                            // [N] proposed centres (by molecule)
     float4 *npos;                          // [natom] proposed absolute positions
@@ -208,12 +206,10 @@ __global__ void spec_plan_kernel(SpecDev S) {
         }
     }
     __syncthreads();   // off[N], the cycle's draw count
-    if (tid >= 32) return;
     // the cycle's ran1 values, from a copy of the state (a discarded cycle leaves the real state
     // untouched): the draws ahead when the previous cycle left them for exactly this state and
-    // count, else walked here by this warp
-    const int lane = tid;
-    for (int i = lane; i < 35; i += 32) S.ran1_next[i] = S.ran1[i];
+    // count, else walked here by the first two warps
+    const int lane = tid & 31;
     const int32_t count = S.off[S.N];
     bool ok = false;
     if (S.ahead) {
@@ -221,32 +217,30 @@ __global__ void spec_plan_kernel(SpecDev S) {
         if (lane < 3) same = same && S.ahead[AH_START + 32 + lane] == S.ran1[32 + lane];
         ok = __all_sync(0xffffffffu, same) && S.ahead[AH_VALID] == 1 && S.ahead[AH_COUNT] == count;
     }
-    __syncwarp();
-    if (ok) {
-        S.ran1_next[lane] = S.ahead[AH_END + lane];
-        if (lane < 3) S.ran1_next[32 + lane] = S.ahead[AH_END + 32 + lane];
+    if (tid < 32) {
+        for (int i = lane; i < 35; i += 32) S.ran1_next[i] = ok ? S.ahead[AH_END + i] : S.ran1[i];
+        if (lane == 0) {
+            S.flags[2] = ok ? 0 : count;
+            S.flags[3] = ok ? 1 : 0;
+            if (ok) S.ahead[AH_USES] += 1;
+        }
     }
-    if (lane == 0) {
-        S.flags[2] = ok ? 0 : count;
-        S.flags[3] = ok ? 1 : 0;
-        if (ok) S.ahead[AH_USES] += 1;
+    if (ok) {   // into the cycle's own buffer: the next draws ahead may start at once
+        const int32_t *from = S.ahead + AH_VALS;
+        int32_t *to = reinterpret_cast<int32_t *>(S.draws);
+        const int quads = ((uintptr_t)from & 15) == 0 ? count / 4 : 0;
+#pragma unroll 4
+        for (int i = tid; i < quads; i += blockDim.x)
+            reinterpret_cast<int4 *>(to)[i] = reinterpret_cast<const int4 *>(from)[i];
+        for (int i = 4 * quads + tid; i < count; i += blockDim.x) to[i] = from[i];
     }
-    __syncwarp();
-    if (ok || count == 0) return;
+    if (ok || count == 0 || tid >= 64) return;
+    __shared__ R1Ring ring;
     __shared__ int32_t tab[34];
+    const int32_t mcall = S.ran1[2];
     Ran1Warp g;
-    g.load(S.ran1_next);
-    const int32_t mcall = S.ran1_next[2];
-    __syncwarp();
-    int64_t done = 0;
-    while (done < count) {
-        const int64_t left = count - done;
-        int32_t mine;
-        const int cnt = g.next(left > 32 ? 32 : (int)left, mine, tab);
-        if (lane < cnt) S.draws[done + lane] = ran1_out(mine);
-        done += cnt;
-    }
-    __syncwarp();
+    r1_fill(ring, tab, S.ran1, count, g, [&](int64_t i, int32_t v) { S.draws[i] = ran1_out(v); });
+    if (tid >= 32) return;
     S.ran1_next[3 + lane] = g.iv;
     if (lane == 0) {
         S.ran1_next[0] = g.idum;
@@ -282,7 +276,7 @@ __global__ void spec_propose_kernel(SpecDev S) {
     }
     const int a0 = S.naf[m];
     const int t = S.mtype[m];
-    const float *u = (S.use_ahead && *S.use_ahead ? S.ahead_vals : S.draws) + S.off[k];
+    const float *u = S.draws + S.off[k];
     int q = 0;
     float x[SP_MAXAT], y[SP_MAXAT], z[SP_MAXAT];
     for (int i = 0; i < n; ++i) {
@@ -1229,27 +1223,23 @@ namespace epsr {
 // between, the cycle was redone by the sequential kernel, the caller set a new state) it
 // walks the stream itself.  Either way it draws the same values.
 
-__global__ void ahead_fill_kernel(const int32_t *state, int32_t *ahead, const int32_t *count) {
-    const int lane = threadIdx.x;
+__global__ void __launch_bounds__(64) ahead_fill_kernel(const int32_t *state, int32_t *ahead, const int32_t *count) {
+    __shared__ R1Ring ring;
     __shared__ int32_t tab[34];
+    const int lane = threadIdx.x & 31;
     const int64_t n = *count;
-    if (lane == 0) ahead[AH_VALID] = 0;
-    ahead[AH_START + lane] = state[lane];
-    if (lane < 3) ahead[AH_START + 32 + lane] = state[32 + lane];
-    Ran1Warp g;
-    g.load(state);
-    const int32_t mcall = state[2];
-    float *out = reinterpret_cast<float *>(ahead + AH_VALS);
-    __syncwarp();
-    int64_t done = 0;
-    while (done < n) {
-        const int64_t left = n - done;
-        int32_t mine;
-        const int cnt = g.next(left > 32 ? 32 : (int)left, mine, tab);
-        if (lane < cnt) out[done + lane] = ran1_out(mine);
-        done += cnt;
+    if (threadIdx.x < 32) {
+        if (lane == 0) ahead[AH_VALID] = 0;
+        ahead[AH_START + lane] = state[lane];
+        if (lane < 3) ahead[AH_START + 32 + lane] = state[32 + lane];
     }
+    const int32_t mcall = state[2];
+    Ran1Warp g;
+    float *out = reinterpret_cast<float *>(ahead + AH_VALS);
+    r1_fill(ring, tab, state, n, g, [&](int64_t i, int32_t v) { out[i] = ran1_out(v); });
+    if (threadIdx.x >= 32) return;
     ahead[AH_END + 3 + lane] = g.iv;
+    __syncwarp();
     if (lane == 0) {
         ahead[AH_END + 0] = g.idum;
         ahead[AH_END + 1] = g.iy;
@@ -1276,7 +1266,9 @@ static int ahead_stream(AheadStream **out) {
     if (!g_ahead_smem) {
         int optin = 0;
         EPSR_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-        g_ahead_smem = (size_t)optin - 256;   // room for the kernel's own static table
+        cudaFuncAttributes fa;
+        EPSR_CUDA(cudaFuncGetAttributes(&fa, ahead_fill_kernel));
+        g_ahead_smem = (size_t)optin - fa.sharedSizeBytes;   // all of it: the kernel's own ring and table have the rest
     }
     if (dev < 0 || dev >= 16) {
         epsr_set_error("epsr_molfit: device ordinal %d beyond the draws-ahead table", dev);
@@ -1459,18 +1451,15 @@ int epsr_molfit_spec(const epsr_box_t *box, const epsr_cells_t *cells, epsr_stor
 
     // draws ahead: only with a buffer that holds a whole cycle's values (at most 7 a move)
     const bool ahead = mc->ahead && mc->ahead_cap >= (int64_t)N * 7;
-    int32_t *use = S.flags + 3;
-    if (ahead) {
-        S.ahead_vals = reinterpret_cast<const float *>(mc->ahead + AH_VALS);
-        S.use_ahead = use;
-    }
     if (ahead) S.ahead = mc->ahead;
     int rc = EPSR_OK;
     EPSR_TIMED("spec_plan_kernel", s, spec_plan_kernel<<<1, 1024, 0, s>>>(S));
     EPSR_CUDA(cudaGetLastError());
-    EPSR_TIMED("spec_propose_kernel", s, spec_propose_kernel<<<(max(N, S.nedge) + 127) / 128, 128, 0, s>>>(S));
     // the next cycle's values, from the state after this cycle's draws, on the second stream
-    // once nothing of this cycle reads the buffer any more; joined before this call returns
+    // once nothing of this cycle reads the buffer any more; joined before this call returns.  It
+    // is launched before the wide passes: it takes an SM to itself, and behind the energy pass,
+    // whose CTAs wait for every SM, it began only when that pass was over (20,000 water: 0.49 ms
+    // later, and the walk ended 0.3 ms after everything else of the cycle).
     AheadStream *as = nullptr;
     if (ahead) {
         rc = ahead_stream(&as);
@@ -1482,10 +1471,11 @@ int epsr_molfit_spec(const epsr_box_t *box, const epsr_cells_t *cells, epsr_stor
         // the SM to itself for the 2-3 ms it runs
         EPSR_SMEM_OPTIN(ahead_fill_kernel);
         EPSR_TIMED("ahead_fill_kernel", as->st,
-                   ahead_fill_kernel<<<1, 32, g_ahead_smem, as->st>>>(S.ran1_next, mc->ahead, S.off + N));
+                   ahead_fill_kernel<<<1, 64, g_ahead_smem, as->st>>>(S.ran1_next, mc->ahead, S.off + N));
         EPSR_CUDA(cudaGetLastError());
         EPSR_CUDA(cudaEventRecord(as->join, as->st));
     }
+    EPSR_TIMED("spec_propose_kernel", s, spec_propose_kernel<<<(max(N, S.nedge) + 127) / 128, 128, 0, s>>>(S));
     {
         const int ma = box->maxat > 0 && box->maxat <= SP_MAXAT ? box->maxat : SP_MAXAT;
         S.ev = max(2 * ma * ma, 4096);
