@@ -6,49 +6,52 @@
 // launch fits any number of data sets in turn on the same basis, continuing one ran1
 // stream, as the reference's successive calls do.
 //
-// Layout.  The basis rows are split over the CTAs of a cluster; each keeps its rows in
-// shared memory for the whole launch, four terms to a 16-byte word, except the first 64
-// terms of each row, which its thread holds in registers; a thread evaluates its row per
-// trial (expand :4924, the sequential clamped sum of a row).  Every partial
+// Layout.  The basis rows are split over the CTAs of a cluster; a thread evaluates its row per
+// trial (expand :4924, the sequential clamped sum of a row) with the row's first 128 terms in its
+// registers (64 in the wide form of the CTA) and the rest in shared memory, four terms to a
+// 16-byte word.  Every partial
 // sum of a row is bounded by the row's L1 norm times the largest |coefficient|; when that
 // bound stays below the clamp level (e^25) the clamp cannot act and the plain sequential
 // sum is the reference's value, otherwise the row is summed with the clamp.  The CTAs
-// exchange their chi^2 contributions through distributed shared memory: each pushes its
+// exchange their chi^2 contributions through distributed shared memory: each stores its
 // part (a double partial, or every residual for the reference's sequential float sum) into
-// every CTA and arrives on that CTA's mbarrier; each then forms the same chi^2, so all take
+// every CTA, the stores completing their bytes on that CTA's mbarrier (no release stands between a
+// store and its signal); each then forms the same chi^2, so all take
 // the same decisions without a second exchange.  Thread 0 of each CTA takes every decision
 // (Metropolis test, smoothing, stopping) and broadcasts it through shared memory, so all
-// threads pass the same barriers.
+// threads pass the same barriers.  The strict sum is one chain of additions over all rows, 4.7
+// cycles each (1,000 rows x 97 terms: 21,700 cycles a trial when every fourth row waited for its
+// word, 8,400 now).
 //
-// ran1.  The chain is sequential; warp 15 of every CTA generates the same stream into a
-// ring in its CTA's shared memory, running ahead of the trials (bounded by the ring) and
-// publishing how many values exist.  Rows and coefficients are handled by the warps of the
-// other three schedulers of the SM (warps 0-2, 4-6, 8-10, 12-14), so the generator's
-// scheduler is left to it; warps 3, 7 and 11 only take part in the barriers.  The workers
-// synchronise among themselves with a named barrier that the generator warp is not part of.
-// At the end the state the reference leaves after exactly the values the fit consumed is
-// rebuilt from the generator's per-batch checkpoints.
+// ran1.  The chain is sequential and one trial's values outlast one trial's arithmetic, so it has
+// an SM to itself: the cluster's last CTA generates the stream with two warps (ran1_pair.cuh) and
+// stores the values into a ring in every worker CTA's shared memory, running ahead of the trials
+// (bounded by the ring).  On a warp of each worker CTA, beside its rows' shared-memory reads, the
+// same chain took 46 cycles a value instead of 29.  At the end the state the reference leaves after
+// exactly the values the fit consumed is rebuilt from the generator's checkpoints.
 //
 // Every wait (ring, exchange, ring space) is bounded in time: on timeout the kernel records
 // status 1, stops the fit and returns.
 #include <cooperative_groups.h>
 
-#include "common.cuh"
+#include <algorithm>
+
+#include "ran1_pair.cuh"
 
 namespace cg = cooperative_groups;
 
 namespace epsr {
 
-constexpr int FX_THREADS = 512;
-constexpr int FX_WARPS = FX_THREADS / 32;
-constexpr int FX_GEN_WARP = 15;                 // the stream warp
-constexpr int FX_NBAR = 480;                    // threads of the worker barrier (warps 0-14)
-constexpr int FX_SLOTS = 384;                   // row / coefficient slots (12 warps, schedulers 0-2)
-constexpr int FX_RQ = 16;                       // leading quads of a row held in its thread's registers
+constexpr int FX_MAXT = 512;                    // most threads of a worker CTA (256 when rows and terms fit)
+constexpr int FX_WARPS = FX_MAXT / 32;
+constexpr int FX_SLOTS = FX_MAXT;               // row / coefficient slots of a worker CTA at most
+constexpr int FX_ROWS = 160;                    // rows a CTA takes while the cluster has CTAs left
+constexpr int FX_MAXW = 8;                      // worker CTAs of a cluster
+// leading quads of a row held in its thread's registers: the narrow CTA has room for 128 terms
+__host__ __device__ constexpr int fx_rq(int threads) { return threads == FX_MAXT ? 16 : 32; }
 constexpr int FX_RING = 2048;                   // ran1 values held per worker CTA (power of two)
-constexpr int FX_CK = 128;                      // generator checkpoints (power of two)
+constexpr int FX_CK = 32;                       // generator checkpoints (power of two)
 constexpr int FX_CKE = 8;                       // batches between checkpoints (power of two)
-constexpr int FX_GB = 4;                        // generator batches between reads of the control words
 constexpr int FX_CKW = 36;                      // ints per checkpoint: idum, iy, iv[32], pad[2]
 constexpr unsigned long long FX_WAIT_NS = 2000000000ull;  // a wait gives up after 2 s
 
@@ -60,7 +63,7 @@ struct FxDev {
     float *scal;              // [nprob][4] {stepr, acceptr, rejrat, chisq}
     long long *trials;        // [nprob]
     int *status;              // [1]: 0 ok, 1 a bounded wait gave up
-    int nprob, nmin, npt, ncfirst, nterms, nits, nfreq, strict, rpc;
+    int nprob, nmin, npt, ncfirst, nterms, nits, nfreq, strict, rpc, nw;
     int32_t *ran1;
 };
 
@@ -71,41 +74,28 @@ __device__ __forceinline__ uint32_t map_rank(uint32_t a, uint32_t rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
     return r;
 }
-__device__ __forceinline__ void st_cl_f32(uint32_t a, float v) {
-    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+// a store into another CTA of the cluster that completes its bytes on that CTA's mbarrier
+__device__ __forceinline__ void st_async_f32(uint32_t a, float v, uint32_t bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(a),
+                 "r"(__float_as_int(v)), "r"(bar)
+                 : "memory");
 }
-__device__ __forceinline__ void st_cl_f64(uint32_t a, double v) {
-    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+__device__ __forceinline__ void st_async_f64(uint32_t a, double v, uint32_t bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(a),
+                 "l"(__double_as_longlong(v)), "r"(bar)
+                 : "memory");
 }
 __device__ __forceinline__ void st_cl_s64(uint32_t a, long long v) {
     asm volatile("st.shared::cluster.b64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
 }
-__device__ __forceinline__ void st_release_cl_s64(uint32_t a, long long v) {
-    asm volatile("st.release.cluster.shared::cluster.b64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
-}
 __device__ __forceinline__ void st_release_cl_s32(uint32_t a, int v) {
     asm volatile("st.release.cluster.shared::cluster.b32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
-}
-__device__ __forceinline__ long long ld_relaxed_cl_s64(uint32_t a) {
-    long long v;
-    asm volatile("ld.relaxed.cluster.shared::cluster.b64 %0, [%1];" : "=l"(v) : "r"(a) : "memory");
-    return v;
-}
-__device__ __forceinline__ long long ld_acquire_s64(const long long *p) {
-    long long v;
-    asm volatile("ld.acquire.cluster.shared::cta.b64 %0, [%1];" : "=l"(v) : "r"(smem_addr(p)) : "memory");
-    return v;
-}
-__device__ __forceinline__ int ld_acquire_s32(const int *p) {
-    int v;
-    asm volatile("ld.acquire.cluster.shared::cta.b32 %0, [%1];" : "=r"(v) : "r"(smem_addr(p)) : "memory");
-    return v;
 }
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory");
 }
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t a) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(a) : "memory");
+__device__ __forceinline__ void mbar_expect(uint64_t *bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ bool mbar_test(uint32_t a, uint32_t parity) {
     uint32_t ok;
@@ -118,13 +108,12 @@ __device__ __forceinline__ bool mbar_test(uint32_t a, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-__device__ __forceinline__ void fence_cluster() { asm volatile("fence.acq_rel.cluster;" ::: "memory"); }
-// Barrier of the worker warps (0-14) after code in which a warp may have diverged (a
-// bounded spin, a branch on the thread index): the warp is reconverged first, because the
-// barrier requires every thread of a warp to arrive together.
+// Barrier of a worker CTA after code in which a warp may have diverged (a bounded spin, a branch
+// on the thread index): the warp is reconverged first, because the barrier requires every thread
+// of a warp to arrive together.
 __device__ __forceinline__ void block_sync() {
     __syncwarp();
-    asm volatile("bar.sync 1, %0;" ::"n"(FX_NBAR) : "memory");
+    __syncthreads();
 }
 __device__ __forceinline__ unsigned long long now_ns() {
     unsigned long long t;
@@ -133,8 +122,8 @@ __device__ __forceinline__ unsigned long long now_ns() {
 }
 
 struct FxShared {                 // statically sized control block (one per CTA)
-    long long cons;               // lowest stream index the workers may still read
-    int done;                     // set by the workers when the fit is over
+    long long cons;               // generator: lowest stream index the workers may still read
+    int done;                     // generator: set by the workers when the fit is over
     int abort, stop;
     int accept, smooth, draw;     // thread 0's decision of the current trial
     float val;                    // chi^2 broadcast
@@ -143,21 +132,24 @@ struct FxShared {                 // statically sized control block (one per CTA
     double red[FX_WARPS];
 };
 
-__host__ __device__ inline int fx_ntq(int nt) { return (nt + 3) / 4; }
-// quads of a row kept in shared memory (those after the first FX_RQ)
-__host__ __device__ inline int fx_nsq(int nt) { return fx_ntq(nt) > FX_RQ ? fx_ntq(nt) - FX_RQ : 0; }
+// quads of a row, in whole groups of four (terms past nterms are zero on both sides)
+__host__ __device__ inline int fx_ntq(int nt) { return (nt + 15) / 16 * 4; }
+// quads of a row kept in shared memory (those after the registers')
+__host__ __device__ inline int fx_nsq(int nt, int threads) {
+    return fx_ntq(nt) > fx_rq(threads) ? fx_ntq(nt) - fx_rq(threads) : 0;
+}
 // floats per exchange buffer: every row of the cluster, padded to whole 16-byte words so the
 // second buffer starts 16-byte aligned (it is read four rows at a time)
 __host__ __device__ inline int fx_gstride(int nw, int rpc) { return (nw * rpc + 3) & ~3; }
 
-size_t fx_smem_bytes(int nt, int rpc, int nw) {
+size_t fx_smem_bytes(int nt, int rpc, int nw, int threads) {
     const int ntq = fx_ntq(nt);
     size_t b = 0;
-    b += 16 * (size_t)fx_nsq(nt) * rpc;                 // ex4
+    b += 16 * (size_t)fx_nsq(nt, threads) * rpc;                 // ex4
     b += sizeof(float) * (size_t)rpc;                   // yr
     b += sizeof(float) * (size_t)rpc;                   // e1 (row L1 norms)
     b = (b + 15) & ~(size_t)15;
-    b += sizeof(float) * (4 + 4 * (size_t)ntq);         // wt (wt + 1 16-byte aligned)
+    b += sizeof(float) * (4 + 4 * ((size_t)ntq + 4));   // wt (wt + 1 16-byte aligned, a group past the end)
     b += sizeof(float) * (size_t)(nt + 1);              // wtold
     b = (b + 15) & ~(size_t)15;
     b += sizeof(unsigned long long) * FX_RING;          // ring
@@ -166,27 +158,161 @@ size_t fx_smem_bytes(int nt, int rpc, int nw) {
     b = (b + 15) & ~(size_t)15;
     b += sizeof(double) * 2 * (size_t)nw;               // parts[2][nw]
     b += sizeof(uint64_t) * 2;                          // exchange mbarriers
-    b += sizeof(long long) * FX_CK;                     // ckpos
-    b += sizeof(int32_t) * FX_CK * FX_CKW;              // checkpoints
     return b;
 }
 
-__global__ void __launch_bounds__(FX_THREADS, 1) fitexp_cluster_kernel(FxDev F) {
+struct FxGen {                    // the generator CTA's shared memory
+    R1Ring pair;
+    int32_t tab[34];
+    long long ckpos[FX_CK];
+    int32_t ck[FX_CK][FX_CKW];    // idum, iy, iv[32] before a batch
+    int first, go;
+};
+
+// The generator CTA: values 0, 1, ... of the stream into the workers' rings until they are done,
+// then the state after the values they took.  Warps 0 and 1 call.
+__device__ void fx_generate(const FxDev &F, FxGen &G, FxShared &S, unsigned long long *ring) {
+    const int lane = threadIdx.x & 31;
+    if (threadIdx.x >= 32) {
+        asm volatile("bar.sync 7, 64;" ::: "memory");
+        if (*(volatile int *)&G.go) r1_walk(G.pair, G.pair.tab[lane] >> 26, *(volatile int *)&G.first, 0x7fffffff);
+        return;
+    }
+    volatile FxShared *vs = &S;
+    Ran1Warp g;
+    g.load(F.ran1);
+    const int32_t mcall0 = F.ran1[2];
+    long long pos = 0, nb = 0;
+    uint32_t dst[FX_MAXW];
+#pragma unroll
+    for (int d = 0; d < FX_MAXW; ++d) dst[d] = d < F.nw ? map_rank(smem_addr(ring), (uint32_t)d) : 0u;
+    auto push = [&](int cnt, int32_t mine) {
+        const long long q = pos + lane;
+        const long long w = (long long)(((unsigned long long)(uint32_t)(q + 1) << 32) |
+                                        (unsigned long long)__float_as_uint(ran1_out(mine)));
+        if (lane < cnt)
+#pragma unroll
+            for (int d = 0; d < FX_MAXW; ++d)
+                if (d < F.nw) st_cl_s64(dst[d] + 8u * (uint32_t)(q & (FX_RING - 1)), w);
+        pos += cnt;
+    };
+    auto checkpoint = [&](int32_t idum, int32_t iy, int32_t iv) {   // the state before a batch
+        if ((nb++ & (FX_CKE - 1)) == 0) {
+            const int slot = (int)(((nb - 1) / FX_CKE) & (FX_CK - 1));
+            G.ck[slot][2 + lane] = iv;
+            if (lane == 0) {
+                G.ck[slot][0] = idum;
+                G.ck[slot][1] = iy;
+                G.ckpos[slot] = pos;
+            }
+        }
+    };
+    // room for a batch in every ring; false when the workers are done (or gave up: 2 s without room)
+    auto room = [&]() -> bool {
+        unsigned long long t0 = 0;
+        while (true) {
+            __syncwarp();
+            if (vs->done) return false;
+            if (vs->cons + FX_RING - pos >= 32) return true;
+            int give_up = 0;
+            if (lane == 0) {
+                const unsigned long long t = now_ns();
+                if (t0 == 0) t0 = t;
+                else if (t - t0 > FX_WAIT_NS) {
+                    atomicExch(F.status, 1);
+                    give_up = 1;
+                }
+            }
+            if (__shfl_sync(0xffffffffu, give_up, 0)) return false;
+            __nanosleep(64);
+        }
+    };
+    for (int i = lane; i < FX_CK; i += 32) G.ckpos[i] = -1;
+    __syncwarp();
+    bool more = true;
+    // until the stream is clean: one batch as a rule (the initialisation happens inside); a
+    // degenerate stream stays here
+    while (more && !(g.clean && g.idum > 0)) {
+        more = room();
+        if (!more) break;
+        checkpoint(g.idum, g.iy, g.iv);
+        int32_t mine;
+        const int cnt = g.next(32, mine, G.tab);
+        push(cnt, mine);
+    }
+    G.pair.tab[lane] = g.iv;
+    if (lane == 0) {
+        r1_init(G.pair);
+        *(volatile int *)&G.first = g.iy >> 26;
+        *(volatile int *)&G.go = more;
+    }
+    __syncwarp();
+    asm volatile("bar.sync 7, 64;" ::: "memory");
+    if (more) {
+        R1Values v;
+        v.begin(G.pair, g);
+        constexpr int A = R1_NB / 2;   // batches made ahead
+#pragma unroll
+        for (int j = 0; j < A; ++j) v.make(G.pair, j);
+        for (int b = 0; more; b += A) {
+#pragma unroll
+            for (int j = 0; j < A; ++j) {
+                if (!more) continue;
+                more = room();
+                if (!more) continue;
+                if (!v.walked(G.pair, b + j)) {
+                    if (lane == 0) atomicExch(F.status, 1);
+                    more = false;
+                    continue;
+                }
+                checkpoint(v.idum, v.iy, G.pair.tab[lane]);
+                push(32, v.take(G.pair, b + j, j));
+                v.make(G.pair, j);
+            }
+        }
+        v.leave(G.pair);
+    }
+    // the state after exactly the values taken, from the last checkpoint at or before it (or from
+    // the launch's state when none is left)
+    __syncwarp();
+    if (lane == 0 && vs->done == 1) {
+        const long long cursor = vs->cons;
+        int best = -1;
+        for (int k = 0; k < FX_CK; ++k)
+            if (G.ckpos[k] >= 0 && G.ckpos[k] <= cursor && (best < 0 || G.ckpos[k] > G.ckpos[best])) best = k;
+        Ran1 R;
+        long long from = 0;
+        ran1_load(R, F.ran1);
+        if (best >= 0) {
+            R.idum = G.ck[best][0];
+            R.iy = G.ck[best][1];
+            for (int i = 0; i < 32; ++i) R.iv[i] = G.ck[best][2 + i];
+            from = G.ckpos[best];
+        }
+        for (long long k = from; k < cursor; ++k) ran1_next(R);
+        R.mcall = (int32_t)((uint32_t)mcall0 + (uint32_t)cursor);
+        ran1_store(R, F.ran1);
+    }
+}
+
+template <int T>
+__global__ void __launch_bounds__(T, 1) fitexp_cluster_kernel(FxDev F) {
     cg::cluster_group cl = cg::this_cluster();
     const int rank = (int)cl.block_rank();
-    const int nw = (int)cl.num_blocks();
+    const int nw = F.nw;                                // worker CTAs; rank nw generates
     extern __shared__ __align__(16) unsigned char fx_raw[];
     __shared__ FxShared S;
-    __shared__ int32_t g_tab[34];
+    __shared__ FxGen G;
     const int nt = F.nterms, rpc = F.rpc, ntq = fx_ntq(nt);
-    const int nsq = fx_nsq(nt);
+    constexpr int FX_RQ = fx_rq(T);
+    const int nsq = fx_nsq(nt, T);
     // [nsq*rpc]: ex4[q*rpc + r] = terms 4(FX_RQ+q)..4(FX_RQ+q)+3 of row r
     float4 *ex4 = (float4 *)fx_raw;
     float *yr = (float *)(ex4 + (size_t)nsq * rpc);     // [rpc]
     float *e1 = yr + rpc;                               // [rpc] sum over terms of |basis value|
     size_t off = ((size_t)((unsigned char *)(e1 + rpc) - fx_raw) + 15) & ~(size_t)15;
     float *wt = (float *)(fx_raw + off) + 3;            // wt[0..4*ntq]; wt + 1 is 16-byte aligned
-    float *wtold = wt + 1 + 4 * ntq;                    // [nt+1]
+    float *wtold = wt + 1 + 4 * (ntq + 4);                    // [nt+1]
     off = ((size_t)((unsigned char *)(wtold + nt + 1) - fx_raw) + 15) & ~(size_t)15;
     // [FX_RING] stream values, each with its position + 1 in the high word, so a reader knows
     // from the one 8-byte load whether the value it wants is there yet
@@ -196,11 +322,20 @@ __global__ void __launch_bounds__(FX_THREADS, 1) fitexp_cluster_kernel(FxDev F) 
     off = ((off + sizeof(float) * 2 * (size_t)fx_gstride(nw, rpc)) + 15) & ~(size_t)15;
     double *parts = (double *)(fx_raw + off);           // [2][nw]
     uint64_t *xbar = (uint64_t *)(parts + 2 * nw);      // [2]
-    long long *ckpos = (long long *)(xbar + 2);         // [FX_CK]
-    int32_t *ck = (int32_t *)(ckpos + FX_CK);           // [FX_CK][FX_CKW]
 
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     volatile FxShared *vs = &S;
+    if (rank == nw) {
+        if (tid == 0) {
+            S.cons = 0;
+            S.done = 0;
+        }
+        cl.sync();
+        if (tid < 64) fx_generate(F, G, S, ring);
+        __syncwarp();
+        cl.sync();   // no CTA leaves while others may still write into its shared memory
+        return;
+    }
     const int row0 = 1 + rank * rpc;                    // first (1-based) row of this CTA
     const int nrow = max(0, min(rpc, F.npt - row0 + 1));
     for (int idx = tid; idx < nsq * rpc; idx += blockDim.x) {
@@ -212,97 +347,34 @@ __global__ void __launch_bounds__(FX_THREADS, 1) fitexp_cluster_kernel(FxDev F) 
         }
         ex4[idx] = make_float4(e[0], e[1], e[2], e[3]);
     }
-    for (int i = tid; i <= 4 * ntq; i += blockDim.x) wt[i] = 0.0f;   // terms past nterms stay zero
+    for (int i = tid; i <= 4 * (ntq + 4); i += blockDim.x) wt[i] = 0.0f;   // terms past nterms stay zero
     for (int r = tid; r < rpc; r += blockDim.x) {
         float a = 0.0f;
         for (int m = 0; m < nt && r < nrow; ++m) a = __fadd_ru(a, fabsf(F.expr[1 + (size_t)(row0 - 1 + r) * nt + m]));
         e1[r] = a;
     }
-    for (int i = tid; i < FX_CK; i += blockDim.x) ckpos[i] = -1;
     for (int i = tid; i < FX_RING; i += blockDim.x) ring[i] = 0ull;   // no position yet
     if (tid < FX_WARPS) S.wmx[tid] = 0.0f;
     if (tid == 0) {
-        S.cons = 0;
-        S.done = 0;
         S.abort = 0;
         S.stop = 0;
-        mbar_init(&xbar[0], (uint32_t)nw);
-        mbar_init(&xbar[1], (uint32_t)nw);
+        mbar_init(&xbar[0], 1);
+        mbar_init(&xbar[1], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    const int32_t mcall0 = F.ran1[2];
     cl.sync();
+    const uint32_t gen_cons = map_rank(smem_addr(&S.cons), (uint32_t)nw), gen_done = map_rank(smem_addr(&S.done), (uint32_t)nw);
 
-    // ================================================================ stream warp
-    if (wid == FX_GEN_WARP) {
-        Ran1Warp g;
-        g.load(F.ran1);
-        long long pos = 0, nb = 0;
-        unsigned long long t0 = 0;
-        // the warp is converged at the top of every pass, so each control word is read by one
-        // warp-wide load and every lane takes the same branch
-        while (true) {
-            __syncwarp();
-            if (vs->done) break;
-            const long long room = vs->cons + FX_RING - pos;
-            if (room < 32) {   // ring full: wait for the workers (bounded)
-                int give_up = 0;
-                if (lane == 0) {
-                    const unsigned long long t = now_ns();
-                    if (t0 == 0) t0 = t;
-                    else if (t - t0 > FX_WAIT_NS || vs->abort) {
-                        atomicExch(F.status, 1);
-                        vs->abort = 1;
-                        give_up = 1;
-                    }
-                }
-                if (__shfl_sync(0xffffffffu, give_up, 0)) break;
-                __nanosleep(64);
-                continue;
-            }
-            t0 = 0;
-            // up to FX_GB batches before the control words are read again
-            const int nbat = room >= 32 * FX_GB ? FX_GB : (int)(room >> 5);
-            for (int bi = 0; bi < nbat; ++bi) {
-                if ((nb & (FX_CKE - 1)) == 0) {   // the state before this batch, every FX_CKE batches
-                    const int slot = (int)((nb / FX_CKE) & (FX_CK - 1));
-                    ck[slot * FX_CKW + 2 + lane] = g.iv;
-                    if (lane == 0) {
-                        ck[slot * FX_CKW + 0] = g.idum;
-                        ck[slot * FX_CKW + 1] = g.iy;
-                        ckpos[slot] = pos;
-                    }
-                }
-                ++nb;
-                int32_t mine;
-                const int cnt = g.next(32, mine, g_tab);
-                if (lane < cnt) {
-                    const long long q = pos + lane;
-                    ring[q & (FX_RING - 1)] = ((unsigned long long)(uint32_t)(q + 1) << 32) |
-                                              (unsigned long long)__float_as_uint(ran1_out(mine));
-                }
-                pos += cnt;
-            }
-        }
-        __syncwarp();
-        __syncthreads();   // meets the workers after they set done (barrier 0, all 512 threads)
-        cl.sync();
-        return;
-    }
-
-    // ================================================================ workers (warps 0-14)
     const float summax = exp_r(25.0f);
     const int K = nt - F.ncfirst + 1;                   // draws per trial
-    // row / coefficient slot of this thread: the warps of schedulers 0-2, -1 otherwise
-    const int slot = (wid & 3) != 3 ? (wid - (wid >> 2)) * 32 + lane : -1;
-    const int swarp = (wid & 3) != 3 ? wid - (wid >> 2) : -1;   // slot warp 0..11
-    const int ic = (slot >= 0 && slot < K) ? F.ncfirst + slot : -1;   // coefficient this thread perturbs
+    const int slot = tid, swarp = wid;                  // row / coefficient slot of this thread
+    const int ic = slot < K ? F.ncfirst + slot : -1;   // coefficient this thread perturbs
     // the first FX_RQ quads of this thread's row (row `slot`), in registers for the launch
     float4 rq[FX_RQ];
 #pragma unroll
     for (int k = 0; k < FX_RQ; ++k) {
         float e[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        if (slot >= 0 && slot < nrow) {
+        if (slot < nrow) {
             for (int j = 0; j < 4; ++j) {
                 const int m = 4 * k + j;
                 if (m < nt) e[j] = F.expr[1 + (size_t)(row0 - 1 + slot) * nt + m];
@@ -354,7 +426,10 @@ __global__ void __launch_bounds__(FX_THREADS, 1) fitexp_cluster_kernel(FxDev F) 
         float test;
         int draw = 0;
         if (exponent > 0.0f && exponent <= 20.0f) {
-            test = __fsub_rn(exp_r(-exponent), get(cursor));
+            // the sign of exp(-x) - u: a fast exponential decides all but the near cases
+            const float u = get(cursor);
+            test = __expf(-exponent) - u;
+            if (fabsf(test) < 1.0e-4f) test = __fsub_rn(exp_r(-exponent), u);
             draw = 1;
         } else if (exponent > 20.0f) {
             test = -1.0f;
@@ -383,7 +458,9 @@ __global__ void __launch_bounds__(FX_THREADS, 1) fitexp_cluster_kernel(FxDev F) 
         vs->smooth = sm;
         vs->draw = draw;
         vs->stop = vs->abort;
-        vs->cons = cursor + draw;
+        // every worker has taken the values before `cursor` (its part of chi^2 is here), but the
+        // draw at `cursor` perhaps not yet
+        if (rank == 0) st_cl_s64(gen_cons, cursor);
     };
 
     int xb = 0;                                         // exchange buffer
@@ -399,7 +476,7 @@ __global__ void __launch_bounds__(FX_THREADS, 1) fitexp_cluster_kernel(FxDev F) 
     auto chisq = [&](bool strict_sum, float *yout, bool trial) -> float {
         float *gb = gat + (size_t)xb * fx_gstride(nw, rpc);
         double mypart = 0.0;
-        if (slot >= 0) {
+        {
             float wmax = vs->wfix;
             const float *wm = (const float *)S.wmx;   // complete since the last barrier
 #pragma unroll
@@ -411,24 +488,44 @@ __global__ void __launch_bounds__(FX_THREADS, 1) fitexp_cluster_kernel(FxDev F) 
                 const float4 *e4 = ex4 + r;
                 // every partial sum is at most e1[r] * max|wt| (times 1 + 2^-20 for rounding)
                 if (__fmul_ru(__fmul_ru(e1[r], wmax), 1.001f) < summax) {
+                    // four quads at a time, the coefficients of the next four on their way: the
+                    // additions are a chain, 4.7 cycles each, and loads that waited in it cost 30
+                    float4 c[4];
 #pragma unroll
-                    for (int k = 0; k < FX_RQ; ++k) {
+                    for (int j = 0; j < 4; ++j) c[j] = w4[j];
+#pragma unroll
+                    for (int k = 0; k < FX_RQ; k += 4) {
                         if (k < ntq) {
-                            const float4 c = w4[k];
-                            sum = __fadd_rn(sum, __fmul_rn(rq[k].x, c.x));
-                            sum = __fadd_rn(sum, __fmul_rn(rq[k].y, c.y));
-                            sum = __fadd_rn(sum, __fmul_rn(rq[k].z, c.z));
-                            sum = __fadd_rn(sum, __fmul_rn(rq[k].w, c.w));
+                            float4 n[4];
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) n[j] = w4[k + 4 + j];
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                sum = __fadd_rn(sum, __fmul_rn(rq[k + j].x, c[j].x));
+                                sum = __fadd_rn(sum, __fmul_rn(rq[k + j].y, c[j].y));
+                                sum = __fadd_rn(sum, __fmul_rn(rq[k + j].z, c[j].z));
+                                sum = __fadd_rn(sum, __fmul_rn(rq[k + j].w, c[j].w));
+                            }
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) c[j] = n[j];
                         }
                     }
-#pragma unroll 2
-                    for (int q = 0; q < nsq; ++q) {
-                        const float4 c = w4[FX_RQ + q];
-                        const float4 e = e4[q * rpc];
-                        sum = __fadd_rn(sum, __fmul_rn(e.x, c.x));
-                        sum = __fadd_rn(sum, __fmul_rn(e.y, c.y));
-                        sum = __fadd_rn(sum, __fmul_rn(e.z, c.z));
-                        sum = __fadd_rn(sum, __fmul_rn(e.w, c.w));
+                    for (int q = 0; q < nsq; q += 4) {
+                        float4 n[4], f[4];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            f[j] = e4[(q + j) * rpc];
+                            n[j] = w4[FX_RQ + q + 4 + j];
+                        }
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            sum = __fadd_rn(sum, __fmul_rn(f[j].x, c[j].x));
+                            sum = __fadd_rn(sum, __fmul_rn(f[j].y, c[j].y));
+                            sum = __fadd_rn(sum, __fmul_rn(f[j].z, c[j].z));
+                            sum = __fadd_rn(sum, __fmul_rn(f[j].w, c[j].w));
+                        }
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) c[j] = n[j];
                     }
                 } else {  // the reference's clamped sum (expand :4924)
 #pragma unroll
@@ -454,30 +551,35 @@ __global__ void __launch_bounds__(FX_THREADS, 1) fitexp_cluster_kernel(FxDev F) 
                 const float q2 = __fmul_rn(term, term);
                 if (yout) yout[i] = sum;
                 if (strict_sum) {
-                    const uint32_t la = smem_addr(gb + (rank * rpc + r));
-                    for (int d = 0; d < nw; ++d) st_cl_f32(map_rank(la, (uint32_t)d), q2);
+                    const uint32_t la = smem_addr(gb + (rank * rpc + r)), lb = smem_addr(&xbar[xb]);
+                    for (int d = 0; d < nw; ++d)
+                        st_async_f32(map_rank(la, (uint32_t)d), q2, map_rank(lb, (uint32_t)d));
                 } else if (i >= F.nmin) {
                     mypart += (double)q2;
                 }
             }
         }
         __syncwarp();
-        if (strict_sum) {
-            fence_cluster();
-        } else {
+        if (!strict_sum) {
             mypart = warp_sum_d(mypart);
             if (lane == 0) vs->red[wid] = mypart;
+            block_sync();
         }
-        block_sync();
         if (wid == 0) {
             const uint32_t ba = smem_addr(&xbar[xb]);
-            double t = 0.0;
-            if (!strict_sum) t = warp_sum_d(lane < FX_GEN_WARP ? vs->red[lane] : 0.0);
-            if (lane < nw) {
-                if (!strict_sum) st_cl_f64(map_rank(smem_addr(parts + xb * nw + rank), (uint32_t)lane), t);
-                mbar_arrive_cluster(map_rank(ba, (uint32_t)lane));
+            if (!strict_sum) {
+                double p[T / 32], t = 0.0;
+#pragma unroll
+                for (int k = 0; k < T / 32; ++k) p[k] = vs->red[k];
+#pragma unroll
+                for (int k = 0; k < T / 32; ++k) t += p[k];
+                if (lane < nw)
+                    st_async_f64(map_rank(smem_addr(parts + xb * nw + rank), (uint32_t)lane), t,
+                                 map_rank(ba, (uint32_t)lane));
             }
             if (lane == 0) {
+                // this CTA's own arrival, and the bytes that every worker sends it
+                mbar_expect(&xbar[xb], strict_sum ? 4u * (uint32_t)F.npt : 8u * (uint32_t)nw);
                 const uint32_t par = (xph >> xb) & 1u;
                 if (!mbar_test(ba, par)) {
                     const unsigned long long t0 = now_ns();
@@ -491,23 +593,39 @@ __global__ void __launch_bounds__(FX_THREADS, 1) fitexp_cluster_kernel(FxDev F) 
                 }
                 float v;
                 if (strict_sum) {
+                    // sequential, the words sixteen rows ahead on their way
                     const int a = F.nmin - 1, b = F.npt;    // 0-based rows a..b-1
                     float c = 0.0f;
                     int i = a;
                     for (; i < b && (i & 3); ++i) c = __fadd_rn(c, gb[i]);
                     const float4 *g4 = (const float4 *)gb;
-                    for (; i + 3 < b; i += 4) {
-                        const float4 u = g4[i >> 2];
-                        c = __fadd_rn(c, u.x);
-                        c = __fadd_rn(c, u.y);
-                        c = __fadd_rn(c, u.z);
-                        c = __fadd_rn(c, u.w);
+                    const int q1 = b >> 2;
+                    int q = i >> 2;
+                    float4 u[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) u[j] = g4[min(q + j, max(q1 - 1, 0))];
+                    for (; q + 4 <= q1; q += 4) {
+                        float4 n[4];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) n[j] = g4[min(q + 4 + j, q1 - 1)];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            c = __fadd_rn(c, u[j].x);
+                            c = __fadd_rn(c, u[j].y);
+                            c = __fadd_rn(c, u[j].z);
+                            c = __fadd_rn(c, u[j].w);
+                            u[j] = n[j];
+                        }
                     }
-                    for (; i < b; ++i) c = __fadd_rn(c, gb[i]);
+                    for (i = max(i, 4 * q); i < b; ++i) c = __fadd_rn(c, gb[i]);
                     v = c;
                 } else {
-                    double u = 0.0;
-                    for (int q = 0; q < nw; ++q) u += parts[xb * nw + q];
+                    double p[FX_MAXW], u = 0.0;
+#pragma unroll
+                    for (int k = 0; k < FX_MAXW; ++k) p[k] = k < nw ? parts[xb * nw + k] : 0.0;
+#pragma unroll
+                    for (int k = 0; k < FX_MAXW; ++k)
+                        if (k < nw) u += p[k];
                     v = (float)u;
                 }
                 vs->val = v;
@@ -527,8 +645,8 @@ __global__ void __launch_bounds__(FX_THREADS, 1) fitexp_cluster_kernel(FxDev F) 
         float *yout = F.yout + (size_t)pi * (F.npt + 1);
         const float *wto_g = F.wtold_g + (size_t)pi * (nt + 1);
         float *scal = F.scal + (size_t)pi * 4;
-        for (int r = tid; r < rpc; r += FX_NBAR) yr[r] = r < nrow ? yin[row0 + r] : 0.0f;
-        for (int i = tid; i <= nt; i += FX_NBAR) {
+        for (int r = tid; r < rpc; r += T) yr[r] = r < nrow ? yin[row0 + r] : 0.0f;
+        for (int i = tid; i <= nt; i += T) {
             wtold[i] = wto_g[i];
             wt[i] = wtold[i];
         }
@@ -566,7 +684,7 @@ __global__ void __launch_bounds__(FX_THREADS, 1) fitexp_cluster_kernel(FxDev F) 
                     ++trials;
                     // perturb coefficients ncfirst..nterms with the next K values (:4856-4861),
                     // each thread waiting for its own value
-                    if (swarp >= 0 && swarp * 32 < K) {
+                    if (swarp * 32 < K) {
                         float a = 0.0f;
                         if (ic > 0) {
                             const float du = __fsub_rn(__fmul_rn(2.0f, get(cursor + slot)), 1.0f);
@@ -610,7 +728,7 @@ __global__ void __launch_bounds__(FX_THREADS, 1) fitexp_cluster_kernel(FxDev F) 
                 stepr = __fmul_rn(stepr, rejfac);
             }
             block_sync();   // every thread's own wtold update is in
-            for (int k = 1 + tid; k <= nt; k += FX_NBAR) wt[k] = wtold[k];
+            for (int k = 1 + tid; k <= nt; k += T) wt[k] = wtold[k];
             block_sync();
             if (tid == 0) wmax_all();
             block_sync();
@@ -620,7 +738,7 @@ __global__ void __launch_bounds__(FX_THREADS, 1) fitexp_cluster_kernel(FxDev F) 
         if (rank == 0) {
             float *wt_g = F.wt_g + (size_t)pi * (nt + 1);
             float *wtold_o = F.wtold_g + (size_t)pi * (nt + 1);
-            for (int k = tid; k <= nt; k += FX_NBAR) {
+            for (int k = tid; k <= nt; k += T) {
                 wt_g[k] = wt[k];
                 wtold_o[k] = wtold[k];
             }
@@ -634,28 +752,13 @@ __global__ void __launch_bounds__(FX_THREADS, 1) fitexp_cluster_kernel(FxDev F) 
         }
         block_sync();
     }
-    // stop the stream warp, then rebuild the state after exactly `cursor` draws from the
-    // last checkpoint at or before it (or from the launch's state when none is left)
-    if (tid == 0) vs->done = 1;
-    __syncwarp();
-    __syncthreads();
-    if (rank == 0 && tid == 0 && !vs->abort) {
-        int best = -1;
-        for (int k = 0; k < FX_CK; ++k)
-            if (ckpos[k] >= 0 && ckpos[k] <= cursor && (best < 0 || ckpos[k] > ckpos[best])) best = k;
-        Ran1 R;
-        long long from = 0;
-        ran1_load(R, F.ran1);
-        if (best >= 0) {
-            R.idum = ck[best * FX_CKW + 0];
-            R.iy = ck[best * FX_CKW + 1];
-            for (int i = 0; i < 32; ++i) R.iv[i] = ck[best * FX_CKW + 2 + i];
-            from = ckpos[best];
-        }
-        for (long long k = from; k < cursor; ++k) ran1_next(R);
-        R.mcall = (int32_t)((uint32_t)mcall0 + (uint32_t)cursor);
-        ran1_store(R, F.ran1);
+    // the generator leaves, and writes the state after the values taken unless a wait gave up
+    block_sync();
+    if (rank == 0 && tid == 0) {
+        st_cl_s64(gen_cons, cursor);
+        st_release_cl_s32(gen_done, vs->abort ? 2 : 1);
     }
+    __syncwarp();
     cl.sync();  // no CTA leaves while others may still write into its shared memory
 }
 
@@ -665,13 +768,20 @@ using namespace epsr;
 
 static inline size_t al256f(size_t x) { return (x + 255) & ~(size_t)255; }
 
-// Smallest cluster whose CTAs hold their rows with one row per slot thread (at most 8 CTAs).
-static int fx_workers(int npt, int nterms, int *rpc_out) {
-    const size_t budget = 220 * 1024;
-    for (int c = 1; c <= 8; ++c) {
+// Worker CTAs: as many as give each FX_ROWS rows (a trial's rows are summed side by side, so the
+// fewer a CTA has the shorter the trial; 600 rows x 116 terms, double sums: 5,370 cycles a trial on
+// two CTAs with the stream's warp among their own, 3,360 now, the length of its 117 values), up to seven beside
+// the generator's CTA, the portable cluster size; more only for rows that need the memory.  Rows
+// and terms for 256 threads: barriers of half the warps, and registers for the whole row.
+static int fx_workers(int npt, int nterms, int ncoef, int *rpc_out, int *threads_out) {
+    const size_t budget = 200 * 1024;
+    const int want = std::min((npt + FX_ROWS - 1) / FX_ROWS, FX_MAXW - 1);
+    for (int c = std::max(want, 1); c <= FX_MAXW; ++c) {
         const int rpc = (npt + c - 1) / c;
-        if (rpc <= FX_SLOTS && fx_smem_bytes(nterms, rpc, c) <= budget) {
+        const int threads = rpc <= 256 && ncoef <= 256 ? 256 : FX_MAXT;
+        if (rpc <= threads && fx_smem_bytes(nterms, rpc, c, threads) <= budget) {
             *rpc_out = rpc;
+            *threads_out = threads;
             return c;
         }
     }
@@ -707,8 +817,8 @@ extern "C" int epsr_fit_expansion_batch(int32_t nprob, const float *yin, const f
         epsr_set_error("epsr_fit_expansion_batch: at most %d perturbed terms", FX_SLOTS);
         return EPSR_ERR_UNSUPPORTED;
     }
-    int rpc = 0;
-    const int nw = fx_workers(npt, nterms, &rpc);
+    int rpc = 0, threads = 0;
+    const int nw = fx_workers(npt, nterms, nterms - ncfirst + 1, &rpc, &threads);
     if (!nw) {
         epsr_set_error("epsr_fit_expansion_batch: %d rows x %d terms exceed 8 CTAs of shared memory", npt, nterms);
         return EPSR_ERR_UNSUPPORTED;
@@ -740,22 +850,31 @@ extern "C" int epsr_fit_expansion_batch(int32_t nprob, const float *yin, const f
     F.nfreq = nfreq;
     F.strict = strict ? 1 : 0;
     F.rpc = rpc;
+    F.nw = nw;
     F.ran1 = ran1;
-    const size_t shm = fx_smem_bytes(nterms, rpc, nw);
-    EPSR_SMEM_OPTIN(fitexp_cluster_kernel);
+    const size_t shm = fx_smem_bytes(nterms, rpc, nw, threads);
+    const bool small = threads != FX_MAXT;
+    EPSR_SMEM_OPTIN(fitexp_cluster_kernel<256>);
+    EPSR_SMEM_OPTIN(fitexp_cluster_kernel<FX_MAXT>);
+    if (nw == FX_MAXW) {   // nine CTAs: past the portable cluster size
+        EPSR_CUDA(cudaFuncSetAttribute(fitexp_cluster_kernel<256>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        EPSR_CUDA(cudaFuncSetAttribute(fitexp_cluster_kernel<FX_MAXT>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(nw, 1, 1);
-    cfg.blockDim = dim3(FX_THREADS, 1, 1);
+    cfg.gridDim = dim3(nw + 1, 1, 1);
+    cfg.blockDim = dim3(small ? 256 : FX_MAXT, 1, 1);
     cfg.dynamicSmemBytes = shm;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = nw;
+    attr[0].val.clusterDim.x = nw + 1;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    EPSR_TIMED("fitexp_cluster_kernel", s, EPSR_CUDA(cudaLaunchKernelEx(&cfg, fitexp_cluster_kernel, F)));
+    EPSR_TIMED("fitexp_cluster_kernel", s,
+               EPSR_CUDA(small ? cudaLaunchKernelEx(&cfg, fitexp_cluster_kernel<256>, F)
+                               : cudaLaunchKernelEx(&cfg, fitexp_cluster_kernel<FX_MAXT>, F)));
     int hstatus = 0;
     EPSR_D2H(scal_host, scal, sizeof(float) * 4 * (size_t)nprob, s);
     EPSR_D2H(trials_host, trials, sizeof(long long) * (size_t)nprob, s);

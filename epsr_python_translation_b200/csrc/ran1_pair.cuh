@@ -15,7 +15,8 @@
 // lane, a[u], a[v]) supply what the lanes read next.  Everything that involves c and u is prepared
 // while the shuffles run, so a comparison and two selects stand between a fetch and the next.
 //
-// Measured on B200, the walk alone: 24.8 cycles a value, 29.5 step by step on keys, and 31.4 for
+// Measured on B200, the walk alone: 24.8 cycles a value (29 with the ring between the warps), 29.5
+// step by step on keys, and 31.4 for
 // one warp that shuffles values and keys step by step; the dependent shuffle alone is 26.  A branch
 // for the two lanes whose e is late, instead of their selects: 26.6.
 #pragma once
@@ -32,8 +33,10 @@ struct alignas(16) R1Ring {       // shared memory; rows are read 16 bytes at a 
     unsigned short slots[R1_NB][16];
     int tab[32];                  // the table of the value warp
     uint64_t made[R1_NB], walked[R1_NB];   // mbarriers: a batch's keys are there; its slots are
+    int stop;                     // 1: the walk leaves
 };
 
+__device__ __forceinline__ int r1_vol(const int *p) { return *(const volatile int *)p; }
 __device__ __forceinline__ void r1_arrive(uint64_t *bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"((uint32_t)__cvta_generic_to_shared(bar)) : "memory");
 }
@@ -42,11 +45,13 @@ __device__ __forceinline__ void r1_init(R1Ring &R) {   // one thread; a barrier 
         umma::mbar_init(&R.made[i], 1);
         umma::mbar_init(&R.walked[i], 1);
     }
+    R.stop = 0;
     umma::fence_mbar_init();
 }
 
 // The slot warp.  a: the key of this lane's slot; c: the first slot.  Walks batches 0 .. nb - 1
-// as their keys (and the first key of the batch after) arrive; gives up when they do not.
+// as their keys (and the first key of the batch after) arrive; gives up when they do not, and
+// leaves when R.stop is set.
 __device__ __forceinline__ void r1_walk(R1Ring &R, int a, int c, int nb) {
     const int lane = threadIdx.x & 31;
     int e = 0;
@@ -55,19 +60,20 @@ __device__ __forceinline__ void r1_walk(R1Ring &R, int a, int c, int nb) {
         const int f = __shfl_sync(0xffffffffu, a, a);
         e = a == lane ? R.keys[0][0] : f;
     }
+    int4 k = nb > 0 ? *(const int4 *)R.keys[0] : make_int4(0, 0, 0, 0);
     for (int b = 0; b < nb; ++b) {
         // the batch after the next one's keys: asked for early, waited for at the end
         bool there = true;
+        int stop = 0;
         const int4 *k4 = (const int4 *)R.keys[b & (R1_NB - 1)];
-        const int after = R.keys[(b + 1) & (R1_NB - 1)][0];
-        int4 k = k4[0];
+        const int4 after = *(const int4 *)R.keys[(b + 1) & (R1_NB - 1)];
         unsigned short *out = R.slots[b & (R1_NB - 1)];
 #pragma unroll
         for (int s = 0; s < 16; ++s) {
             // the keys written in this double step, and the first of the next
             const int u = (s & 1) ? k.z : k.x, v = (s & 1) ? k.w : k.y;
             int4 kn = k;
-            if (s & 1) kn = s < 15 ? k4[(s >> 1) + 1] : make_int4(after, 0, 0, 0);
+            if (s & 1) kn = s < 15 ? k4[(s >> 1) + 1] : after;
             const int u2 = (s & 1) ? kn.x : k.z;
             const int p = __shfl_sync(0xffffffffu, a, c);
             const int q = __shfl_sync(0xffffffffu, e, c);
@@ -89,12 +95,14 @@ __device__ __forceinline__ void r1_walk(R1Ring &R, int a, int c, int nb) {
             if (lane == 0) out[s] = (unsigned short)(c | (p << 8));
             c = q;
             k = kn;
+            if (s == 8) stop = r1_vol(&R.stop);
             if (s == 8) there = umma::mbar_try(&R.made[(b + 2) & (R1_NB - 1)], (uint32_t)((b + 2) / R1_NB) & 1u);
         }
         if (lane == 0) r1_arrive(&R.walked[b & (R1_NB - 1)]);
         if (!there && b + 1 < nb &&
             !umma::mbar_wait(&R.made[(b + 2) & (R1_NB - 1)], (uint32_t)((b + 2) / R1_NB) & 1u, nullptr))
             return;
+        if (stop) return;
     }
 }
 
@@ -125,6 +133,13 @@ struct R1Values {
         __syncwarp();
         if (lane == 0) r1_arrive(&R.made[made & (R1_NB - 1)]);
         ++made;
+    }
+    __device__ __forceinline__ void leave(R1Ring &R) {   // no batch follows: the walk goes home
+        __syncwarp();
+        if ((threadIdx.x & 31) == 0) {
+            *(volatile int *)&R.stop = 1;
+            for (int i = 0; i < 2; ++i) r1_arrive(&R.made[(made + i) & (R1_NB - 1)]);
+        }
     }
     __device__ __forceinline__ bool walked(R1Ring &R, int b) {
         return __all_sync(0xffffffffu,
