@@ -11,7 +11,7 @@
 // (4) normalisation in float32 exactly as the reference (counts are exact integers; the
 //     reference's float accumulation equals them while a bin stays below 2^24).
 
-#include "common.cuh"
+#include "pairhist.cuh"
 
 namespace epsr {
 
@@ -28,55 +28,51 @@ struct AgDev {
 // (1) selection.  draws: one ran1 value per candidate im in [im1, im2] (:3765).  The rule
 // "u < probaccept or type not yet sampled or type fraction < probaccept" is sequential only
 // through "not yet sampled", which holds exactly for the first candidate of each type; so the
-// selection is a parallel filter followed by an ordered compaction (one block).  It also
-// returns the per-type atom counts of the sampled molecules (csampled, exact integers like the
-// reference's float sums of 1.0), the origin-atom prefix and the pair-update count.
-__device__ __forceinline__ int ag_bscan(int v, int *total) {
-    __shared__ int ws[32];
-    __shared__ int wp[33];
+// selection is a parallel filter followed by an ordered compaction (one block), which reads no more
+// than a molecule's type, draw and atom range: 8,000 molecules took 73 us while it also walked
+// the selected molecules' atoms, 44 us now.  It returns the origin-atom prefix and the
+// pair-update count.
+// Block-wide exclusive scan of two counts; *total = the block's sums.
+__device__ __forceinline__ int2 ag_bscan(int2 v, int2 *total) {
+    __shared__ int2 ws[32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-    int incl = v;
+    int2 incl = v;
     for (int o = 1; o < 32; o <<= 1) {
-        int t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += t;
+        const int a = __shfl_up_sync(0xffffffffu, incl.x, o), b = __shfl_up_sync(0xffffffffu, incl.y, o);
+        if (lane >= o) {
+            incl.x += a;
+            incl.y += b;
+        }
     }
     if (lane == 31) ws[wid] = incl;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int a = 0;
-        for (int w = 0; w < nw; ++w) {
-            wp[w] = a;
-            a += ws[w];
-        }
-        wp[32] = a;
-    }
+    // every warp sums the warps before it
+    const int2 w = lane < nw ? ws[lane] : make_int2(0, 0);
+    total->x = __reduce_add_sync(0xffffffffu, w.x);
+    total->y = __reduce_add_sync(0xffffffffu, w.y);
+    const int bx = __reduce_add_sync(0xffffffffu, lane < wid ? w.x : 0);
+    const int by = __reduce_add_sync(0xffffffffu, lane < wid ? w.y : 0);
     __syncthreads();
-    const int r = wp[wid] + incl - v;
-    *total = wp[32];
-    __syncthreads();
-    return r;
+    return make_int2(bx + incl.x - v.x, by + incl.y - v.y);
 }
 
 __global__ void ag_select_kernel(AgDev A, const float *draws, int im1, int im2, float probaccept,
-                                 const int32_t *itype, int32_t *origins, int32_t *prefix, int32_t *counts_out,
-                                 float *csampled, long long *pairs_out) {
+                                 int32_t *origins, int32_t *prefix, int32_t *counts_out,
+                                 long long *pairs_out) {
     __shared__ int first[64];
     __shared__ int cntt[64];
-    __shared__ int catoms[64];
     __shared__ unsigned long long spairs;
     const int tid = threadIdx.x;
     for (int t = tid; t < 64; t += blockDim.x) {
         first[t] = 0x7fffffff;
         cntt[t] = 0;
-        catoms[t] = 0;
     }
     if (tid == 0) spairs = 0ull;
     __syncthreads();
     for (int m = tid; m < A.nmol; m += blockDim.x) atomicAdd(&cntt[A.mtype[m]], 1);
-    for (int im = im1 + tid; im <= im2; im += blockDim.x) atomicMin(&first[A.mtype[im]], im);
-    if (A.full && tid == 0) {
-        const int m = A.nmol - 1;
-        for (int a = A.naf[m]; a < A.naf[m] + A.nato[m]; ++a) atomicAdd(&catoms[itype[a]], 1);
+    for (int im = im1 + tid; im <= im2; im += blockDim.x) {
+        volatile int *f = &first[A.mtype[im]];   // only ever falls, so a stale value costs an atomic at most
+        if (im < *f) atomicMin((int *)f, im);
     }
     __syncthreads();
     int carry = 0, acarry = 0;
@@ -90,24 +86,23 @@ __global__ void ag_select_kernel(AgDev A, const float *draws, int im1, int im2, 
             sel = draws[im - im1] < probaccept || first[mt] == im || frac < probaccept;
             if (sel) {
                 na = A.nato[im];
-                for (int a = A.naf[im]; a < A.naf[im] + na; ++a) atomicAdd(&catoms[itype[a]], 1);
-                const long long tgt = A.full ? (long long)(A.natom - A.naf[im] - na) : (long long)(A.natom - na);
+                const int a0 = A.naf[im];
+                const long long tgt = A.full ? (long long)(A.natom - a0 - na) : (long long)(A.natom - na);
                 mypairs += (unsigned long long)((long long)na * tgt);
             }
         }
-        int tot, atot;
-        const int pos = carry + ag_bscan(sel, &tot);
-        const int apos = acarry + ag_bscan(na, &atot);
+        int2 tot;
+        const int2 before = ag_bscan(make_int2(sel, na), &tot);
+        const int pos = carry + before.x, apos = acarry + before.y;
         if (sel) {
             origins[pos] = im;
             prefix[pos] = apos;
         }
-        carry += tot;
-        acarry += atot;
+        carry += tot.x;
+        acarry += tot.y;
     }
     atomicAdd(&spairs, mypairs);
     __syncthreads();
-    for (int t = tid; t < A.ntype; t += blockDim.x) csampled[t] = (float)catoms[t];
     if (tid == 0) {
         counts_out[0] = carry;   // sampled molecules
         counts_out[1] = acarry;  // origin atoms
@@ -115,7 +110,16 @@ __global__ void ag_select_kernel(AgDev A, const float *draws, int im1, int im2, 
     }
 }
 
-// (2) intramolecular pairs
+// (2) intramolecular pairs.  Lanes are molecules at the same pair: a rigid molecule's lanes share the
+// bin, and one lane then adds for all (2,700 DMSO + 5,300 water: 24 us, 38 us one by one).
+__device__ __forceinline__ void add_count(unsigned long long *c) {
+    const unsigned m = __activemask();
+    int all;
+    __match_all_sync(m, (unsigned long long)c, &all);
+    if (!all) atomicAdd(c, 1ull);
+    else if ((threadIdx.x & 31) == __ffs(m) - 1) atomicAdd(c, (unsigned long long)__popc(m));
+}
+
 __global__ void ag_intra_kernel(AgDev A, const int32_t *itype, unsigned long long *counts, long long *pairs_out) {
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= A.nmol) return;
@@ -130,73 +134,89 @@ __global__ void ag_intra_kernel(AgDev A, const int32_t *itype, unsigned long lon
             float zz = __fmul_rn(__fsub_rn(A.za[ia], A.za[ja]), A.sizefactor);
             const float d = dist_f(A.L, xx, yy, zz);
             const int iz1 = nint_i(__fdiv_rn(d, A.stepcl)) + 2;
-            if (iz1 > 1 && iz1 <= A.npt1) atomicAdd(counts + (size_t)icref * A.ldw + iz1, 1ull);
+            if (iz1 > 1 && iz1 <= A.npt1) add_count(counts + (size_t)icref * A.ldw + iz1);
             ++np;
         }
     }
     atomicAdd((unsigned long long *)pairs_out, (unsigned long long)np);
 }
 
-// origin atoms of the selected molecules: (atom, molecule) pairs in selection order
-__global__ void ag_origin_atoms_kernel(AgDev A, const int32_t *origins, const int32_t *norigin, const int32_t *prefix,
-                                       int2 *oatoms) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= *norigin) return;
-    const int im = origins[k];
-    for (int q = 0; q < A.nato[im]; ++q) oatoms[prefix[k] + q] = make_int2(A.naf[im] + q, im);
+// Origin atoms of the selected molecules, (atom, molecule) pairs in selection order, and the sampled
+// atoms of each type (csampled: exact integers, like the reference's float sums of 1.0), to which a
+// full pass adds the last molecule.
+__global__ void ag_origin_atoms_kernel(AgDev A, const int32_t *itype, const int32_t *origins, const int32_t *norigin,
+                                       const int32_t *prefix, int2 *oatoms, int32_t *csampled) {
+    __shared__ int catoms[64];
+    for (int t = threadIdx.x; t < 64; t += blockDim.x) catoms[t] = 0;
+    __syncthreads();
+    const int k = blockIdx.x * blockDim.x + threadIdx.x, no = *norigin;
+    if (k < no || (A.full && k == no)) {
+        const int im = k < no ? origins[k] : A.nmol - 1;
+        const int a0 = A.naf[im], n = A.nato[im], p0 = k < no ? prefix[k] : 0;
+#pragma unroll 4
+        for (int q = 0; q < n; ++q) {
+            atomicAdd(&catoms[__ldg(itype + a0 + q)], 1);
+            if (k < no) oatoms[p0 + q] = make_int2(a0 + q, im);
+        }
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < A.ntype; t += blockDim.x)
+        if (catoms[t]) atomicAdd(csampled + t, catoms[t]);
 }
 
-// (3) intermolecular all-pairs
-constexpr int AG_THREADS = 256;
-
-__global__ void __launch_bounds__(AG_THREADS) ag_inter_kernel(AgDev A, const int2 *oatoms, const int32_t *noatoms_p,
-                                                              const int32_t *molof, int tile,
-                                                              unsigned long long *counts, unsigned long long *potex) {
+// (3) intermolecular all-pairs (pairhist.cuh): CTA (x, y) takes 256 origins and every gridDim.x-th
+// tile of targets, so that its histogram is cleared and merged once
+template <bool CUBIC>
+__global__ void __launch_bounds__(1024) ag_inter_kernel(AgDev A, const int2 *oatoms, const int32_t *noatoms_p,
+                                                        const int32_t *molof, int tile, unsigned long long *counts,
+                                                        unsigned long long *potex) {
     extern __shared__ unsigned char sm[];
+    __shared__ int cls[PH_TYPES * PH_TYPES];
     const int nbins = A.npairs * A.ldw;
-    unsigned int *hist = (unsigned int *)sm;
-    unsigned int *hpot = hist + nbins;
     // the float4 tile must start on a 16-byte boundary
     const size_t tp_off = ((sizeof(unsigned int) * ((size_t)nbins + A.npairs)) + 15) & ~(size_t)15;
     float4 *tp = (float4 *)(sm + tp_off);
     int *tm = (int *)(tp + tile);
     const int noatoms = *noatoms_p;
-    const int t0 = blockIdx.x * tile;
-    const int tn = min(tile, A.natom - t0);
-    const int obase = blockIdx.y * AG_THREADS;
-    if (obase >= noatoms || tn <= 0) return;
-    for (int i = threadIdx.x; i < nbins; i += blockDim.x) hist[i] = 0;
-    for (int i = threadIdx.x; i < A.npairs; i += blockDim.x) hpot[i] = 0;
-    for (int i = threadIdx.x; i < tn; i += blockDim.x) {
-        tp[i] = A.pos[t0 + i];
-        tm[i] = molof[t0 + i];
-    }
-    __syncthreads();
-    const int k = obase + threadIdx.x;
-    if (k < noatoms) {
-        const int2 oa = oatoms[k];
-        const float4 p1 = A.pos[oa.x];
-        const int im = oa.y;
-        const int it = __float_as_int(p1.w);
-        const int *pr = A.npairref + it * A.ntype;
-        for (int q = 0; q < tn; ++q) {
-            const int jm = tm[q];
-            const bool use = A.full ? (jm > im) : (jm != im);
-            if (!use) continue;
-            const float4 p2 = tp[q];
-            const int icref = __ldg(pr + __float_as_int(p2.w));
-            // xx = x1 - x2 (ato_manipulation_rev4.py:3798)
-            const float d = dist_f(A.L, __fsub_rn(p1.x, p2.x), __fsub_rn(p1.y, p2.y), __fsub_rn(p1.z, p2.z));
-            const int iz1 = nint_i(__fdiv_rn(d, A.stepcl)) + 2;
-            if (iz1 > 1 && iz1 <= A.npt1) atomicAdd(hist + icref * A.ldw + iz1, 1u);
-            if (__fmul_rn(d, A.dmax) < fabsf(__ldg(A.rminex + icref))) atomicAdd(hpot + icref, 1u);
-        }
+    const int obase = blockIdx.y * PH_ORIGINS;
+    if (obase >= noatoms) return;
+    PairHist H;
+    H.hist = (unsigned int *)sm;
+    H.hpot = H.hist + nbins;
+    H.npairref = A.npairref;
+    H.rminex = A.rminex;
+    H.ld = A.ldw;
+    H.ntype = A.ntype;
+    H.nlim = max(A.npt1 - 1, 0);
+    H.stepcl = A.stepcl;
+    H.rcp = CUBIC ? hist_rcp(A.stepcl) : nanf("");
+    H.dmax = A.dmax;
+    H.rmax = hist_rmax(A.rminex, A.npairs);
+    H.L = A.L;
+    for (int i = threadIdx.x; i < nbins + A.npairs; i += blockDim.x) H.hist[i] = 0;
+    hist_stage_types(H, cls);
+    __shared__ int mols[2];   // the tile's first and last molecule
+    const int parts = blockDim.x / PH_ORIGINS, part = threadIdx.x / PH_ORIGINS;
+    const int k = obase + threadIdx.x % PH_ORIGINS;
+    const int2 oa = k < noatoms ? oatoms[k] : make_int2(0, 0);
+    const float4 p1 = A.pos[oa.x];
+    const int im = oa.y;
+    for (int t0 = blockIdx.x * tile; t0 < A.natom; t0 += gridDim.x * tile) {
+        const int tn = min(tile, A.natom - t0);
+        __syncthreads();
+        hist_stage_tile(H, A.pos + t0, molof + t0, tn, tp, tm, mols);
+        // origins are in molecule order
+        if (k >= noatoms || (A.full && mols[1] <= oatoms[obase].y)) continue;
+        const int per = ((tn + parts - 1) / parts + 3) & ~3;
+        const int q0 = min(part * per, tn), q1 = min(q0 + per, tn);
+        if (A.ntype <= PH_TYPES) hist_tile<CUBIC, true>(H, p1, im, A.full, tp, tm, q0, q1, mols, cls);
+        else hist_tile<CUBIC, false>(H, p1, im, A.full, tp, tm, q0, q1, mols, cls);
     }
     __syncthreads();
     for (int i = threadIdx.x; i < nbins; i += blockDim.x)
-        if (hist[i]) atomicAdd(counts + (size_t)A.npairs * A.ldw + i, (unsigned long long)hist[i]);
+        if (H.hist[i]) atomicAdd(counts + (size_t)A.npairs * A.ldw + i, (unsigned long long)H.hist[i]);
     for (int i = threadIdx.x; i < A.npairs; i += blockDim.x)
-        if (hpot[i]) atomicAdd(potex + i, (unsigned long long)hpot[i]);
+        if (H.hpot[i]) atomicAdd(potex + i, (unsigned long long)H.hpot[i]);
 }
 
 __global__ void ag_molof_kernel(AgDev A, int32_t *molof) {
@@ -206,16 +226,16 @@ __global__ void ag_molof_kernel(AgDev A, int32_t *molof) {
 
 // (4) normalisation (:3857-3897)
 __global__ void ag_norm_kernel(AgDev A, const unsigned long long *counts, const unsigned long long *potc,
-                               const float *csampled, const float *cfrac, const int32_t *n1extr,
+                               const int32_t *csampled, const float *cfrac, const int32_t *n1extr,
                                const int32_t *n2extr, int natomr, float addwav, const float *ycoh, float *wav,
                                float *potex) {
     const int ic = blockIdx.x;
     const int it = n1extr[ic], jt = n2extr[ic];
     float cprod = __fmul_rn(__fmul_rn(cfrac[it], cfrac[jt]), (float)natomr);
-    float cprod2 = __fmul_rn(csampled[it], cfrac[jt]);
+    float cprod2 = __fmul_rn((float)csampled[it], cfrac[jt]);
     if (it != jt) {
         cprod = __fmul_rn(cprod, 2.0f);
-        cprod2 = __fadd_rn(cprod2, __fmul_rn(csampled[jt], cfrac[it]));
+        cprod2 = __fadd_rn(cprod2, __fmul_rn((float)csampled[jt], cfrac[it]));
     }
     float *w1 = wav + (size_t)ic * A.ldw;
     float *w2 = wav + (size_t)(A.npairs + ic) * A.ldw;
@@ -254,6 +274,22 @@ extern "C" int64_t epsr_atogen_scratch_bytes(int32_t nmol, int32_t natom, int32_
 }
 
 extern "C" int64_t epsr_atogen_last_pair_updates(void) { return g_last_pairs; }
+
+// CTAs that share a chunk of origins: the number whose waves take the least, a tile costing its
+// targets and a CTA besides them the clearing and merging of its histogram (about 1/32 target a bin).
+static int ag_splits(int ychunks, int ntiles, int tile, size_t nbins, int slots) {
+    long long best = 0;
+    int x = 1;
+    for (int i = 1; i <= ntiles; ++i) {
+        const long long waves = ((long long)ychunks * i + slots - 1) / slots;
+        const long long cost = waves * ((long long)((ntiles + i - 1) / i) * tile + (long long)(nbins / 32));
+        if (i == 1 || cost < best) {
+            best = cost;
+            x = i;
+        }
+    }
+    return x;
+}
 
 extern "C" int epsr_atogen(const epsr_box_t *box, int32_t npt1, float sizefactor, float dmax, const float *rminex,
                            const float *cfrac, const float *ycoh, const int32_t *n1extr, const int32_t *n2extr,
@@ -295,7 +331,7 @@ extern "C" int epsr_atogen(const epsr_box_t *box, int32_t npt1, float sizefactor
     int32_t *prefix = (int32_t *)take(sizeof(int32_t) * nmol);
     int2 *oatoms = (int2 *)take(sizeof(int2) * natom);
     int32_t *molof = (int32_t *)take(sizeof(int32_t) * natom);
-    float *csampled = (float *)take(sizeof(float) * (box->ntype + 1));
+    int32_t *csampled = (int32_t *)take(sizeof(int32_t) * (box->ntype + 1));
     int32_t *misc = (int32_t *)take(sizeof(int32_t) * 8);
     long long *pairc = (long long *)take(sizeof(long long) * 2);
 
@@ -339,6 +375,7 @@ extern "C" int epsr_atogen(const epsr_box_t *box, int32_t npt1, float sizefactor
     const size_t nbins = (size_t)box->npairs * ldw;
     EPSR_CUDA(cudaMemsetAsync(counts, 0, sizeof(unsigned long long) * (2 * nbins + box->npairs), s));
     EPSR_CUDA(cudaMemsetAsync(pairc, 0, sizeof(long long) * 2, s));
+    EPSR_CUDA(cudaMemsetAsync(csampled, 0, sizeof(int32_t) * (box->ntype + 1), s));
     int rc = epsr_box_positions(box, stream);
     if (rc) return rc;
     const int ncand = im2 - im1 + 1;
@@ -346,18 +383,17 @@ extern "C" int epsr_atogen(const epsr_box_t *box, int32_t npt1, float sizefactor
         rc = epsr_ran1_fill(ran1, draws, ncand, stream);
         if (rc) return rc;
     }
-    ag_select_kernel<<<1, 1024, 0, s>>>(A, draws, im1, im2, probaccept, box->itype, origins, prefix, misc, csampled,
-                                         pairc);
+    ag_select_kernel<<<1, 1024, 0, s>>>(A, draws, im1, im2, probaccept, origins, prefix, misc, pairc);
     ag_intra_kernel<<<(nmol + 127) / 128, 128, 0, s>>>(A, box->itype, counts, pairc + 1);
     ag_molof_kernel<<<nmol, 32, 0, s>>>(A, molof);
-    ag_origin_atoms_kernel<<<(nmol + 127) / 128, 128, 0, s>>>(A, origins, misc, prefix, oatoms);
+    ag_origin_atoms_kernel<<<(nmol + 128) / 128, 128, 0, s>>>(A, box->itype, origins, misc, prefix, oatoms, csampled);
     EPSR_CUDA(cudaGetLastError());
     int32_t hmisc[2];
     EPSR_D2H(hmisc, misc, sizeof(hmisc), s);
     const int noatoms = hmisc[1];
-    // tile of target atoms: enough blocks to fill the GPU several times over
+    // tile of target atoms: 1,024, fewer in small boxes so that there are CTAs for the SMs
     int tile = 1024;
-    const int ychunks = (noatoms + AG_THREADS - 1) / AG_THREADS;
+    const int ychunks = (noatoms + PH_ORIGINS - 1) / PH_ORIGINS;
     while (tile > 128 && (long long)ychunks * ((natom + tile - 1) / tile) < 4 * 148) tile >>= 1;
     const size_t tp_off = ((sizeof(unsigned int) * (nbins + box->npairs)) + 15) & ~(size_t)15;
     const size_t shm = tp_off + (sizeof(float4) + sizeof(int)) * tile;
@@ -365,11 +401,16 @@ extern "C" int epsr_atogen(const epsr_box_t *box, int32_t npt1, float sizefactor
         epsr_set_error("epsr_atogen: histogram of %zu bins does not fit in shared memory", nbins);
         return EPSR_ERR_UNSUPPORTED;
     }
-    if (shm > 48 * 1024)
-        EPSR_SMEM_OPTIN(ag_inter_kernel);
     if (noatoms > 0) {
-        dim3 grid((natom + tile - 1) / tile, ychunks);
-        EPSR_TIMED("ag_inter_kernel", s, ag_inter_kernel<<<grid, AG_THREADS, shm, s>>>(A, oatoms, misc + 1, molof, tile, counts, counts + 2 * nbins));
+        const int threads = hist_threads(shm);
+        const dim3 grid(ag_splits(ychunks, (natom + tile - 1) / tile, tile, nbins, 148 * (1024 / threads)), ychunks);
+        if (box->cubic) {
+            if (shm > 48 * 1024) EPSR_SMEM_OPTIN(ag_inter_kernel<true>);
+            EPSR_TIMED("ag_inter_kernel", s, ag_inter_kernel<true><<<grid, threads, shm, s>>>(A, oatoms, misc + 1, molof, tile, counts, counts + 2 * nbins));
+        } else {
+            if (shm > 48 * 1024) EPSR_SMEM_OPTIN(ag_inter_kernel<false>);
+            EPSR_TIMED("ag_inter_kernel", s, ag_inter_kernel<false><<<grid, threads, shm, s>>>(A, oatoms, misc + 1, molof, tile, counts, counts + 2 * nbins));
+        }
     }
     ag_norm_kernel<<<box->npairs, 256, 0, s>>>(A, counts, counts + 2 * nbins, csampled, cfrac, n1extr, n2extr, natomr,
                                                 addwav, ycoh, wav, potex);

@@ -212,12 +212,14 @@ __device__ __forceinline__ int bin_index(float d, float stepcl, float rcp) {
 // root's approximation, the residual exact by the fused product.  Equal to __fsqrt_rn for zero and
 // for every float from 2^-60 to 2^4 (tests/test_pair_math_gpu.py compares all of them); squared
 // distances in box units lie there.
-__device__ __forceinline__ float sqrt_unit(float x) {
+__device__ __forceinline__ float sqrt_unit_from(float x, float y) {
     float s;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(s) : "f"(fmaxf(x, 1e-37f)));
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(s) : "f"(y));
     const float d = __fmul_rn(x, s);
     return __fmaf_rn(__fmaf_rn(-d, d, x), __fmul_rn(0.5f, s), d);
 }
+__device__ __forceinline__ float sqrt_unit(float x) { return sqrt_unit_from(x, fmaxf(x, 1e-37f)); }
+__device__ __forceinline__ float sqrt_unit_nz(float x) { return sqrt_unit_from(x, x); }   // a NaN for 0
 
 // pair_energy for a cubic box, bit for bit: the same distance, index, table entry and sum
 __device__ __forceinline__ float pair_energy_cubic_bins(const Bins &B, float4 p1, float4 p2, int icref) {
