@@ -16,18 +16,20 @@
 // exchange their chi^2 contributions through distributed shared memory: each stores its
 // part (a double partial, or every residual for the reference's sequential float sum) into
 // every CTA, the stores completing their bytes on that CTA's mbarrier (no release stands between a
-// store and its signal); each then forms the same chi^2, so all take
-// the same decisions without a second exchange.  Thread 0 of each CTA takes every decision
-// (Metropolis test, smoothing, stopping) and broadcasts it through shared memory, so all
-// threads pass the same barriers.  The strict sum is one chain of additions over all rows, 4.7
-// cycles each (1,000 rows x 97 terms: 21,700 cycles a trial when every fourth row waited for its
-// word, 8,400 now).
+// store and its signal).  Every warp of every CTA waits for the parts, forms the same chi^2 and
+// takes the same decision, so a trial passes one barrier of the CTA, after the coefficients are
+// perturbed (600 rows x 116 terms, double sums: 3,390 cycles a trial while warp 0 collected its CTA's
+// sums and published the decision behind two more barriers, 3,240 now: 1,100 the row's 116 additions
+// and their loads, 750 the two trees of double additions, 40 cycles each, the rest the perturbation,
+// the exchange and the test, and the stream close behind).  The strict sum is one chain of additions over all
+// rows, 4.7 cycles each (1,000 rows x 97 terms: 21,700 cycles a trial when every fourth row waited for
+// its word, 8,340 now).
 //
 // ran1.  The chain is sequential and one trial's values outlast one trial's arithmetic, so it has
-// an SM to itself: the cluster's last CTA generates the stream with two warps (ran1_pair.cuh) and
+// an SM to itself: the cluster's last CTA generates the stream with three warps (ran1_pair.cuh) and
 // stores the values into a ring in every worker CTA's shared memory, running ahead of the trials
 // (bounded by the ring).  On a warp of each worker CTA, beside its rows' shared-memory reads, the
-// same chain took 46 cycles a value instead of 29.  At the end the state the reference leaves after
+// same chain took 46 cycles a value instead of 27.  At the end the state the reference leaves after
 // exactly the values the fit consumed is rebuilt from the generator's checkpoints.
 //
 // Every wait (ring, exchange, ring space) is bounded in time: on timeout the kernel records
@@ -43,7 +45,6 @@ namespace cg = cooperative_groups;
 namespace epsr {
 
 constexpr int FX_MAXT = 512;                    // most threads of a worker CTA (256 when rows and terms fit)
-constexpr int FX_WARPS = FX_MAXT / 32;
 constexpr int FX_SLOTS = FX_MAXT;               // row / coefficient slots of a worker CTA at most
 constexpr int FX_ROWS = 160;                    // rows a CTA takes while the cluster has CTAs left
 constexpr int FX_MAXW = 8;                      // worker CTAs of a cluster
@@ -124,12 +125,8 @@ __device__ __forceinline__ unsigned long long now_ns() {
 struct FxShared {                 // statically sized control block (one per CTA)
     long long cons;               // generator: lowest stream index the workers may still read
     int done;                     // generator: set by the workers when the fit is over
-    int abort, stop;
-    int accept, smooth, draw;     // thread 0's decision of the current trial
-    float val;                    // chi^2 broadcast
-    float wfix;                   // largest |wt| of the unperturbed terms 1..ncfirst-1
-    float wmx[FX_WARPS];          // largest |wt| of the terms each warp perturbed
-    double red[FX_WARPS];
+    int abort;
+    float wmx;                    // largest |wt| of the perturbed terms
 };
 
 // quads of a row, in whole groups of four (terms past nterms are zero on both sides)
@@ -146,9 +143,6 @@ size_t fx_smem_bytes(int nt, int rpc, int nw, int threads) {
     const int ntq = fx_ntq(nt);
     size_t b = 0;
     b += 16 * (size_t)fx_nsq(nt, threads) * rpc;                 // ex4
-    b += sizeof(float) * (size_t)rpc;                   // yr
-    b += sizeof(float) * (size_t)rpc;                   // e1 (row L1 norms)
-    b = (b + 15) & ~(size_t)15;
     b += sizeof(float) * (4 + 4 * ((size_t)ntq + 4));   // wt (wt + 1 16-byte aligned, a group past the end)
     b += sizeof(float) * (size_t)(nt + 1);              // wtold
     b = (b + 15) & ~(size_t)15;
@@ -156,7 +150,7 @@ size_t fx_smem_bytes(int nt, int rpc, int nw, int threads) {
     b = (b + 15) & ~(size_t)15;
     b += sizeof(float) * 2 * (size_t)fx_gstride(nw, rpc);   // gat[2][gstride]
     b = (b + 15) & ~(size_t)15;
-    b += sizeof(double) * 2 * (size_t)nw;               // parts[2][nw]
+    b += sizeof(double) * 2 * (size_t)nw * ((rpc + 31) / 32);   // parts[2][nw][warps with rows]
     b += sizeof(uint64_t) * 2;                          // exchange mbarriers
     return b;
 }
@@ -166,16 +160,20 @@ struct FxGen {                    // the generator CTA's shared memory
     int32_t tab[34];
     long long ckpos[FX_CK];
     int32_t ck[FX_CK][FX_CKW];    // idum, iy, iv[32] before a batch
-    int first, go;
+    int first, idum, go;
 };
 
 // The generator CTA: values 0, 1, ... of the stream into the workers' rings until they are done,
-// then the state after the values they took.  Warps 0 and 1 call.
+// then the state after the values they took.  Warps 0 to 2 call.
 __device__ void fx_generate(const FxDev &F, FxGen &G, FxShared &S, unsigned long long *ring) {
     const int lane = threadIdx.x & 31;
     if (threadIdx.x >= 32) {
-        asm volatile("bar.sync 7, 64;" ::: "memory");
-        if (*(volatile int *)&G.go) r1_walk(G.pair, G.pair.tab[lane] >> 26, *(volatile int *)&G.first, 0x7fffffff);
+        Ran1Warp h;
+        h.load(F.ran1);   // its powers of IA
+        asm volatile("bar.sync 7, 96;" ::: "memory");
+        if (!*(volatile int *)&G.go) return;
+        if (threadIdx.x < 64) r1_walk(G.pair, G.pair.tab[lane] >> 26, *(volatile int *)&G.first, 0x7fffffff);
+        else r1_make(G.pair, *(volatile int *)&G.idum, h.mul, 0x7fffffff);
         return;
     }
     volatile FxShared *vs = &S;
@@ -244,31 +242,22 @@ __device__ void fx_generate(const FxDev &F, FxGen &G, FxShared &S, unsigned long
     if (lane == 0) {
         r1_init(G.pair);
         *(volatile int *)&G.first = g.iy >> 26;
+        *(volatile int *)&G.idum = g.idum;
         *(volatile int *)&G.go = more;
     }
     __syncwarp();
-    asm volatile("bar.sync 7, 64;" ::: "memory");
+    asm volatile("bar.sync 7, 96;" ::: "memory");
     if (more) {
         R1Values v;
-        v.begin(G.pair, g);
-        constexpr int A = R1_NB / 2;   // batches made ahead
-#pragma unroll
-        for (int j = 0; j < A; ++j) v.make(G.pair, j);
-        for (int b = 0; more; b += A) {
-#pragma unroll
-            for (int j = 0; j < A; ++j) {
-                if (!more) continue;
-                more = room();
-                if (!more) continue;
-                if (!v.walked(G.pair, b + j)) {
-                    if (lane == 0) atomicExch(F.status, 1);
-                    more = false;
-                    continue;
-                }
-                checkpoint(v.idum, v.iy, G.pair.tab[lane]);
-                push(32, v.take(G.pair, b + j, j));
-                v.make(G.pair, j);
+        v.begin(g);
+        while (room()) {
+            if (!v.walked(G.pair)) {
+                if (lane == 0) atomicExch(F.status, 1);
+                break;
             }
+            if ((nb & (FX_CKE - 1)) == 0) checkpoint(v.idum(), v.iy(), G.pair.tab[lane]);
+            else ++nb;
+            push(32, v.take(G.pair));
         }
         v.leave(G.pair);
     }
@@ -308,9 +297,7 @@ __global__ void __launch_bounds__(T, 1) fitexp_cluster_kernel(FxDev F) {
     const int nsq = fx_nsq(nt, T);
     // [nsq*rpc]: ex4[q*rpc + r] = terms 4(FX_RQ+q)..4(FX_RQ+q)+3 of row r
     float4 *ex4 = (float4 *)fx_raw;
-    float *yr = (float *)(ex4 + (size_t)nsq * rpc);     // [rpc]
-    float *e1 = yr + rpc;                               // [rpc] sum over terms of |basis value|
-    size_t off = ((size_t)((unsigned char *)(e1 + rpc) - fx_raw) + 15) & ~(size_t)15;
+    size_t off = 16 * (size_t)nsq * rpc;
     float *wt = (float *)(fx_raw + off) + 3;            // wt[0..4*ntq]; wt + 1 is 16-byte aligned
     float *wtold = wt + 1 + 4 * (ntq + 4);                    // [nt+1]
     off = ((size_t)((unsigned char *)(wtold + nt + 1) - fx_raw) + 15) & ~(size_t)15;
@@ -320,8 +307,9 @@ __global__ void __launch_bounds__(T, 1) fitexp_cluster_kernel(FxDev F) {
     off = ((size_t)((unsigned char *)(ring + FX_RING) - fx_raw) + 15) & ~(size_t)15;
     float *gat = (float *)(fx_raw + off);               // [2][gstride] residuals by global row
     off = ((off + sizeof(float) * 2 * (size_t)fx_gstride(nw, rpc)) + 15) & ~(size_t)15;
-    double *parts = (double *)(fx_raw + off);           // [2][nw]
-    uint64_t *xbar = (uint64_t *)(parts + 2 * nw);      // [2]
+    const int nwr = (rpc + 31) / 32, nparts = nw * nwr; // warps of a CTA that have rows; their sums
+    double *parts = (double *)(fx_raw + off);           // [2][nparts]
+    uint64_t *xbar = (uint64_t *)(parts + 2 * nparts);  // [2]
 
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     volatile FxShared *vs = &S;
@@ -331,7 +319,7 @@ __global__ void __launch_bounds__(T, 1) fitexp_cluster_kernel(FxDev F) {
             S.done = 0;
         }
         cl.sync();
-        if (tid < 64) fx_generate(F, G, S, ring);
+        if (tid < 96) fx_generate(F, G, S, ring);
         __syncwarp();
         cl.sync();   // no CTA leaves while others may still write into its shared memory
         return;
@@ -348,16 +336,11 @@ __global__ void __launch_bounds__(T, 1) fitexp_cluster_kernel(FxDev F) {
         ex4[idx] = make_float4(e[0], e[1], e[2], e[3]);
     }
     for (int i = tid; i <= 4 * (ntq + 4); i += blockDim.x) wt[i] = 0.0f;   // terms past nterms stay zero
-    for (int r = tid; r < rpc; r += blockDim.x) {
-        float a = 0.0f;
-        for (int m = 0; m < nt && r < nrow; ++m) a = __fadd_ru(a, fabsf(F.expr[1 + (size_t)(row0 - 1 + r) * nt + m]));
-        e1[r] = a;
-    }
+    float e1 = 0.0f;                                    // this row's sum over terms of |basis value|
+    for (int m = 0; m < nt && tid < nrow; ++m) e1 = __fadd_ru(e1, fabsf(F.expr[1 + (size_t)(row0 - 1 + tid) * nt + m]));
     for (int i = tid; i < FX_RING; i += blockDim.x) ring[i] = 0ull;   // no position yet
-    if (tid < FX_WARPS) S.wmx[tid] = 0.0f;
     if (tid == 0) {
         S.abort = 0;
-        S.stop = 0;
         mbar_init(&xbar[0], 1);
         mbar_init(&xbar[1], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -367,7 +350,7 @@ __global__ void __launch_bounds__(T, 1) fitexp_cluster_kernel(FxDev F) {
 
     const float summax = exp_r(25.0f);
     const int K = nt - F.ncfirst + 1;                   // draws per trial
-    const int slot = tid, swarp = wid;                  // row / coefficient slot of this thread
+    const int slot = tid;                               // row / coefficient slot of this thread
     const int ic = slot < K ? F.ncfirst + slot : -1;   // coefficient this thread perturbs
     // the first FX_RQ quads of this thread's row (row `slot`), in registers for the launch
     float4 rq[FX_RQ];
@@ -391,10 +374,11 @@ __global__ void __launch_bounds__(T, 1) fitexp_cluster_kernel(FxDev F) {
         unsigned long long v = *e;
         if ((uint32_t)(v >> 32) != want) {
             const unsigned long long t0 = now_ns();
-            while (true) {
-                __nanosleep(32);
+            for (int n = 1;; ++n) {
                 v = *e;
-                if ((uint32_t)(v >> 32) == want || vs->abort) break;
+                if ((uint32_t)(v >> 32) == want) break;
+                if (n & 31) continue;
+                if (vs->abort) break;
                 if (now_ns() - t0 > FX_WAIT_NS) {
                     atomicExch(F.status, 1);
                     vs->abort = 1;
@@ -405,238 +389,218 @@ __global__ void __launch_bounds__(T, 1) fitexp_cluster_kernel(FxDev F) {
         return __uint_as_float((uint32_t)v);
     };
 
-    // state of the trial loop that thread 0's Metropolis decision reads (the same in every
-    // worker thread)
+    // state of the trial loop (the same in every worker thread)
     long long cursor = 0;
-    float chisqold = 0.0f, accept = 0.0f;
+    float chisqold = 0.0f, accept = 0.0f, racc = 0.0f;
     int icount = 0;
+    float yrow = 0.0f;                                  // this row's data
+    float wfix = 0.0f;                                  // largest |wt| of the unperturbed terms 1..ncfirst-1
 
-    // the largest |wt| over the perturbed terms, for the clamp bound (thread 0; a barrier
-    // follows before any row reads it)
+    // the largest |wt| over the perturbed terms (thread 0; a barrier follows)
     auto wmax_all = [&]() {
         float b = 0.0f;
         for (int m = F.ncfirst; m <= nt; ++m) b = fmaxf(b, fabsf(wt[m]));
-        vs->wmx[0] = b;
-        for (int k = 1; k < FX_WARPS; ++k) vs->wmx[k] = 0.0f;
+        vs->wmx = b;
     };
-    // the Metropolis test (:4871-4880) and the smoothing (:4882-4893) of trial chi^2 cn,
-    // taken by thread 0 and published in the control block
-    auto decide = [&](float cn) {
-        const float exponent = __fdiv_rn(__fsub_rn(cn, chisqold), accept);
-        float test;
-        int draw = 0;
-        if (exponent > 0.0f && exponent <= 20.0f) {
-            // the sign of exp(-x) - u: a fast exponential decides all but the near cases
-            const float u = get(cursor);
-            test = __expf(-exponent) - u;
-            if (fabsf(test) < 1.0e-4f) test = __fsub_rn(exp_r(-exponent), u);
-            draw = 1;
-        } else if (exponent > 20.0f) {
-            test = -1.0f;
-        } else {
-            test = 1.0f;
-        }
-        const int acc = test >= 0.0f;
-        int sm = 0;
-        if (acc && icount + 1 == F.nfreq) {
-            sm = 1;        // smoop(ncfirst, nterms, 1, wt)
-            const int n1 = F.ncfirst, n2 = nt;
-            if (!(n2 - 2 < n1)) {
-                float sm_ = 0.0f, sn = wt[n1];
-                float sum1 = __fmul_rn(0.25f, __fadd_rn(sm_, sn));
-                for (int i = n1; i <= n2; ++i) {
-                    sm_ = sn;
-                    sn = (i + 1) <= n2 ? wt[i + 1] : 0.0f;
-                    const float sum2 = __fmul_rn(0.25f, __fadd_rn(sm_, sn));
-                    wt[i] = __fadd_rn(sum1, sum2);
-                    sum1 = sum2;
-                }
+    // smoop(ncfirst, nterms, 1, wt) (:4882-4893; thread 0; a barrier follows)
+    auto smooth = [&]() {
+        const int n1 = F.ncfirst, n2 = nt;
+        if (!(n2 - 2 < n1)) {
+            float sm_ = 0.0f, sn = wt[n1];
+            float sum1 = __fmul_rn(0.25f, __fadd_rn(sm_, sn));
+            for (int i = n1; i <= n2; ++i) {
+                sm_ = sn;
+                sn = (i + 1) <= n2 ? wt[i + 1] : 0.0f;
+                const float sum2 = __fmul_rn(0.25f, __fadd_rn(sm_, sn));
+                wt[i] = __fadd_rn(sum1, sum2);
+                sum1 = sum2;
             }
-            wmax_all();
         }
-        vs->accept = acc;
-        vs->smooth = sm;
-        vs->draw = draw;
-        vs->stop = vs->abort;
-        // every worker has taken the values before `cursor` (its part of chi^2 is here), but the
-        // draw at `cursor` perhaps not yet
-        if (rank == 0) st_cl_s64(gen_cons, cursor);
+        wmax_all();
+    };
+    // The Metropolis test (:4871-4880) of trial chi^2 cn, u the stream's next value; draw: whether
+    // the test took it.  The sign of exp(-x) - u needs neither the division nor the exponential
+    // exact but near a tie.
+    auto metropolis = [&](float cn, float u, bool &draw) -> bool {
+        const float num = __fsub_rn(cn, chisqold);
+        draw = false;
+        if (num <= 0.0f && accept > 0.0f) return true;
+        const float x = __fmul_rn(num, racc);
+        if (x > 1.0e-30f && x < 19.9f) {
+            draw = true;
+            const float test = __expf(-x) - u;
+            if (fabsf(test) >= 1.0e-4f) return test > 0.0f;
+        }
+        const float exponent = __fdiv_rn(num, accept);
+        draw = exponent > 0.0f && exponent <= 20.0f;
+        if (draw) return __fsub_rn(exp_r(-exponent), u) >= 0.0f;
+        return !(exponent > 20.0f);
     };
 
     int xb = 0;                                         // exchange buffer
     uint32_t xph = 0u;                                  // mbarrier phase parity, bit b for buffer b
-    // chi^2 of the current wt over rows nmin..npt, the same value in every CTA, returned to
-    // all workers; with `trial`, thread 0 also takes the Metropolis decision on it before the
-    // result is published.  Rows, a worker barrier, then warp 0 alone: it forms this CTA's
-    // part, lane d pushes it into CTA d and arrives on CTA d's mbarrier (the nw pushes in
-    // parallel), lane 0 waits for every CTA's part and thread 0 forms the total in a fixed
-    // order; a second barrier publishes it.  strict_sum: the reference's sequential float sum
-    // over rows of the residuals that every row thread pushed to every CTA; else a double sum.
-    // yout, if given, receives this CTA's row sums.
-    auto chisq = [&](bool strict_sum, float *yout, bool trial) -> float {
+    // chi^2 of the current wt over rows nmin..npt, the same value in every worker thread of the
+    // cluster.  Every warp sums its rows and pushes the sum into every worker CTA (lane d into CTA d),
+    // the stores completing their bytes on that CTA's mbarrier; every warp waits there and forms the
+    // total for itself, in one fixed order, so no barrier of the CTA and no broadcast follows.
+    // strict_sum: the reference's sequential float sum over the residuals, which every row thread
+    // pushes to every CTA; else a double sum.  wmax: a bound on |wt|.  u, if given, receives the
+    // stream's next value while the sums travel.  yout, if given, receives this CTA's row sums.
+    // A buffer is written again two sums later, when every warp of the cluster has pushed its
+    // sum in between and so has read this one.
+    auto chisq = [&](bool strict_sum, float wmax, float *yout, float *u) -> float {
         float *gb = gat + (size_t)xb * fx_gstride(nw, rpc);
         double mypart = 0.0;
-        {
-            float wmax = vs->wfix;
-            const float *wm = (const float *)S.wmx;   // complete since the last barrier
+        if (slot < nrow) {
+            const int r = slot;
+            float sum = 0.0f;
+            const float4 *w4 = (const float4 *)(wt + 1);
+            const float4 *e4 = ex4 + r;
+            // every partial sum is at most e1 * wmax (times 1 + 2^-20 for rounding)
+            if (__fmul_ru(__fmul_ru(e1, wmax), 1.001f) < summax) {
+                // four quads at a time, the coefficients of the next four on their way: the
+                // additions are a chain, 4.7 cycles each, and loads that waited in it cost 30
+                float4 c[4];
 #pragma unroll
-            for (int k = 0; k < FX_WARPS; ++k) wmax = fmaxf(wmax, wm[k]);
-            if (slot < nrow) {
-                const int r = slot;
-                float sum = 0.0f;
-                const float4 *w4 = (const float4 *)(wt + 1);
-                const float4 *e4 = ex4 + r;
-                // every partial sum is at most e1[r] * max|wt| (times 1 + 2^-20 for rounding)
-                if (__fmul_ru(__fmul_ru(e1[r], wmax), 1.001f) < summax) {
-                    // four quads at a time, the coefficients of the next four on their way: the
-                    // additions are a chain, 4.7 cycles each, and loads that waited in it cost 30
-                    float4 c[4];
+                for (int j = 0; j < 4; ++j) c[j] = w4[j];
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) c[j] = w4[j];
+                for (int k = 0; k < FX_RQ; k += 4) {
+                    if (k < ntq) {
+                        float4 n[4];
 #pragma unroll
-                    for (int k = 0; k < FX_RQ; k += 4) {
-                        if (k < ntq) {
-                            float4 n[4];
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) n[j] = w4[k + 4 + j];
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) {
-                                sum = __fadd_rn(sum, __fmul_rn(rq[k + j].x, c[j].x));
-                                sum = __fadd_rn(sum, __fmul_rn(rq[k + j].y, c[j].y));
-                                sum = __fadd_rn(sum, __fmul_rn(rq[k + j].z, c[j].z));
-                                sum = __fadd_rn(sum, __fmul_rn(rq[k + j].w, c[j].w));
-                            }
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) c[j] = n[j];
-                        }
-                    }
-                    for (int q = 0; q < nsq; q += 4) {
-                        float4 n[4], f[4];
+                        for (int j = 0; j < 4; ++j) n[j] = w4[k + 4 + j];
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
-                            f[j] = e4[(q + j) * rpc];
-                            n[j] = w4[FX_RQ + q + 4 + j];
-                        }
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            sum = __fadd_rn(sum, __fmul_rn(f[j].x, c[j].x));
-                            sum = __fadd_rn(sum, __fmul_rn(f[j].y, c[j].y));
-                            sum = __fadd_rn(sum, __fmul_rn(f[j].z, c[j].z));
-                            sum = __fadd_rn(sum, __fmul_rn(f[j].w, c[j].w));
+                            sum = __fadd_rn(sum, __fmul_rn(rq[k + j].x, c[j].x));
+                            sum = __fadd_rn(sum, __fmul_rn(rq[k + j].y, c[j].y));
+                            sum = __fadd_rn(sum, __fmul_rn(rq[k + j].z, c[j].z));
+                            sum = __fadd_rn(sum, __fmul_rn(rq[k + j].w, c[j].w));
                         }
 #pragma unroll
                         for (int j = 0; j < 4; ++j) c[j] = n[j];
                     }
-                } else {  // the reference's clamped sum (expand :4924)
+                }
+                for (int q = 0; q < nsq; q += 4) {
+                    float4 n[4], f[4];
 #pragma unroll
-                    for (int k = 0; k < FX_RQ; ++k) {
-                        const float ev[4] = {rq[k].x, rq[k].y, rq[k].z, rq[k].w};
+                    for (int j = 0; j < 4; ++j) {
+                        f[j] = e4[(q + j) * rpc];
+                        n[j] = w4[FX_RQ + q + 4 + j];
+                    }
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const int m = 4 * k + j;
-                            if (m < nt) {
-                                sum = __fadd_rn(sum, __fmul_rn(ev[j], wt[1 + m]));
-                                if (fabsf(sum) > summax) sum = fsign(summax, sum);
-                            }
+                    for (int j = 0; j < 4; ++j) {
+                        sum = __fadd_rn(sum, __fmul_rn(f[j].x, c[j].x));
+                        sum = __fadd_rn(sum, __fmul_rn(f[j].y, c[j].y));
+                        sum = __fadd_rn(sum, __fmul_rn(f[j].z, c[j].z));
+                        sum = __fadd_rn(sum, __fmul_rn(f[j].w, c[j].w));
+                    }
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) c[j] = n[j];
+                }
+            } else {  // the reference's clamped sum (expand :4924)
+#pragma unroll
+                for (int k = 0; k < FX_RQ; ++k) {
+                    const float ev[4] = {rq[k].x, rq[k].y, rq[k].z, rq[k].w};
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const int m = 4 * k + j;
+                        if (m < nt) {
+                            sum = __fadd_rn(sum, __fmul_rn(ev[j], wt[1 + m]));
+                            if (fabsf(sum) > summax) sum = fsign(summax, sum);
                         }
                     }
-                    for (int m = 4 * FX_RQ; m < nt; ++m) {
-                        const float *ee = (const float *)(e4 + ((m >> 2) - FX_RQ) * rpc);
-                        sum = __fadd_rn(sum, __fmul_rn(ee[m & 3], wt[1 + m]));
-                        if (fabsf(sum) > summax) sum = fsign(summax, sum);
-                    }
                 }
-                const int i = row0 + r;
-                const float term = __fsub_rn(yr[r], sum);
-                const float q2 = __fmul_rn(term, term);
-                if (yout) yout[i] = sum;
-                if (strict_sum) {
-                    const uint32_t la = smem_addr(gb + (rank * rpc + r)), lb = smem_addr(&xbar[xb]);
-                    for (int d = 0; d < nw; ++d)
-                        st_async_f32(map_rank(la, (uint32_t)d), q2, map_rank(lb, (uint32_t)d));
-                } else if (i >= F.nmin) {
-                    mypart += (double)q2;
+                for (int m = 4 * FX_RQ; m < nt; ++m) {
+                    const float *ee = (const float *)(e4 + ((m >> 2) - FX_RQ) * rpc);
+                    sum = __fadd_rn(sum, __fmul_rn(ee[m & 3], wt[1 + m]));
+                    if (fabsf(sum) > summax) sum = fsign(summax, sum);
                 }
+            }
+            const int i = row0 + r;
+            const float term = __fsub_rn(yrow, sum);
+            const float q2 = __fmul_rn(term, term);
+            if (yout) yout[i] = sum;
+            if (strict_sum) {
+                const uint32_t la = smem_addr(gb + (rank * rpc + r)), lb = smem_addr(&xbar[xb]);
+                for (int d = 0; d < nw; ++d)
+                    st_async_f32(map_rank(la, (uint32_t)d), q2, map_rank(lb, (uint32_t)d));
+            } else if (i >= F.nmin) {
+                mypart = (double)q2;
             }
         }
         __syncwarp();
-        if (!strict_sum) {
+        const uint32_t ba = smem_addr(&xbar[xb]);
+        if (!strict_sum && wid < nwr) {
             mypart = warp_sum_d(mypart);
-            if (lane == 0) vs->red[wid] = mypart;
-            block_sync();
+            if (lane < nw)
+                st_async_f64(map_rank(smem_addr(parts + xb * nparts + rank * nwr + wid), (uint32_t)lane), mypart,
+                             map_rank(ba, (uint32_t)lane));
         }
-        if (wid == 0) {
-            const uint32_t ba = smem_addr(&xbar[xb]);
-            if (!strict_sum) {
-                double p[T / 32], t = 0.0;
-#pragma unroll
-                for (int k = 0; k < T / 32; ++k) p[k] = vs->red[k];
-#pragma unroll
-                for (int k = 0; k < T / 32; ++k) t += p[k];
-                if (lane < nw)
-                    st_async_f64(map_rank(smem_addr(parts + xb * nw + rank), (uint32_t)lane), t,
-                                 map_rank(ba, (uint32_t)lane));
-            }
-            if (lane == 0) {
-                // this CTA's own arrival, and the bytes that every worker sends it
-                mbar_expect(&xbar[xb], strict_sum ? 4u * (uint32_t)F.npt : 8u * (uint32_t)nw);
-                const uint32_t par = (xph >> xb) & 1u;
-                if (!mbar_test(ba, par)) {
-                    const unsigned long long t0 = now_ns();
-                    while (!mbar_test(ba, par)) {
-                        if (vs->abort || now_ns() - t0 > FX_WAIT_NS) {
-                            atomicExch(F.status, 1);
-                            vs->abort = 1;
-                            break;
-                        }
+        // this CTA's own arrival, and the bytes that every worker sends it
+        if (tid == 0) mbar_expect(&xbar[xb], strict_sum ? 4u * (uint32_t)F.npt : 8u * (uint32_t)nparts);
+        if (u) *u = get(cursor);
+        __syncwarp();
+        const uint32_t par = (xph >> xb) & 1u;
+        if (!__all_sync(0xffffffffu, mbar_test(ba, par))) {
+            const unsigned long long t0 = now_ns();
+            while (!__all_sync(0xffffffffu, mbar_test(ba, par))) {
+                if (__any_sync(0xffffffffu, vs->abort || now_ns() - t0 > FX_WAIT_NS)) {
+                    if (lane == 0) {
+                        atomicExch(F.status, 1);
+                        vs->abort = 1;
                     }
+                    break;
                 }
-                float v;
-                if (strict_sum) {
-                    // sequential, the words sixteen rows ahead on their way
-                    const int a = F.nmin - 1, b = F.npt;    // 0-based rows a..b-1
-                    float c = 0.0f;
-                    int i = a;
-                    for (; i < b && (i & 3); ++i) c = __fadd_rn(c, gb[i]);
-                    const float4 *g4 = (const float4 *)gb;
-                    const int q1 = b >> 2;
-                    int q = i >> 2;
-                    float4 u[4];
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) u[j] = g4[min(q + j, max(q1 - 1, 0))];
-                    for (; q + 4 <= q1; q += 4) {
-                        float4 n[4];
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) n[j] = g4[min(q + 4 + j, q1 - 1)];
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            c = __fadd_rn(c, u[j].x);
-                            c = __fadd_rn(c, u[j].y);
-                            c = __fadd_rn(c, u[j].z);
-                            c = __fadd_rn(c, u[j].w);
-                            u[j] = n[j];
-                        }
-                    }
-                    for (i = max(i, 4 * q); i < b; ++i) c = __fadd_rn(c, gb[i]);
-                    v = c;
-                } else {
-                    double p[FX_MAXW], u = 0.0;
-#pragma unroll
-                    for (int k = 0; k < FX_MAXW; ++k) p[k] = k < nw ? parts[xb * nw + k] : 0.0;
-#pragma unroll
-                    for (int k = 0; k < FX_MAXW; ++k)
-                        if (k < nw) u += p[k];
-                    v = (float)u;
-                }
-                vs->val = v;
-                if (trial) decide(v);
             }
+        }
+        float v;
+        if (strict_sum) {
+            // sequential, the words sixteen rows ahead on their way
+            const int a = F.nmin - 1, b = F.npt;    // 0-based rows a..b-1
+            float c = 0.0f;
+            int i = a;
+            for (; i < b && (i & 3); ++i) c = __fadd_rn(c, gb[i]);
+            const float4 *g4 = (const float4 *)gb;
+            const int q1 = b >> 2;
+            int q = i >> 2;
+            float4 w[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) w[j] = g4[min(q + j, max(q1 - 1, 0))];
+            for (; q + 4 <= q1; q += 4) {
+                float4 n[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) n[j] = g4[min(q + 4 + j, q1 - 1)];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    c = __fadd_rn(c, w[j].x);
+                    c = __fadd_rn(c, w[j].y);
+                    c = __fadd_rn(c, w[j].z);
+                    c = __fadd_rn(c, w[j].w);
+                    w[j] = n[j];
+                }
+            }
+            for (i = max(i, 4 * q); i < b; ++i) c = __fadd_rn(c, gb[i]);
+            v = c;
+        } else {
+            double t = 0.0;
+            for (int k = lane; k < nparts; k += 32) t += parts[xb * nparts + k];
+            v = (float)warp_sum_d(t);
         }
         xph ^= 1u << xb;
         xb ^= 1;
-        block_sync();
-        return vs->val;
+        return v;
     };
+    // A barrier of the worker CTA at which a wait that gave up in any thread ends the fit in all (a warp
+    // that gave up may have taken another branch than the rest; every barrier of the trials is this
+    // one, so all leave at the same one).
+    bool stop = false;
+    auto meet = [&]() -> bool {
+        __syncwarp();
+        stop = __syncthreads_or(vs->abort) != 0;
+        return stop;
+    };
+    // the largest |coefficient| a trial can reach from at most m: a step is stepr absolute below 1, relative above
+    auto reach = [&](float m, float stepr) { return fmaxf(wfix, 1.0001f * fmaxf(m + fabsf(stepr), m * (1.0f + fabsf(stepr)))); };
 
     const float acceptr = 0.05f;
     const int npoints = F.npt - F.nmin + 1;
@@ -645,19 +609,17 @@ __global__ void __launch_bounds__(T, 1) fitexp_cluster_kernel(FxDev F) {
         float *yout = F.yout + (size_t)pi * (F.npt + 1);
         const float *wto_g = F.wtold_g + (size_t)pi * (nt + 1);
         float *scal = F.scal + (size_t)pi * 4;
-        for (int r = tid; r < rpc; r += T) yr[r] = r < nrow ? yin[row0 + r] : 0.0f;
+        yrow = slot < nrow ? yin[row0 + slot] : 0.0f;
         for (int i = tid; i <= nt; i += T) {
             wtold[i] = wto_g[i];
             wt[i] = wtold[i];
         }
         block_sync();
-        if (tid == 0) {
-            float a = 0.0f;
-            for (int m = 1; m < F.ncfirst; ++m) a = fmaxf(a, fabsf(wt[m]));
-            vs->wfix = a;
-            wmax_all();
-        }
+        wfix = 0.0f;
+        for (int m = 1; m < F.ncfirst; ++m) wfix = fmaxf(wfix, fabsf(wt[m]));
+        if (tid == 0) wmax_all();
         block_sync();
+        float wmx = vs->wmx;                         // bound on |wtold| of the perturbed terms
         float stepr = scal[0];
         float rejrat = scal[2];
         float chisqnew = scal[3];
@@ -668,57 +630,56 @@ __global__ void __launch_bounds__(T, 1) fitexp_cluster_kernel(FxDev F) {
             wtmax = (a >= wtmax) ? a : wtmax;
         }
         if (stepr < __fmul_rn(1.0e-6f, wtmax)) stepr = __fmul_rn(2.0e-6f, wtmax);
-        if (F.nits > 0 && !vs->stop) {
+        if (F.nits > 0 && !stop) {
             icount = 0;
-            chisqnew = chisq(F.strict != 0, nullptr, false);
+            chisqnew = chisq(F.strict != 0, fmaxf(wfix, wmx), nullptr, nullptr);
             chisqold = chisqnew;
             float chisqtest = -1.0f;
             int itry = 0;
-            bool stop = false;
+            float wo = ic > 0 ? wtold[ic] : 0.0f;       // this thread's coefficient
             while (!stop && (itry < 10 || (itry < 150 && chisqtest < 1.0e-4f))) {
                 ++itry;
                 accept = __fdiv_rn(__fmul_rn(acceptr, chisqold), (float)npoints);
+                racc = __fdiv_rn(1.0f, accept);
                 rejrat = 0.0f;
                 const float chisqstart = __fdiv_rn(chisqold, (float)npoints);
                 for (int st = 1; st <= 100; ++st) {
                     ++trials;
                     // perturb coefficients ncfirst..nterms with the next K values (:4856-4861),
                     // each thread waiting for its own value
-                    if (swarp * 32 < K) {
-                        float a = 0.0f;
-                        if (ic > 0) {
-                            const float du = __fsub_rn(__fmul_rn(2.0f, get(cursor + slot)), 1.0f);
-                            float v;
-                            if (fabsf(wtold[ic]) < 1.0f) v = __fadd_rn(wtold[ic], __fmul_rn(stepr, du));
-                            else v = __fmul_rn(wtold[ic], __fadd_rn(1.0f, __fmul_rn(stepr, du)));
-                            wt[ic] = v;
-                            a = fabsf(v);
-                        }
-                        a = __int_as_float((int)__reduce_max_sync(0xffffffffu, (unsigned)__float_as_int(a)));
-                        if (lane == 0) vs->wmx[swarp] = a;
+                    float wn = 0.0f;
+                    if (ic > 0) {
+                        const float du = __fsub_rn(__fmul_rn(2.0f, get(cursor + slot)), 1.0f);
+                        if (fabsf(wo) < 1.0f) wn = __fadd_rn(wo, __fmul_rn(stepr, du));
+                        else wn = __fmul_rn(wo, __fadd_rn(1.0f, __fmul_rn(stepr, du)));
+                        wt[ic] = wn;
                     }
                     cursor += K;
-                    block_sync();
-                    // chi^2 of the trial and thread 0's decision on it (Metropolis, smoothing)
-                    const float cn = chisq(F.strict != 0, nullptr, true);
-                    const int acc = vs->accept, sm = vs->smooth;
-                    stop = vs->stop != 0;
-                    cursor += vs->draw;
-                    chisqnew = cn;
+                    if (meet()) break;
+                    float u;
+                    const float bound = reach(wmx, stepr);
+                    chisqnew = chisq(F.strict != 0, bound, nullptr, &u);
+                    bool draw;
+                    const bool acc = metropolis(chisqnew, u, draw);
+                    // every worker has taken the values before `cursor` (its part of chi^2 is here),
+                    // but the draw at `cursor` perhaps not yet
+                    if (rank == 0 && tid == 0) st_cl_s64(gen_cons, cursor);
+                    cursor += draw;
                     if (acc) {
-                        ++icount;
-                        if (sm) {
+                        wo = wn;
+                        wmx = bound;
+                        if (++icount == F.nfreq) {
                             icount = 0;
-                            chisqnew = chisq(F.strict != 0, nullptr, false);
+                            if (tid == 0) smooth();
+                            if (meet()) break;
+                            wmx = vs->wmx;
+                            if (ic > 0) wo = wt[ic];
+                            chisqnew = chisq(F.strict != 0, fmaxf(wfix, wmx), nullptr, nullptr);
                         }
                         chisqold = chisqnew;
-                        // each thread keeps the coefficient it perturbs (terms below ncfirst
-                        // never change); the next trial's perturbation reads only its own
-                        if (ic > 0) wtold[ic] = wt[ic];
                     } else {
                         rejrat = __fadd_rn(rejrat, 1.0f);
                     }
-                    if (stop) break;
                 }
                 rejrat = __fdiv_rn(rejrat, 100.0f);
                 const float chisqfinish = __fdiv_rn(chisqold, (float)npoints);
@@ -727,14 +688,17 @@ __global__ void __launch_bounds__(T, 1) fitexp_cluster_kernel(FxDev F) {
                 const float rejfac = rejrat > 0.0f ? __fdiv_rn(0.75f, rejrat) : 2.0f;
                 stepr = __fmul_rn(stepr, rejfac);
             }
-            block_sync();   // every thread's own wtold update is in
+            block_sync();
+            if (ic > 0) wtold[ic] = wo;   // terms below ncfirst never change
+            block_sync();
             for (int k = 1 + tid; k <= nt; k += T) wt[k] = wtold[k];
             block_sync();
             if (tid == 0) wmax_all();
             block_sync();
+            wmx = vs->wmx;
         }
         // final fit over rows 1..npt, chi^2 from nmin (:4908-4914), in the reference's order
-        chisqnew = chisq(true, yout, false);
+        chisqnew = chisq(true, fmaxf(wfix, wmx), yout, nullptr);
         if (rank == 0) {
             float *wt_g = F.wt_g + (size_t)pi * (nt + 1);
             float *wtold_o = F.wtold_g + (size_t)pi * (nt + 1);
@@ -770,7 +734,7 @@ static inline size_t al256f(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // Worker CTAs: as many as give each FX_ROWS rows (a trial's rows are summed side by side, so the
 // fewer a CTA has the shorter the trial; 600 rows x 116 terms, double sums: 5,370 cycles a trial on
-// two CTAs with the stream's warp among their own, 3,360 now, the length of its 117 values), up to seven beside
+// two CTAs with the stream's warp among their own, 3,240 now), up to seven beside
 // the generator's CTA, the portable cluster size; more only for rows that need the memory.  Rows
 // and terms for 256 threads: barriers of half the warps, and registers for the whole row.
 static int fx_workers(int npt, int nterms, int ncoef, int *rpc_out, int *threads_out) {

@@ -234,7 +234,7 @@ __global__ void spec_plan_kernel(SpecDev S) {
             reinterpret_cast<int4 *>(to)[i] = reinterpret_cast<const int4 *>(from)[i];
         for (int i = 4 * quads + tid; i < count; i += blockDim.x) to[i] = from[i];
     }
-    if (ok || count == 0 || tid >= 64) return;
+    if (ok || count == 0 || tid >= 96) return;
     __shared__ R1Ring ring;
     __shared__ int32_t tab[34];
     const int32_t mcall = S.ran1[2];
@@ -1223,7 +1223,7 @@ namespace epsr {
 // between, the cycle was redone by the sequential kernel, the caller set a new state) it
 // walks the stream itself.  Either way it draws the same values.
 
-__global__ void __launch_bounds__(64) ahead_fill_kernel(const int32_t *state, int32_t *ahead, const int32_t *count) {
+__global__ void __launch_bounds__(96) ahead_fill_kernel(const int32_t *state, int32_t *ahead, const int32_t *count) {
     __shared__ R1Ring ring;
     __shared__ int32_t tab[34];
     const int lane = threadIdx.x & 31;
@@ -1471,7 +1471,7 @@ int epsr_molfit_spec(const epsr_box_t *box, const epsr_cells_t *cells, epsr_stor
         // the SM to itself for the 2-3 ms it runs
         EPSR_SMEM_OPTIN(ahead_fill_kernel);
         EPSR_TIMED("ahead_fill_kernel", as->st,
-                   ahead_fill_kernel<<<1, 64, g_ahead_smem, as->st>>>(S.ran1_next, mc->ahead, S.off + N));
+                   ahead_fill_kernel<<<1, 96, g_ahead_smem, as->st>>>(S.ran1_next, mc->ahead, S.off + N));
         EPSR_CUDA(cudaGetLastError());
         EPSR_CUDA(cudaEventRecord(as->join, as->st));
     }

@@ -1,6 +1,6 @@
 // ran1.cu -- device ran1 stream (auxiliary_routines.py:324-391), bit-identical.
 //
-// Two warps produce the sequence (ran1_pair.cuh).  The Park-Miller part is jumped ahead so that
+// Three warps produce the sequence (ran1_pair.cuh).  The Park-Miller part is jumped ahead so that
 // lane l holds idum after l+1 more steps (Schrage's method computes IA*idum mod IM exactly, so
 // a 64-bit modular product with IA^k gives the same value).  The Bays-Durham shuffle is an
 // inherently sequential pointer chase; its 32-entry table lives one entry per lane and is walked
@@ -14,7 +14,7 @@
 
 namespace epsr {
 
-__global__ void __launch_bounds__(64) ran1_fill_kernel(int32_t *state, float *out, int64_t n) {
+__global__ void __launch_bounds__(96) ran1_fill_kernel(int32_t *state, float *out, int64_t n) {
     __shared__ R1Ring ring;
     __shared__ int32_t tab[34];
     const int lane = threadIdx.x & 31;
@@ -38,7 +38,7 @@ extern "C" int epsr_ran1_fill(int32_t *state, float *out, int64_t n, void *strea
         return EPSR_ERR_ARG;
     }
     if (n == 0) return EPSR_OK;
-    epsr::ran1_fill_kernel<<<1, 64, 0, (cudaStream_t)stream>>>(state, out, n);
+    epsr::ran1_fill_kernel<<<1, 96, 0, (cudaStream_t)stream>>>(state, out, n);
     EPSR_CUDA(cudaGetLastError());
     return EPSR_OK;
 }
