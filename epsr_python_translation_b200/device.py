@@ -38,10 +38,12 @@ def press_scalars(nmol, sumc, presst, simt, volume):
 
 
 def table_cutoff(*tabs) -> int:
-    """Last grid index at which any table entry is nonzero (bitwise, so -0 counts)."""
+    """Last grid index at which any table entry is nonzero.  A -0 entry counts as zero: beyond this
+    index an interpolated energy is a zero of either sign, which changes no sum (every sum starts
+    at +0) and no test for a nonzero pair energy."""
     last = 1
     for t in tabs:
-        nz = np.nonzero(np.any(np.ascontiguousarray(t, dtype=f32).view(np.uint32) != 0, axis=0))[0]
+        nz = np.nonzero(np.any(np.ascontiguousarray(t, dtype=f32) != 0, axis=0))[0]
         if nz.size:
             last = max(last, int(nz[-1]))
     return last
