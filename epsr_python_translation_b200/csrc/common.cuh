@@ -442,7 +442,25 @@ struct Ran1Warp {
     }
 };
 
-// ----------------------------------------------------------------- reductions
+// ----------------------------------------------------------------- scans and reductions
+// Exclusive scan of one count a thread across the block (up to 32 warps); *total = the block's sum
+// in every thread.  Every warp sums the warps before it for itself.
+__device__ __forceinline__ int block_scan(int v, int *total) {
+    __shared__ int ws[32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+    int incl = v;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+    }
+    if (lane == 31) ws[wid] = incl;
+    __syncthreads();
+    const int w = lane < nw ? ws[lane] : 0;
+    *total = __reduce_add_sync(0xffffffffu, w);
+    const int before = __reduce_add_sync(0xffffffffu, lane < wid ? w : 0);
+    __syncthreads();
+    return before + incl - v;
+}
 __device__ __forceinline__ double warp_sum_d(double v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

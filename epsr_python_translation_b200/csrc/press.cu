@@ -8,7 +8,8 @@
 // back as float32 -- exactly as the reference (:3960-4040).  Pairs count only while the
 // bin iz <= npt1.  The reduction then sums ergold in float32 and ergnew in double over
 // (im, slot) in store order (:4041-4044): one thread, sequentially, for the reference's
-// bits (strict), or in parallel in double (fast).
+// bits (strict); or the CTA adds its molecule's terms in double and one CTA the molecules (fast: no
+// term goes through memory.  814,000 pairs: 340 us for both kernels, 777 us with one CTA over all terms).
 #include <string.h>
 
 #include "common.cuh"
@@ -22,7 +23,7 @@ struct PressDev {
     Lattice L;
     const float4 *tab;         // [npairs*ld] {xavs, xavs1, ecoul, ecoul1}
     const float *xstar;        // [ld]
-    float stepcl;
+    float stepcl, rcp;         // and step_rcp of it
     int npt1, ld, ntype, M;
     const int32_t *naf, *nato, *npairref, *nergpairm, *molergpair;
     const float *xadd, *yadd, *zadd;
@@ -31,7 +32,61 @@ struct PressDev {
     double *sums;              // [2] {sumc, presst}
 };
 
-__global__ void __launch_bounds__(PR_THREADS) press_pairs_kernel(PressDev P) {
+// a double in two words of a float array (rows of odd length leave them unaligned)
+__device__ __forceinline__ void put_double(float *p, double v) {
+    p[0] = __int_as_float(__double2loint(v));
+    p[1] = __int_as_float(__double2hiint(v));
+}
+__device__ __forceinline__ double get_double(const float *p) {
+    return __hiloint2double(__float_as_int(p[1]), __float_as_int(p[0]));
+}
+
+// x - nint(x) (half away from zero) of a difference of box-fraction coordinates, on the adder
+__device__ __forceinline__ float wrap_small(float x) {
+    const float r = __fsub_rn(x, rint_small(x));
+    return fabsf(r) == 0.5f ? copysignf(0.5f, -x) : r;
+}
+
+// one atom pair's terms; branch-free: the tables are read at iz clamped into 2..npt1 and `in` tells
+// whether the pair counts, so several pairs' loads are in flight
+struct PairTerms {
+    float enwt, enpot, prwt, prpot;
+    bool in;
+};
+template <bool CUBIC>
+__device__ __forceinline__ PairTerms pair_terms(const PressDev &P, float4 p1, float4 p2, const int32_t *prow, float xc,
+                                                float yc, float zc) {
+    float xdif = __fsub_rn(p2.x, p1.x), ydif = __fsub_rn(p2.y, p1.y), zdif = __fsub_rn(p2.z, p1.z);
+    if (CUBIC) {
+        xdif = wrap_small(xdif);
+        ydif = wrap_small(ydif);
+        zdif = wrap_small(zdif);
+    } else {
+        minimagec(P.L, xdif, ydif, zdif);
+    }
+    const float dsq = __fadd_rn(__fadd_rn(__fmul_rn(xdif, xdif), __fmul_rn(ydif, ydif)), __fmul_rn(zdif, zdif));
+    const float dtest = CUBIC ? sqrt_unit(dsq) : __fsqrt_rn(dsq);
+    const int iz = (CUBIC ? bin_index(dtest, P.stepcl, P.rcp) : ifix(__fdiv_rn(dtest, P.stepcl))) + 2;
+    const int izc = min(max(iz, 2), P.npt1);
+    const int icref = __ldg(prow + __float_as_int(p2.w));
+    const float4 t = __ldg(P.tab + (size_t)icref * P.ld + izc);       // bin iz
+    const float4 tm = __ldg(P.tab + (size_t)icref * P.ld + izc - 1);  // bin iz-1
+    const float dtdif = __fsub_rn(dtest, __ldg(P.xstar + izc));
+    const float prfac = dtest > 0.0f ? __fdiv_rn(__fadd_rn(__fadd_rn(__fmul_rn(xc, xdif), __fmul_rn(yc, ydif)),
+                                                           __fmul_rn(zc, zdif)),
+                                                 dtest)
+                                     : 0.0f;
+    PairTerms r;
+    r.in = iz == izc;
+    r.enpot = __fadd_rn(t.z, __fmul_rn(t.w, dtdif));
+    r.prpot = __fmul_rn(__fmul_rn(0.5f, __fadd_rn(t.w, tm.w)), prfac);
+    r.enwt = __fadd_rn(t.x, __fmul_rn(t.y, dtdif));
+    r.prwt = __fmul_rn(__fmul_rn(0.5f, __fadd_rn(t.y, tm.y)), prfac);
+    return r;
+}
+
+template <bool CUBIC>
+__global__ void __launch_bounds__(PR_THREADS) press_pairs_kernel(PressDev P, int fast) {
     extern __shared__ int list[];   // [M] slots with a partner jm > im, by partner atom count
     __shared__ float4 sa[PR_MAXAT];
     __shared__ int bk[PR_MAXAT + 2];
@@ -90,40 +145,47 @@ __global__ void __launch_bounds__(PR_THREADS) press_pairs_kernel(PressDev P) {
             for (int ia = 0; ia < na; ++ia) {
                 const float4 p1 = in_smem ? sa[ia] : __ldg(P.pos + a0 + ia);
                 const int32_t *prow = P.npairref + __float_as_int(p1.w) * P.ntype;
-                for (int ja = 0; ja < nb; ++ja) {
-                    const float4 p2 = __ldg(P.pos + b0 + ja);
-                    float xdif = __fsub_rn(p2.x, p1.x), ydif = __fsub_rn(p2.y, p1.y), zdif = __fsub_rn(p2.z, p1.z);
-                    minimagec(P.L, xdif, ydif, zdif);
-                    const float dsq =
-                        __fadd_rn(__fadd_rn(__fmul_rn(xdif, xdif), __fmul_rn(ydif, ydif)), __fmul_rn(zdif, zdif));
-                    const float dtest = __fsqrt_rn(dsq);
-                    const int iz = ifix(__fdiv_rn(dtest, P.stepcl)) + 2;
-                    // branch-free: tables read at iz clamped into 2..npt1, the sums kept unchanged
-                    // outside that range, so consecutive pairs' loads can be in flight together
-                    const bool in = iz >= 2 && iz <= P.npt1;
-                    const int izc = min(max(iz, 2), P.npt1);
-                    const int icref = __ldg(prow + __float_as_int(p2.w));
-                    const float4 t = __ldg(P.tab + (size_t)icref * P.ld + izc);       // bin iz
-                    const float4 tm = __ldg(P.tab + (size_t)icref * P.ld + izc - 1);  // bin iz-1
-                    const float dtdif = __fsub_rn(dtest, __ldg(P.xstar + izc));
-                    const float prfac =
-                        dtest > 0.0f ? __fdiv_rn(__fadd_rn(__fadd_rn(__fmul_rn(xcdif, xdif), __fmul_rn(ycdif, ydif)),
-                                                           __fmul_rn(zcdif, zdif)),
-                                                 dtest)
-                                     : 0.0f;
-                    const float enpot = __fadd_rn(t.z, __fmul_rn(t.w, dtdif));
-                    const double prpot = (double)__fmul_rn(__fmul_rn(0.5f, __fadd_rn(t.w, tm.w)), prfac);
-                    const float enwt = __fadd_rn(t.x, __fmul_rn(t.y, dtdif));
-                    const float prwt = __fmul_rn(__fmul_rn(0.5f, __fadd_rn(t.y, tm.y)), prfac);
-                    const float eo2 = __fadd_rn(__fadd_rn(eo, enwt), enpot);
-                    const float en2 = __double2float_rn(__dadd_rn((double)__fadd_rn(en, prwt), prpot));
-                    eo = in ? eo2 : eo;
-                    en = in ? en2 : en;
+#pragma unroll 2
+                for (int j = 0; j < nb; ++j) {
+                    const PairTerms t = pair_terms<CUBIC>(P, p1, __ldg(P.pos + b0 + j), prow, xcdif, ycdif, zcdif);
+                    if (t.in) {
+                        // the reference adds the float32 prwt and then, in double, prpot, and stores
+                        // float32: a float added to a float in double and rounded to float is the
+                        // float sum (exact in double unless the smaller is below 2^-29 of the larger,
+                        // when both round to the larger)
+                        eo = __fadd_rn(__fadd_rn(eo, t.enwt), t.enpot);
+                        en = __fadd_rn(__fadd_rn(en, t.prwt), t.prpot);
+                    }
                 }
             }
         }
         P.ergold[row + s] = eo;
         P.ergnew[row + s] = en;
+    }
+    if (!fast) return;
+    // the molecule's sums, by slot, so that they don't depend on the lists' order
+    __shared__ double r0[PR_THREADS / 32], r1[PR_THREADS / 32];
+    __syncthreads();
+    double se = 0.0, sp = 0.0;
+    for (int s = threadIdx.x; s < nn; s += blockDim.x) {
+        se += (double)P.ergold[row + s];
+        sp += (double)P.ergnew[row + s];
+    }
+    se = warp_sum_d(se);
+    sp = warp_sum_d(sp);
+    if ((threadIdx.x & 31) == 0) {
+        r0[threadIdx.x >> 5] = se;
+        r1[threadIdx.x >> 5] = sp;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && P.M >= 2) {   // into the row's first two words of each array, now read
+        double a = 0.0, b = 0.0;
+        for (int w = 0; w < PR_THREADS / 32; ++w) {
+            a += r0[w];
+            b += r1[w];
+        }
+        put_double(P.ergold + row, a);
+        put_double(P.ergnew + row, b);
     }
 }
 
@@ -143,20 +205,16 @@ __global__ void press_sum_strict_kernel(PressDev P, int nmol) {
     P.sums[1] = presst;
 }
 
-// both sums in double, in parallel (one CTA; a fixed order, so the result is reproducible):
-// warp w takes molecules w, w+32, ..., its lanes the slots of each
+// both sums over the molecules' in double (one CTA, a fixed order)
 __global__ void __launch_bounds__(1024) press_sum_fast_kernel(PressDev P, int nmol) {
     __shared__ double r0[32], r1[32];
     double a = 0.0, b = 0.0;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-    for (int im = wid; im < nmol - 1; im += nwarp) {
-        const size_t row = (size_t)im * P.M;
-        const int nn = P.nergpairm[im];
-        for (int s = lane; s < nn; s += 32) {
-            a += (double)P.ergold[row + s];
-            b += (double)P.ergnew[row + s];
+    if (P.M >= 2)   // a row of one slot holds no other molecule
+        for (int im = threadIdx.x; im < nmol - 1; im += blockDim.x) {
+            a += get_double(P.ergold + (size_t)im * P.M);
+            b += get_double(P.ergnew + (size_t)im * P.M);
         }
-    }
     a = warp_sum_d(a);
     b = warp_sum_d(b);
     if (lane == 0) {
@@ -213,6 +271,7 @@ extern "C" int epsr_press(const epsr_box_t *box, const epsr_store_t *store, int3
     P.tab = (const float4 *)box->tab;
     P.xstar = box->xstar;
     P.stepcl = box->stepcl;
+    P.rcp = step_rcp(box->stepcl, npt1);
     P.npt1 = npt1;
     P.ld = box->ld;
     P.ntype = box->ntype;
@@ -236,8 +295,12 @@ extern "C" int epsr_press(const epsr_box_t *box, const epsr_store_t *store, int3
     if (rc) return rc;
     if (nmol > 1) {
         const size_t list_bytes = sizeof(int) * (size_t)M;
-        if (list_bytes > 48 * 1024) EPSR_SMEM_OPTIN(press_pairs_kernel);
-        press_pairs_kernel<<<nmol - 1, PR_THREADS, list_bytes, s>>>(P);
+        if (list_bytes > 48 * 1024) {
+            EPSR_SMEM_OPTIN(press_pairs_kernel<true>);
+            EPSR_SMEM_OPTIN(press_pairs_kernel<false>);
+        }
+        auto *pairs = box->cubic ? press_pairs_kernel<true> : press_pairs_kernel<false>;
+        pairs<<<nmol - 1, PR_THREADS, list_bytes, s>>>(P, strict ? 0 : 1);
         EPSR_CUDA(cudaGetLastError());
         if (strict) press_sum_strict_kernel<<<1, 1, 0, s>>>(P, nmol);
         else press_sum_fast_kernel<<<1, 1024, 0, s>>>(P, nmol);

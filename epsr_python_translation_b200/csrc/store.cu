@@ -19,6 +19,7 @@
 namespace epsr {
 
 constexpr int FM_THREADS = 256;   // threads of a visit position's CTA (its region entries)
+constexpr int FM_WRITE = 8;       // entries a thread writes in a row
 constexpr int FM_MAXAT = 64;      // atom-count buckets of the evaluation list (larger share the last)
 
 struct BoxDev {
@@ -29,17 +30,30 @@ struct BoxDev {
     int ntype;
 };
 
-__device__ __forceinline__ float en_mole_pair_dev(const BoxDev &B, int im, int jm) {
+// en_mole_pair: the sum over (ia, ja) in the reference's order.  Four pairs' loads and energies are in
+// flight before their ordered additions.
+template <bool CUBIC>
+__device__ __forceinline__ float en_mole_pair_dev(const BoxDev &B, float rcp, int im, int jm) {
     float sume = 0.0f;
     const int a0 = B.naf[im], a1 = a0 + B.nato[im];
-    const int b0 = B.naf[jm], b1 = b0 + B.nato[jm];
+    const int b0 = B.naf[jm], nb = B.nato[jm];
     for (int ia = a0; ia < a1; ++ia) {
-        const float4 p1 = B.pos[ia];
-        const int it = __float_as_int(p1.w);
-        for (int ja = b0; ja < b1; ++ja) {
-            const float4 p2 = B.pos[ja];
-            const int icref = __ldg(B.npairref + it * B.ntype + __float_as_int(p2.w));
-            sume = __fadd_rn(sume, pair_energy(B.L, B.T, p1, p2, icref));
+        const float4 p1 = __ldg(B.pos + ia);
+        const int32_t *row = B.npairref + __float_as_int(p1.w) * B.ntype;
+        for (int j = 0; j < nb; j += 4) {
+            float e[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                e[u] = 0.0f;
+                if (j + u < nb) {
+                    const float4 p2 = __ldg(B.pos + b0 + j + u);
+                    const int icref = __ldg(row + __float_as_int(p2.w));
+                    e[u] = CUBIC ? pair_energy_unit(B.T, rcp, p1, p2, icref) : pair_energy(B.L, B.T, p1, p2, icref);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (j + u < nb) sume = __fadd_rn(sume, e[u]);
         }
     }
     return sume;
@@ -49,33 +63,6 @@ __device__ __forceinline__ int fold(int x, int n) {
     while (x < 0) x += n;
     while (x >= n) x -= n;
     return x;
-}
-
-// Block-wide exclusive scan (<= 32 warps); *total = block sum.
-__device__ __forceinline__ int bscan(int v, int *total) {
-    __shared__ int ws[32];
-    __shared__ int wp[33];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-    int incl = v;
-    for (int o = 1; o < 32; o <<= 1) {
-        int t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += t;
-    }
-    if (lane == 31) ws[wid] = incl;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int a = 0;
-        for (int w = 0; w < nw; ++w) {
-            wp[w] = a;
-            a += ws[w];
-        }
-        wp[32] = a;
-    }
-    __syncthreads();
-    int r = wp[wid] + incl - v;
-    *total = wp[32];
-    __syncthreads();
-    return r;
 }
 
 // (1) region list of every cell (make_neighbour_list_from_cells cellneighbourlist.py:187)
@@ -97,7 +84,7 @@ __global__ void region_build_kernel(const int32_t *start, const int32_t *mols, c
             cnt = start[cell + 1] - start[cell];
         }
         int tot;
-        int pre = bscan(cnt, &tot);
+        int pre = block_scan(cnt, &tot);
         if (k < noff) {
             sh[2 * k] = cell;
             sh[2 * k + 1] = carry + pre;
@@ -120,72 +107,105 @@ __global__ void region_build_kernel(const int32_t *start, const int32_t *mols, c
 struct Prefilter {
     int on;
     float cut;          // (izcut-1)*stepcl with margin, box units
-    const float *rad;   // [nmol] molecule radius (box units)
-    const float *xadd, *yadd, *zadd;
+    const float4 *ctr;  // [nmol] centre and radius (box units)
 };
 
-__device__ __forceinline__ bool far_apart(const Prefilter &P, int im, int jm) {
-    if (!P.on) return false;
-    float xd = P.xadd[jm] - P.xadd[im], yd = P.yadd[jm] - P.yadd[im], zd = P.zadd[jm] - P.zadd[im];
-    xd -= rintf(xd);
-    yd -= rintf(yd);
-    zd -= rintf(zd);
-    float d = sqrtf(xd * xd + yd * yd + zd * zd);
-    return d - P.rad[im] - P.rad[jm] > P.cut;
+// certainly beyond the cutoff: the centres' distance exceeds it and both radii (its square with a margin
+// for the roundings)
+__device__ __forceinline__ bool far_apart(const Prefilter &P, float4 c, int jm) {
+    const float4 o = __ldg(P.ctr + jm);
+    const float xd = o.x - c.x, yd = o.y - c.y, zd = o.z - c.z;
+    const float reach = P.cut + c.w + o.w;
+    return wrap_sq_small(xd) + wrap_sq_small(yd) + wrap_sq_small(zd) > reach * reach * 1.00001f;
 }
 
 // (2) the pair energies of each visit position's region entries (0 where not evaluated),
-// and the count of nonzero ones
+// and the count of nonzero ones.  What bounds it: the reads that decide which of the region's
+// entries are near (one in ten), then the energies, a thread a molecule pair.  An entry is looked at
+// once, its answer kept as a bit and a count, and four are in flight.  8,000 molecules of DMSO and water,
+// regions of 2,000, 12 A: 346 us; about 530 us looking twice, with the division and one pair at a time.
+template <bool CUBIC>
 __global__ void __launch_bounds__(FM_THREADS) fm_count_kernel(BoxDev B, Prefilter P, const int32_t *visit,
                                                               const int32_t *molcellno, const int32_t *reg,
-                                                              const int32_t *nn, int M, float *ebuf, int32_t *cnt) {
+                                                              const int32_t *nn, int M, float rcp, float *ebuf,
+                                                              int32_t *cnt) {
     extern __shared__ int list[];   // [M] region entries to evaluate, by partner atom count
     __shared__ int bk[FM_MAXAT + 2];
+    __shared__ int nonzero;
     const int v = blockIdx.x;
     const int im = visit[v];
     const int c = molcellno[im] - 1;
     const int n = nn[c];
+    const int32_t *rg = reg + (size_t)c * M;
+    float *eb = ebuf + (size_t)v * M;
     for (int i = threadIdx.x; i < FM_MAXAT + 2; i += blockDim.x) bk[i] = 0;
+    if (threadIdx.x == 0) nonzero = 0;
+    if (n <= 1) {   // the molecule itself: no entry
+        if (threadIdx.x == 0) cnt[v] = 0;
+        return;
+    }
+    const float4 ctr = P.on ? P.ctr[im] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     __syncthreads();
     // entries evaluated: partner later in molecule order and not certainly beyond the cutoff;
     // the others store 0.  Listing them by the partner's atom count gives the lanes of a warp
     // loops of the same length.
-    auto nb_of = [&](int inn) -> int {
-        const int jm = reg[(size_t)c * M + inn];
-        return (jm > im && !far_apart(P, im, jm)) ? min(B.nato[jm], FM_MAXAT) : 0;
-    };
-    for (int inn = 1 + threadIdx.x; inn < n; inn += blockDim.x) {
-        const int nb = nb_of(inn);
-        if (nb > 0) atomicAdd(&bk[nb], 1);
-        else ebuf[(size_t)v * M + inn] = 0.0f;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {   // bk[b] -> first list position of atom count b; bk[FM_MAXAT+1] = total
-        int a = 0;
-        for (int b = 0; b <= FM_MAXAT; ++b) {
-            const int t = bk[b];
-            bk[b] = a;
-            a += t;
+    auto near = [&](int jm) -> bool { return jm > im && !(P.on && far_apart(P, ctr, jm)); };
+    unsigned mask = 0;   // this thread's first 32 entries
+#pragma unroll 4
+    for (int i = 0; i < 32; ++i) {
+        const int inn = 1 + (int)threadIdx.x + FM_THREADS * i;
+        if (inn >= n) break;
+        const int jm = __ldg(rg + inn);
+        if (near(jm)) {
+            mask |= 1u << i;
+            atomicAdd(&bk[min(B.nato[jm], FM_MAXAT)], 1);
+        } else {
+            eb[inn] = 0.0f;
         }
-        bk[FM_MAXAT + 1] = a;
+    }
+    for (int inn = 1 + (int)threadIdx.x + FM_THREADS * 32; inn < n; inn += FM_THREADS) {
+        const int jm = __ldg(rg + inn);
+        if (near(jm)) atomicAdd(&bk[min(B.nato[jm], FM_MAXAT)], 1);
+        else eb[inn] = 0.0f;
     }
     __syncthreads();
-    for (int inn = 1 + threadIdx.x; inn < n; inn += blockDim.x) {
-        const int nb = nb_of(inn);
-        if (nb > 0) list[atomicAdd(&bk[nb], 1)] = inn;
+    if (threadIdx.x < 32) {   // bk[b] -> first list position of atom count b; bk[FM_MAXAT+1] = total
+        const int lane = threadIdx.x;
+        int carry = 0;
+        for (int b0 = 0; b0 < FM_MAXAT + 2; b0 += 32) {
+            const int b = b0 + lane;
+            const int t = b <= FM_MAXAT ? bk[b] : 0;
+            int incl = t;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int u = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += u;
+            }
+            if (b <= FM_MAXAT + 1) bk[b] = carry + incl - t;
+            carry += __shfl_sync(0xffffffffu, incl, 31);
+        }
+    }
+    __syncthreads();
+    for (; mask; mask &= mask - 1) {
+        const int inn = 1 + (int)threadIdx.x + FM_THREADS * (__ffs(mask) - 1);
+        list[atomicAdd(&bk[min(B.nato[__ldg(rg + inn)], FM_MAXAT)], 1)] = inn;
+    }
+    for (int inn = 1 + (int)threadIdx.x + FM_THREADS * 32; inn < n; inn += FM_THREADS) {
+        const int jm = __ldg(rg + inn);
+        if (near(jm)) list[atomicAdd(&bk[min(B.nato[jm], FM_MAXAT)], 1)] = inn;
     }
     __syncthreads();
     const int total = bk[FM_MAXAT + 1];
     int mine = 0;
     for (int q = threadIdx.x; q < total; q += blockDim.x) {
         const int inn = list[q];
-        const float e = en_mole_pair_dev(B, im, reg[(size_t)c * M + inn]);
-        ebuf[(size_t)v * M + inn] = e;
+        const float e = en_mole_pair_dev<CUBIC>(B, rcp, im, __ldg(rg + inn));
+        eb[inn] = e;
         if (e != 0.0f) ++mine;
     }
-    int tot;
-    bscan(mine, &tot);
-    if (threadIdx.x == 0) cnt[v] = tot;
+    mine = __reduce_add_sync(0xffffffffu, mine);
+    if ((threadIdx.x & 31) == 0 && mine) atomicAdd(&nonzero, mine);
+    __syncthreads();
+    if (threadIdx.x == 0) cnt[v] = nonzero;
 }
 
 // (3) exclusive scan over visit positions / molecules (single block)
@@ -196,7 +216,7 @@ __global__ void scan1_kernel(const int32_t *in, int n, int32_t *out, int flag_no
         int v = 0;
         if (i < n) v = flag_nonzero_float ? (fin[i] != 0.0f ? 1 : 0) : in[i];
         int tot;
-        int pre = bscan(v, &tot);
+        int pre = block_scan(v, &tot);
         if (i < n) out[i] = carry + pre;
         carry += tot;
     }
@@ -230,36 +250,44 @@ __global__ void __launch_bounds__(FM_THREADS) fm_write_kernel(const int32_t *vis
     const int c = molcellno[im] - 1;
     const int n = nn[c];
     int carry = 0;
-    for (int base = 1; base < n; base += blockDim.x) {
-        const int inn = base + threadIdx.x;
-        float e = 0.0f;
-        int jm = -1, flag = 0;
-        if (inn < n) {
-            jm = reg[(size_t)c * M + inn];
-            e = ebuf[(size_t)v * M + inn];
-            flag = e != 0.0f;
+    for (int base = 1; base < n; base += FM_WRITE * FM_THREADS) {   // FM_WRITE entries in a row each
+        const int i0 = base + FM_WRITE * (int)threadIdx.x;
+        float e[FM_WRITE];
+        int mine = 0;
+#pragma unroll
+        for (int u = 0; u < FM_WRITE; ++u) {
+            e[u] = i0 + u < n ? ebuf[(size_t)v * M + i0 + u] : 0.0f;
+            mine += e[u] != 0.0f;
         }
         int tot;
-        const int rank = carry + bscan(flag, &tot);
-        if (flag) {
-            const int g = nintra + off[v] + rank;
-            ergpair[g] = e;
-            int s1 = atomicAdd(rowcnt + im, 1);
-            int s2 = atomicAdd(rowcnt + jm, 1);
-            if (s1 < M && s2 < M) {
-                molergpair[(size_t)im * M + s1] = jm;
-                ergpairref[(size_t)im * M + s1] = g;
-                molergpair[(size_t)jm * M + s2] = im;
-                ergpairref[(size_t)jm * M + s2] = g;
-            } else {
-                atomicExch(err, 2);
+        int g = nintra + off[v] + carry + block_scan(mine, &tot);
+        if (mine) {
+#pragma unroll
+            for (int u = 0; u < FM_WRITE; ++u) {
+                if (!(e[u] != 0.0f)) continue;
+                const int jm = reg[(size_t)c * M + i0 + u];
+                ergpair[g] = e[u];
+                const int s1 = atomicAdd(rowcnt + im, 1);
+                const int s2 = atomicAdd(rowcnt + jm, 1);
+                if (s1 < M && s2 < M) {
+                    molergpair[(size_t)im * M + s1] = jm;
+                    ergpairref[(size_t)im * M + s1] = g;
+                    molergpair[(size_t)jm * M + s2] = im;
+                    ergpairref[(size_t)jm * M + s2] = g;
+                } else {
+                    atomicExch(err, 2);
+                }
+                ++g;
             }
         }
         carry += tot;
     }
 }
 
-// (5) sort each molecule's row by store index; refs become 1-based
+// (5) sort each molecule's row by store index; refs become 1-based.  Rows up to FM_RANK entries by
+// counting the smaller keys (rows of 200: 57 us for 8,000 molecules, 100 us by the bitonic network and its
+// barriers that longer rows take).
+constexpr int FM_RANK = 512;
 __global__ void fm_sort_kernel(int M, const int32_t *rowcnt, int32_t *nergpairm, int32_t *molergpair,
                                int32_t *ergpairref, int cap_pow2) {
     extern __shared__ int32_t sk[];  // keys [cap], vals [cap]
@@ -268,7 +296,7 @@ __global__ void fm_sort_kernel(int M, const int32_t *rowcnt, int32_t *nergpairm,
     int32_t *key = sk, *val = sk + cap_pow2;
     int np2 = 1;
     while (np2 < n) np2 <<= 1;
-    for (int i = threadIdx.x; i < np2; i += blockDim.x) {
+    for (int i = threadIdx.x; i < max(np2, 4); i += blockDim.x) {
         if (i < n) {
             key[i] = ergpairref[(size_t)m * M + i];
             val[i] = molergpair[(size_t)m * M + i];
@@ -278,6 +306,29 @@ __global__ void fm_sort_kernel(int M, const int32_t *rowcnt, int32_t *nergpairm,
         }
     }
     __syncthreads();
+    if (n <= FM_RANK) {   // a row's entry goes where its rank says
+        int rank[FM_RANK / 256] = {0, 0};
+        const int4 *k4 = (const int4 *)key;
+        const int k0 = (int)threadIdx.x < n ? key[threadIdx.x] : 0x7fffffff;
+        const int k1 = (int)threadIdx.x + 256 < n ? key[threadIdx.x + 256] : 0x7fffffff;
+        const int q1 = (int)(threadIdx.x & ~31u) < n ? (n + 3) / 4 : 0;   // warps with an entry
+#pragma unroll 4
+        for (int q = 0; q < q1; ++q) {   // the keys past n are above all
+            const int4 w = k4[q];
+            rank[0] += (w.x < k0) + (w.y < k0) + (w.z < k0) + (w.w < k0);
+            if (n > 256) rank[1] += (w.x < k1) + (w.y < k1) + (w.z < k1) + (w.w < k1);
+        }
+#pragma unroll
+        for (int u = 0; u < FM_RANK / 256; ++u) {
+            const int i = threadIdx.x + 256 * u;
+            if (i < n) {
+                ergpairref[(size_t)m * M + rank[u]] = key[i] + 1;
+                molergpair[(size_t)m * M + rank[u]] = val[i];
+            }
+        }
+        if (threadIdx.x == 0) nergpairm[m] = n;
+        return;
+    }
     for (int k = 2; k <= np2; k <<= 1) {
         for (int j = k >> 1; j > 0; j >>= 1) {
             for (int i = threadIdx.x; i < np2; i += blockDim.x) {
@@ -332,31 +383,18 @@ __global__ void mirror_set_kernel(int nmol, int M, const int32_t *nergpairm, con
     }
 }
 
-__global__ void mol_radius_kernel(const int32_t *naf, const int32_t *nato, const float *xa, const float *ya,
-                                  const float *za, int nmol, float *rad) {
+__global__ void mol_centre_kernel(const int32_t *naf, const int32_t *nato, const float *xa, const float *ya,
+                                  const float *za, const float *xadd, const float *yadd, const float *zadd, int nmol,
+                                  float4 *ctr) {
     int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= nmol) return;
     float r = 0.0f;
     for (int a = naf[m]; a < naf[m] + nato[m]; ++a) r = fmaxf(r, sqrtf(xa[a] * xa[a] + ya[a] * ya[a] + za[a] * za[a]));
-    rad[m] = r * 1.0001f + 1.0e-6f;
+    ctr[m] = make_float4(xadd[m], yadd[m], zadd[m], r * 1.0001f + 1.0e-6f);
 }
 
-// ftest / ftestb: strict = the reference's sequential float sums
-__global__ void fm_sums_kernel(const float *ergpair, int nintra, int ntot, const float *eintra, int nmol,
-                               int strict, float *out2) {
-    if (strict) {
-        if (threadIdx.x == 0) {
-            float ft = 0.0f, fb = 0.0f;
-            for (int m = 0; m < nmol; ++m) fb = __fadd_rn(fb, eintra[m]);
-            for (int g = nintra; g < ntot; ++g) ft = __fadd_rn(ft, ergpair[g]);
-            out2[0] = __fdiv_rn(ft, (float)nmol);
-            out2[1] = __fdiv_rn(fb, (float)nmol);
-        }
-        return;
-    }
-    double a = 0.0, b = 0.0;
-    for (int g = nintra + threadIdx.x; g < ntot; g += blockDim.x) a += ergpair[g];
-    for (int m = threadIdx.x; m < nmol; m += blockDim.x) b += eintra[m];
+// the block's sums of a and b: the means into out2, or the sums into part
+__device__ __forceinline__ void fm_total(double a, double b, int nmol, float *out2, double *part) {
     __shared__ double sa[32], sb[32];
     a = warp_sum_d(a);
     b = warp_sum_d(b);
@@ -371,9 +409,47 @@ __global__ void fm_sums_kernel(const float *ergpair, int nintra, int ntot, const
             ta += sa[w];
             tb += sb[w];
         }
-        out2[0] = (float)(ta / nmol);
-        out2[1] = (float)(tb / nmol);
+        if (out2) {
+            out2[0] = (float)(ta / nmol);
+            out2[1] = (float)(tb / nmol);
+        } else {
+            part[0] = ta;
+            part[1] = tb;
+        }
     }
+}
+
+// ftest / ftestb: strict = the reference's sequential float sums; else double sums by as many CTAs as
+// give each 4,096 entries (814,000: 8 us, 367 us by one)
+constexpr int FM_SUM = 4096;
+__global__ void fm_sums_kernel(const float *ergpair, int nintra, int ntot, const float *eintra, int nmol,
+                               int strict, float *out2, double *part) {
+    if (strict) {
+        if (threadIdx.x == 0) {
+            float ft = 0.0f, fb = 0.0f;
+            for (int m = 0; m < nmol; ++m) fb = __fadd_rn(fb, eintra[m]);
+            for (int g = nintra; g < ntot; ++g) ft = __fadd_rn(ft, ergpair[g]);
+            out2[0] = __fdiv_rn(ft, (float)nmol);
+            out2[1] = __fdiv_rn(fb, (float)nmol);
+        }
+        return;
+    }
+    // double: each CTA its share (a fixed order); with one CTA the sums, else its part
+    double a = 0.0, b = 0.0;
+    const int step = gridDim.x * blockDim.x, first = blockIdx.x * blockDim.x + threadIdx.x;
+#pragma unroll 4
+    for (int g = nintra + first; g < ntot; g += step) a += ergpair[g];
+    for (int m = first; m < nmol; m += step) b += eintra[m];
+    fm_total(a, b, nmol, gridDim.x == 1 ? out2 : nullptr, part + 2 * blockIdx.x);
+}
+
+__global__ void fm_parts_kernel(const double *part, int n, int nmol, float *out2) {
+    double a = 0.0, b = 0.0;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        a += part[2 * i];
+        b += part[2 * i + 1];
+    }
+    fm_total(a, b, nmol, out2, nullptr);
 }
 
 BoxDev make_boxdev(const epsr_box_t *b) {
@@ -466,7 +542,7 @@ extern "C" int epsr_fmolec1(const epsr_box_t *box, const epsr_cells_t *cells, co
     int32_t *off = (int32_t *)take(sizeof(int32_t) * ((size_t)nmol + 1));
     int32_t *iidx = (int32_t *)take(sizeof(int32_t) * ((size_t)nmol + 1));
     int32_t *rowcnt = (int32_t *)take(sizeof(int32_t) * (size_t)nmol);
-    float *rad = (float *)take(sizeof(float) * (size_t)nmol);
+    take(sizeof(float) * (size_t)nmol);
     int32_t *err = (int32_t *)take(sizeof(int32_t) * 8);
     float *sums = (float *)take(sizeof(float) * 2);
     const size_t own_n = 2 * ((size_t)nmol + (size_t)nmol * M / 2 + 16);
@@ -478,21 +554,25 @@ extern "C" int epsr_fmolec1(const epsr_box_t *box, const epsr_cells_t *cells, co
     Prefilter P;
     P.on = box->cubic ? 1 : 0;
     P.cut = (float)((double)(B.T.izcut - 1) * (double)box->stepcl * 1.00001 + 1.0e-6);
-    P.rad = rad;
-    P.xadd = box->xadd;
-    P.yadd = box->yadd;
-    P.zadd = box->zadd;
+    P.ctr = (const float4 *)owners;   // of later; rows of one slot have no room, and no entry to look at
     const int noff = cells->ncellneighb;
     positions_kernel<<<nmol, 32, 0, s>>>(box->naf, box->nato, box->itype, box->xa, box->ya, box->za, box->xadd,
                                          box->yadd, box->zadd, nmol, (float4 *)box->pos);
-    mol_radius_kernel<<<(nmol + 127) / 128, 128, 0, s>>>(box->naf, box->nato, box->xa, box->ya, box->za, nmol, rad);
+    if (P.on && M >= 2)
+        mol_centre_kernel<<<(nmol + 127) / 128, 128, 0, s>>>(box->naf, box->nato, box->xa, box->ya, box->za, box->xadd,
+                                                             box->yadd, box->zadd, nmol, (float4 *)owners);
     region_build_kernel<<<ncell, 256, sizeof(int32_t) * 2 * (size_t)noff, s>>>(
         cells->cell_start, cells->cell_mols, cells->offsets, noff, cells->ncelldiva, cells->ncelldivb,
         cells->ncelldivc, M, reg, nn, err);
     const size_t list_bytes = sizeof(int) * (size_t)M;
-    if (list_bytes > 48 * 1024) EPSR_SMEM_OPTIN(fm_count_kernel);
-    EPSR_TIMED("fm_count_kernel", s, fm_count_kernel<<<nmol, FM_THREADS, list_bytes, s>>>(B, P, cells->cell_mols, cells->molcellno, reg, nn, M, ebuf,
-                                                         cnt));
+    if (list_bytes > 48 * 1024) {
+        EPSR_SMEM_OPTIN(fm_count_kernel<true>);
+        EPSR_SMEM_OPTIN(fm_count_kernel<false>);
+    }
+    const float rcp = step_rcp(B.T.stepcl, B.T.izcut);
+    auto *count = box->cubic ? fm_count_kernel<true> : fm_count_kernel<false>;
+    EPSR_TIMED("fm_count_kernel", s, count<<<nmol, FM_THREADS, list_bytes, s>>>(B, P, cells->cell_mols, cells->molcellno, reg, nn, M, rcp,
+                                                                                ebuf, cnt));
     scan1_kernel<<<1, 1024, 0, s>>>(cnt, nmol, off, 0, nullptr);
     scan1_kernel<<<1, 1024, 0, s>>>(nullptr, nmol, iidx, 1, eintra);
     EPSR_CUDA(cudaGetLastError());
@@ -519,7 +599,13 @@ extern "C" int epsr_fmolec1(const epsr_box_t *box, const epsr_cells_t *cells, co
     }
     if (shm > 48 * 1024) EPSR_SMEM_OPTIN(fm_sort_kernel);
     fm_sort_kernel<<<nmol, 256, shm, s>>>(M, rowcnt, store->nergpairm, store->molergpair, store->ergpairref, cap);
-    fm_sums_kernel<<<1, strict ? 32 : 1024, 0, s>>>(store->ergpair, nintra, (int)ntot, eintra, nmol, strict, sums);
+    // the parts lie where the mirror's owners come later (8 bytes an entry, 16 a part)
+    const int64_t nsum = ntot > nmol ? ntot : nmol;
+    const int nparts = strict || nsum <= FM_SUM ? 1 : (int)(nsum < 256 * FM_SUM ? (nsum + FM_SUM - 1) / FM_SUM : 256);
+    double *part = (double *)owners;
+    fm_sums_kernel<<<nparts, strict ? 32 : 1024, 0, s>>>(store->ergpair, nintra, (int)ntot, eintra, nmol, strict,
+                                                                    sums, part);
+    if (nparts > 1) fm_parts_kernel<<<1, 256, 0, s>>>(part, nparts, nmol, sums);
     if (store->mirror) {
         if ((size_t)2 * ntot > own_n) {
             epsr_set_error("epsr_fmolec1: mirror scratch too small");

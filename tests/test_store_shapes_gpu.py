@@ -1,0 +1,93 @@
+"""The pair store against the C oracle, bit for bit, where its kernels branch: rows beyond the entries that
+are ranked (the bitonic network sorts them), partial groups of four partner atoms (molecules of 1, 3 and
+10 atoms), a triclinic cell, cells of more than 256 members and regions beyond a thread's 32 remembered
+entries, and a store with as many sums as several CTAs take.  The double sums of the fast mode are those of
+the same float32 energies in another order: 1e-12 of the summed magnitudes before their rounding to float."""
+
+import numpy as np
+import pytest
+
+from epsr_python_translation_b200 import configs
+from epsr_python_translation_b200.box import BoxArrays
+from oracle import oracle
+from tests.goldens import assert_bits_equal
+
+pytestmark = pytest.mark.gpu
+f32 = np.float32
+
+
+def _dense():
+    """A box narrower than twice the tables' range: nearly every molecule is a partner."""
+    box = BoxArrays.from_system(configs.c1_water(seed=5, nmol=700))
+    box.dmax = f32(15.0)
+    box.xstar = (box.x / box.dmax).astype(f32)
+    return box
+
+
+def _triclinic():
+    box = BoxArrays.from_system(configs.c2_mixture(seed=6, ndmso=12, nwater=24))
+    box.cubic = False
+    box.lat6 = np.array([1.0, 0.1, 0.05, 0.995, 0.08, 0.99], f32)
+    box.lat9 = np.array([1.0, 0.0, 0.0, 0.1, 0.995, 0.0, 0.05, 0.08, 0.99], f32)
+    return box
+
+
+BOXES = {
+    "dense_700": (_dense, 10), "triclinic": (_triclinic, 10),
+    "silica": (lambda: BoxArrays.from_system(configs.silica(seed=3, natom=303)), 10),
+    "mixture": (lambda: BoxArrays.from_system(configs.c2_mixture(seed=4, ndmso=41, nwater=83)), 7),
+    "crowded_cells": (lambda: BoxArrays.from_system(configs.c1_water(seed=8, nmol=2300)), 290),
+}
+
+
+@pytest.mark.parametrize("name", list(BOXES))
+def test_store_matches_oracle(name):
+    from epsr_python_translation_b200.device import DeviceBox
+    make, nmolcell = BOXES[name]
+    box = make()
+    eintra = np.random.default_rng(1).standard_normal(box.nmol).astype(f32)
+    eintra[::3] = 0
+    oc = oracle.cell_list(box, nmolcell, box.sepmax)
+    ost = oracle.fmolec1(box, oc, eintra, capacity=box.nmol * min(box.nmol, 800))
+    d = DeviceBox(box)
+    d.cell_list(nmolcell, box.sepmax)
+    sums = d.fmolec1(eintra, strict=True)
+    st = d.download_store()
+    assert st["nergpair"] == ost["nergpair"]
+    n = st["nergpair"]
+    assert_bits_equal(st["ergpair"], ost["ergpair"][:n], "ergpair")
+    assert np.array_equal(st["nergpairm"], ost["nergpairm"])
+    M = st["nnbrefmax"]
+    om, oref = ost["molergpair"].reshape(box.nmol, M), ost["ergpairref"].reshape(box.nmol, M)
+    for m in range(box.nmol):
+        k = int(st["nergpairm"][m])
+        assert np.array_equal(st["molergpair"][m, :k], om[m, :k]) and np.array_equal(st["ergpairref"][m, :k], oref[m, :k])
+    if name == "dense_700":
+        assert st["nergpairm"].max() > 512
+    fast = d.fmolec1(eintra, strict=False)
+    e = st["ergpair"][int(np.count_nonzero(eintra)):].astype(np.float64)
+    for got, v in ((fast[0], e), (fast[1], eintra.astype(np.float64))):
+        ref = v.sum() / box.nmol
+        assert abs(float(got) - ref) <= 2.0 ** -24 * abs(ref) + 1e-12 * np.abs(v).sum() / box.nmol
+    assert np.isfinite(sums[0])
+
+
+def test_long_region_matches_fine_cells():
+    """A region of 9,000 molecules (past a thread's remembered entries) holds the pairs that fine cells find."""
+    from epsr_python_translation_b200.device import DeviceBox
+    box = BoxArrays.from_system(configs.c3_water(seed=2, nmol=9000))
+    pairs = []
+    for nmolcell in (1200, 10):
+        d = DeviceBox(box)
+        d.cell_list(nmolcell, box.sepmax)
+        d.fmolec1(np.zeros(box.nmol, f32), strict=False)
+        st = d.download_store()
+        rows = np.repeat(np.arange(box.nmol), st["nergpairm"])
+        cols = np.concatenate([st["molergpair"][m, :k] for m, k in enumerate(st["nergpairm"])])
+        ref = np.concatenate([st["ergpairref"][m, :k] for m, k in enumerate(st["nergpairm"])])
+        e = st["ergpair"][ref - 1]
+        o = np.lexsort((cols, rows))
+        pairs.append((rows[o], cols[o], e[o], st["nnbrefmax"]))
+    assert pairs[0][3] == 9000 and pairs[1][3] < 9000
+    assert np.array_equal(pairs[0][0], pairs[1][0]) and np.array_equal(pairs[0][1], pairs[1][1])
+    assert_bits_equal(pairs[0][2], pairs[1][2], "energies")
