@@ -17,12 +17,12 @@
 //            the correction c = (B - old') - (A - S) that applies if partner p accepted;
 //            the corrections of partners visited at most 64 moves earlier are kept by the
 //            earlier move (its row: the effect of its acceptance on each of the next 64 moves)
-//   resolve  one CTA walks the moves in order.  The resolver warp holds a running sum for
+//   resolve  one warp walks the moves in order.  The resolver warp holds a running sum for
 //            each of the next 64 moves (two per lane); deciding a move is one comparison in
 //            the lane that holds its sum and a ballot, after which every lane adds the
 //            decided move's row entry for its two moves -- no reduction on the decision
 //            chain.  The rows and thresholds arrive by bulk copies into a four-block ring of
-//            shared memory.  Helper warps sum, per move, the corrections of accepted partners
+//            shared memory.  Helper warps -- of this CTA and of a second one in its cluster -- sum, per move, the corrections of accepted partners
 //            visited more than 64 moves earlier, reading the decisions the resolver publishes
 //            once per 32 moves; each handoff is a 64-bit word carrying its own tag, so no
 //            fence sits on the decision chain;
@@ -591,12 +591,38 @@ constexpr int SP_HCAP = 256;                                  // far partners a 
 constexpr int SP_HSTAGE = SP_HCAP * 12;                       // one staged list: terms, then positions
 constexpr int SP_HOFF = SP_SROWS + SP_STHR + SP_NSLOT * 8 + SP_FR * 8;
 constexpr int SP_SHDR = SP_HOFF + SP_NH * 2 * SP_HSTAGE;
+static_assert(SP_RT / 32 * 2 * SP_HSTAGE <= SP_SHDR, "the second CTA's stages end below the decision words");
 
 __host__ __device__ constexpr size_t spec_resolve_smem(int N) {
     return (size_t)SP_SHDR + 8 * (size_t)((N + SP_BLK - 1) / SP_BLK);
 }
 
-__global__ void __launch_bounds__(SP_RT, 1) spec_resolve_kernel(SpecDev S) {
+// What bounds it: the resolver's block of 32 moves takes 3,400 cycles (106 a move: two additions, a
+// comparison and a ballot decide two moves, then four additions update the sums), if the far parts
+// are there.  A helper takes 3,900 cycles a move (its list's copies, decision words and a tree of
+// double additions, eight warps a scheduler), so the 24 helpers beside the resolver kept it waiting
+// 1,200 cycles a block, and staging the rows itself cost it another 500.  The second CTA's 32 helpers
+// and a stager warp take both off it: 8,000 moves of DMSO and water 663 -> 604 us, 20,000 of water 1,636 ->
+// 1,262 us.
+// The second CTA of the pair is helpers alone (its stages where the first keeps its rows); it has its
+// own copy of the decision words, which the resolver stores into both.
+__device__ __forceinline__ uint32_t cluster_addr(const void *p, uint32_t rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(umma::smem_u32(p)), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cluster_st64(uint32_t a, uint64_t v) {
+    asm volatile("st.relaxed.cluster.shared::cluster.u64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
+}
+__device__ __forceinline__ void cluster_st32(uint32_t a, int v) {
+    asm volatile("st.relaxed.cluster.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ void cluster_sync_all() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__global__ void __launch_bounds__(SP_RT, 1) __cluster_dims__(2, 1, 1) spec_resolve_kernel(SpecDev S) {
     extern __shared__ __align__(128) unsigned char rsm[];
     float2 *srows = reinterpret_cast<float2 *>(rsm);
     float *sthr = reinterpret_cast<float *>(rsm + SP_SROWS);
@@ -607,6 +633,7 @@ __global__ void __launch_bounds__(SP_RT, 1) spec_resolve_kernel(SpecDev S) {
     if (S.flags[0]) return;
     const int N = S.N;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const uint32_t rank = blockIdx.x;
     const int nblk = (N + SP_BLK - 1) / SP_BLK;
     for (int i = tid; i < SP_FR; i += blockDim.x) vfar[i] = 0ull;
     for (int i = tid; i < nblk; i += blockDim.x) vpub[i] = 0ull;
@@ -615,42 +642,36 @@ __global__ void __launch_bounds__(SP_RT, 1) spec_resolve_kernel(SpecDev S) {
         for (int i = 0; i < SP_NSLOT; ++i) umma::mbar_init(&bars[i], 1);
         umma::fence_mbar_init();
     }
-    __syncthreads();
+    cluster_sync_all();
     const float temp = __fdiv_rn(1.0f, S.simt);
     auto fail = [&]() {
         abort_flag = 1;
+        cluster_st32(cluster_addr((const void *)&abort_flag, rank ^ 1u), 1);
         S.flags[1] = 1;
     };
+    // rows and thresholds of block b into its slot (one thread)
+    auto stage = [&](int b) {
+        const int slot = b % SP_NSLOT;
+        const int nr = min(SP_BLK, N - SP_BLK * b);
+        const uint32_t rb = (uint32_t)nr * SP_W * 8, tb = ((uint32_t)nr * 4 + 15u) & ~15u;
+        umma::mbar_expect_tx(&bars[slot], rb + tb);
+        umma::bulk_load(srows + (size_t)slot * SP_BLK * SP_W, S.nearT + (size_t)b * SP_BLK * SP_W, rb, &bars[slot]);
+        umma::bulk_load(sthr + slot * SP_BLK, S.thr + (size_t)b * SP_BLK, tb, &bars[slot]);
+    };
 
-    if (wid == 0) {
+    if (rank == 0 && wid == 0) {
         // ---- the resolver warp
-        auto stage = [&](int b) {   // lane 0: rows and thresholds of block b into its slot
-            const int slot = b % SP_NSLOT;
-            const int nr = min(SP_BLK, N - SP_BLK * b);
-            const uint32_t rb = (uint32_t)nr * SP_W * 8, tb = ((uint32_t)nr * 4 + 15u) & ~15u;
-            umma::mbar_expect_tx(&bars[slot], rb + tb);
-            umma::bulk_load(srows + (size_t)slot * SP_BLK * SP_W, S.nearT + (size_t)b * SP_BLK * SP_W, rb, &bars[slot]);
-            umma::bulk_load(sthr + slot * SP_BLK, S.thr + (size_t)b * SP_BLK, tb, &bars[slot]);
-        };
-        int issued = 0, waited = 0;
-        if (lane == 0)
-            for (; issued < min(nblk, SP_NSLOT - 1); ++issued) stage(issued);
         float A0 = 0.0f, A1 = 0.0f;   // running sums of the pending moves = lane, lane + 32 (mod 64)
         double fadd = 0.0;
         int err = 0;
         for (int b = 0; b < nblk && !err; ++b) {
             const int slot = b % SP_NSLOT;
-            if (lane == 0 && issued < nblk) {   // the slot block b-1 used: this warp has read it
-                umma::fence_proxy_async();
-                stage(issued++);
-            }
             // every lane waits on the block's mbarrier (its completion makes the copied bytes visible)
             const bool got = umma::mbar_wait(&bars[slot], (uint32_t)((b / SP_NSLOT) & 1), nullptr);
             if (__any_sync(0xffffffffu, !got)) {
                 err = 1;
                 break;
             }
-            ++waited;
             const float2 *rows = srows + (size_t)slot * SP_BLK * SP_W;
             const float *th = sthr + slot * SP_BLK;
             const int nr = min(SP_BLK, N - SP_BLK * b);
@@ -747,28 +768,50 @@ __global__ void __launch_bounds__(SP_RT, 1) spec_resolve_kernel(SpecDev S) {
                 S.fdiff[ko] = fd_own;
                 if (acc) fadd += (double)fd_own;
             }
-            if (lane == 0) vpub[b] = ((uint64_t)(uint32_t)(b + 1) << 32) | wbits;
-        }
-        if (lane == 0) {
-            if (err) {
-                fail();
-                // the copies still in flight land before the CTA's shared memory goes away
-                for (int b = waited; b < issued; ++b) umma::mbar_wait(&bars[b % SP_NSLOT], (uint32_t)((b / SP_NSLOT) & 1), nullptr);
+            __syncwarp();   // every lane has read the block's slot before the stager sees the word
+            if (lane == 0) {
+                const uint64_t word = ((uint64_t)(uint32_t)(b + 1) << 32) | wbits;
+                vpub[b] = word;
+                cluster_st64(cluster_addr((const void *)(vpub + b), 1u), word);
             }
         }
+        if (lane == 0 && err) fail();
         fadd = warp_sum_d(fadd);   // each lane's accepted moves, then the lanes in a fixed order
         if (lane == 0) *S.fadd_acc = fadd;
-    } else if ((wid & 3) != 0) {
+    } else if (rank == 0 && wid == 4) {
+        // ---- the stager (a warp beside the resolver's, asleep nearly always): block b's slot is free
+        // once block b - SP_NSLOT is decided
+        if (lane == 0) {
+            int b = 0;
+            for (; b < nblk; ++b) {
+                bool go = true;
+                if (b >= SP_NSLOT) {
+                    long long it = 0;
+                    while ((uint32_t)(vpub[b - SP_NSLOT] >> 32) != (uint32_t)(b - SP_NSLOT + 1) && go) {
+                        go = !(++it > SP_SPIN_LIMIT || abort_flag);
+                        __nanosleep(100);
+                    }
+                }
+                if (!go) break;
+                umma::fence_proxy_async();
+                stage(b);
+            }
+            // the copies in flight land before the CTA's shared memory goes away
+            for (int c = max(b - SP_NSLOT, 0); c < b; ++c)
+                umma::mbar_wait(&bars[c % SP_NSLOT], (uint32_t)((c / SP_NSLOT) & 1), nullptr);
+        }
+    } else if (rank == 1 || (wid & 3) != 0) {
         // ---- helper warps: the far part of each move's change, one move a step.  A move's
         // listed far partners (up to SP_HCAP; a longer list reads the rest from global memory)
         // are copied into one of the helper's two shared-memory stages by cp.async one step
         // before they are summed, with its list length and base loaded two steps before; those
         // two scalars live in three register sets that take turns (the loop body is written
         // out three times), so nothing waits on a load in flight.
-        const int h = wid - 1 - (wid >> 2);
+        const int h = rank ? SP_NH + wid : wid - 1 - (wid >> 2);
         const int M = S.M;
-        const int st = SP_NH;
-        unsigned char *hb = rsm + SP_HOFF + (size_t)h * 2 * SP_HSTAGE;
+        const int st = SP_NH + SP_RT / 32;
+        unsigned char *hb = rank ? rsm + (size_t)wid * 2 * SP_HSTAGE : rsm + SP_HOFF + (size_t)h * 2 * SP_HSTAGE;
+        const uint32_t far0 = cluster_addr((const void *)vfar, 0u);
         struct Scal {
             int nf;
             double bk;
@@ -846,7 +889,7 @@ __global__ void __launch_bounds__(SP_RT, 1) spec_resolve_kernel(SpecDev S) {
             sum = warp_sum_d(sum);
             if (lane == 0) {
                 const float fk = (float)(g.bk + sum);
-                vfar[kk % SP_FR] = ((uint64_t)(uint32_t)(kk + 1) << 32) | __float_as_uint(fk);
+                cluster_st64(far0 + 8u * (uint32_t)(kk % SP_FR), ((uint64_t)(uint32_t)(kk + 1) << 32) | __float_as_uint(fk));
             }
             return true;
         };
@@ -874,6 +917,7 @@ __global__ void __launch_bounds__(SP_RT, 1) spec_resolve_kernel(SpecDev S) {
         }
         cp_async_wait_all();   // no copy lands after the CTA's shared memory goes away
     }
+    cluster_sync_all();   // no CTA leaves while the other may store into its shared memory
 }
 
 // ----------------------------------------------------------------- walk (exact sums)
@@ -1223,7 +1267,10 @@ namespace epsr {
 // between, the cycle was redone by the sequential kernel, the caller set a new state) it
 // walks the stream itself.  Either way it draws the same values.
 
-__global__ void __launch_bounds__(96) ahead_fill_kernel(const int32_t *state, int32_t *ahead, const int32_t *count) {
+// out: the values' place in `ahead`.  (As a parameter: computed here, the compiler's order of the walk took 33
+// cycles a value instead of 27.)
+__global__ void __launch_bounds__(96) ahead_fill_kernel(const int32_t *state, int32_t *ahead, const int32_t *count,
+                                                        float *out) {
     __shared__ R1Ring ring;
     __shared__ int32_t tab[34];
     const int lane = threadIdx.x & 31;
@@ -1235,7 +1282,6 @@ __global__ void __launch_bounds__(96) ahead_fill_kernel(const int32_t *state, in
     }
     const int32_t mcall = state[2];
     Ran1Warp g;
-    float *out = reinterpret_cast<float *>(ahead + AH_VALS);
     r1_fill(ring, tab, state, n, g, [&](int64_t i, int32_t v) { out[i] = ran1_out(v); });
     if (threadIdx.x >= 32) return;
     ahead[AH_END + 3 + lane] = g.iv;
@@ -1471,7 +1517,8 @@ int epsr_molfit_spec(const epsr_box_t *box, const epsr_cells_t *cells, epsr_stor
         // the SM to itself for the 2-3 ms it runs
         EPSR_SMEM_OPTIN(ahead_fill_kernel);
         EPSR_TIMED("ahead_fill_kernel", as->st,
-                   ahead_fill_kernel<<<1, 96, g_ahead_smem, as->st>>>(S.ran1_next, mc->ahead, S.off + N));
+                   ahead_fill_kernel<<<1, 96, g_ahead_smem, as->st>>>(S.ran1_next, mc->ahead, S.off + N,
+                                                                      reinterpret_cast<float *>(mc->ahead + AH_VALS)));
         EPSR_CUDA(cudaGetLastError());
         EPSR_CUDA(cudaEventRecord(as->join, as->st));
     }
@@ -1516,7 +1563,7 @@ int epsr_molfit_spec(const epsr_box_t *box, const epsr_cells_t *cells, epsr_stor
             rsmem = max(rsmem, (size_t)optin - 1024);
         }
         EPSR_SMEM_OPTIN(spec_resolve_kernel);
-        EPSR_TIMED("spec_resolve_kernel", s, spec_resolve_kernel<<<1, SP_RT, rsmem, s>>>(S));
+        EPSR_TIMED("spec_resolve_kernel", s, spec_resolve_kernel<<<2, SP_RT, rsmem, s>>>(S));
     }
     EPSR_TIMED("spec_commit_kernel", s, spec_commit_kernel<<<(N + SP_CW - 1) / SP_CW, 32 * SP_CW, 0, s>>>(S));
     EPSR_CUDA(cudaGetLastError());
