@@ -50,7 +50,6 @@ constexpr int SP_RT = 1024;     // resolver CTA: warp 0 resolves, the warps of s
 constexpr long long SP_SPIN_LIMIT = 1ll << 26;
 // words of the draws-ahead buffer (described with the draws-ahead kernels below)
 constexpr int AH_VALID = 0, AH_COUNT = 1, AH_USES = 2, AH_START = 4, AH_END = 40, AH_VALS = 80;
-constexpr int SP_MAXEDGE = 16384;  // table points indexed by bin edges (beyond: the energy pass divides)
 
 struct SpecDev {
     Lattice L;
@@ -95,9 +94,7 @@ struct SpecDev {
     int32_t *acc;                          // [N] by visit position
     float *fdiff;                          // [N] by visit position
     double *fadd_acc;                      // [1]
-    Bins bins;                             // the energy pass's table index by bin edges (cubic boxes)
-    float4 *edge_w;                        // [nedge] written by the propose pass
-    int nedge;                             // 0: the energy pass divides (triclinic box, or too many bins)
+    float rcp;                             // step_rcp of the tables
     int ev;                                // the energy pass's staged values per chunk (>= 2 maxat^2)
     const int32_t *ngrot;                  // [N] rotational groups of each molecule, or NULL
     int32_t *ninter;                       // [2*nmoltype] zeroed by a cycle without internal rotations, or NULL
@@ -265,7 +262,6 @@ __device__ __forceinline__ float metropolis_threshold(float u) {
 
 __global__ void spec_propose_kernel(SpecDev S) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < S.nedge) S.edge_w[k] = bin_edge_entry(S.T.stepcl, S.T.xstar, S.T.ld, k);
     if (k >= S.N) return;
     const float pi = 3.14159265358979323846f;
     const int m = S.visit[k];
@@ -374,7 +370,7 @@ __device__ __forceinline__ int warp_incl_scan(int v, int lane) {
 // four CTAs of the energy pass per SM (40 warps): its shared memory allows four, and the
 // register budget that gives (51 a thread) holds the three pair evaluations in flight unspilled
 constexpr int SP_EN_MINB = 4;
-template <bool BINS>
+template <bool CUBIC>
 __global__ void __launch_bounds__(SP_ET, SP_EN_MINB) spec_energy_kernel(SpecDev S) {
     extern __shared__ __align__(16) unsigned char en_smem[];
     const int ev = S.ev;                                                 // staged values per chunk
@@ -453,10 +449,10 @@ __global__ void __launch_bounds__(SP_ET, SP_EN_MINB) spec_energy_kernel(SpecDev 
                 const int c0 = col[__float_as_int(q0.w) * ntype], c1 = col[__float_as_int(q1.w) * ntype],
                           c2 = col[__float_as_int(q2.w) * ntype];
                 float e0, e1, e2;
-                if (BINS) {
-                    e0 = pair_energy_cubic_bins(S.bins, q0, p2, c0);
-                    e1 = pair_energy_cubic_bins(S.bins, q1, p2, c1);
-                    e2 = pair_energy_cubic_bins(S.bins, q2, p2, c2);
+                if (CUBIC) {
+                    e0 = pair_energy_unit(T, S.rcp, q0, p2, c0);
+                    e1 = pair_energy_unit(T, S.rcp, q1, p2, c1);
+                    e2 = pair_energy_unit(T, S.rcp, q2, p2, c2);
                 } else {
                     e0 = pair_energy(L, T, q0, p2, c0);
                     e1 = pair_energy(L, T, q1, p2, c1);
@@ -1352,7 +1348,6 @@ static size_t spec_bytes(int N, int natom, int M, int nmt) {
          spal(sizeof(float2) * (size_t)N * M);
     b += spal(sizeof(int32_t) * N);   // nnk
     b += spal(sizeof(int32_t) * N) + spal(sizeof(float) * N) + spal(sizeof(double));
-    b += spal(sizeof(float4) * SP_MAXEDGE);   // bin edges of the energy pass
     return b;
 }
 
@@ -1481,19 +1476,7 @@ int epsr_molfit_spec(const epsr_box_t *box, const epsr_cells_t *cells, epsr_stor
     S.acc = (int32_t *)take(sizeof(int32_t) * N);
     S.fdiff = (float *)take(sizeof(float) * N);
     S.fadd_acc = (double *)take(sizeof(double));
-    {
-        float4 *edge = (float4 *)take(sizeof(float4) * SP_MAXEDGE);
-        const int nedge = max(S.T.izcut - 1, 1);
-        if (box->cubic && nedge <= SP_MAXEDGE && S.T.stepcl > 0.0f) {
-            S.nedge = nedge;
-            S.edge_w = edge;
-            S.bins.tab = S.T.tab;
-            S.bins.edge = edge;
-            S.bins.ld = S.T.ld;
-            S.bins.izcut = S.T.izcut;
-            S.bins.cinv = bins_cinv(S.T.stepcl);
-        }
-    }
+    S.rcp = step_rcp(S.T.stepcl, S.T.izcut);
 
     // draws ahead: only with a buffer that holds a whole cycle's values (at most 7 a move)
     const bool ahead = mc->ahead && mc->ahead_cap >= (int64_t)N * 7;
@@ -1522,14 +1505,14 @@ int epsr_molfit_spec(const epsr_box_t *box, const epsr_cells_t *cells, epsr_stor
         EPSR_CUDA(cudaGetLastError());
         EPSR_CUDA(cudaEventRecord(as->join, as->st));
     }
-    EPSR_TIMED("spec_propose_kernel", s, spec_propose_kernel<<<(max(N, S.nedge) + 127) / 128, 128, 0, s>>>(S));
+    EPSR_TIMED("spec_propose_kernel", s, spec_propose_kernel<<<(N + 127) / 128, 128, 0, s>>>(S));
     {
         const int ma = box->maxat > 0 && box->maxat <= SP_MAXAT ? box->maxat : SP_MAXAT;
         S.ev = max(2 * ma * ma, 4096);
     }
     const size_t en_bytes = sizeof(float) * (size_t)S.ev + sizeof(uint16_t) * (size_t)((S.ev + 1) & ~1) +
                             sizeof(int) * (size_t)box->ntype * box->ntype;
-    if (S.nedge) {
+    if (S.L.cubic) {
         EPSR_SMEM_OPTIN(spec_energy_kernel<true>);
         EPSR_TIMED("spec_energy_kernel", s, spec_energy_kernel<true><<<N, SP_ET, en_bytes, s>>>(S));
     } else {
