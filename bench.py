@@ -42,9 +42,8 @@ METRIC = "MC molecule-moves/s (+ g(r) pair-updates/s)"
 # fit, from an ncu --set full capture of one launch (independent of the trial count: the
 # basis is read from HBM once per launch)
 FIT_DRAM_BYTES_PER_LAUNCH = 409856
-# SM cycles per ran1 value of the warp shuffle chain (two shuffles a step) on an otherwise
-# idle SM (clock64 timing of 640,000 values)
-FIT_CHAIN_CYCLES_PER_VALUE = 40.0
+# SM cycles per ran1 value of the stream on an otherwise idle SM (a fill of 140,000 values)
+FIT_CHAIN_CYCLES_PER_VALUE = 27.2
 # FP32 operations per atom pair of a pair energy (3 sub, 6 minimum image, 5 d^2, 1 sqrt,
 # 2 div, 4 table arithmetic, 2 adds, 1 scale, 2 more) and per atogen pair-update
 # dram__bytes_read.sum + dram__bytes_write.sum per atom pair of one spec_energy_kernel launch
@@ -62,8 +61,8 @@ TIMED_KERNELS = ("spec_energy_kernel", "spec_corr_kernel", "spec_resolve_kernel"
 # the ordered walk of spec_resolve_kernel on its own (one warp, rows in shared memory, no far
 # parts to wait for), measured on B200: the latency floor of a resolved move
 RESOLVE_WALK_CYCLES_PER_MOVE = 88.5
-# a dependent warp shuffle on B200 (the step of the ran1 walk)
-RAN1_SHUFFLE_CYCLES = 32
+# half a dependent warp shuffle on B200 (26 cycles): the ran1 walk takes two steps a shuffle
+RAN1_SHUFFLE_CYCLES = 13
 
 
 def parse():
@@ -705,14 +704,14 @@ def roofline(it, ktimes, a):
                 "floor_source": "the walk alone on B200, %.1f cycles per move at %.0f MHz" % (RESOLVE_WALK_CYCLES_PER_MOVE, mhz),
                 "launch_ms": launch_ms, "launches": n}, extra
     if dom in ("ahead_fill_kernel", "ran1_fill_kernel"):
-        # the next cycle's ran1 values: 7 a move (3 rotation, 3 translation, 1 acceptance), one
-        # dependent warp shuffle per value
+        # the next cycle's ran1 values: 7 a move (3 rotation, 3 translation, 1 acceptance), two
+        # values per dependent warp shuffle
         values = 7 * it.box.nmol
         floor_ms = values * RAN1_SHUFFLE_CYCLES / mhz / 1000.0
         return {"bound": "latency (ran1 shuffle chain)", "kernel": dom, "achieved": floor_ms / launch_ms, "peak": 1.0,
                 "unit": "chain floor / measured time per launch", "frac": floor_ms / launch_ms, "traffic": None,
                 "values_per_launch": values, "floor_ms": floor_ms,
-                "floor_source": "one dependent warp shuffle per value, %d cycles on B200 at %.0f MHz" % (RAN1_SHUFFLE_CYCLES, mhz),
+                "floor_source": "two values per dependent warp shuffle, %d cycles a value on B200 at %.0f MHz" % (RAN1_SHUFFLE_CYCLES, mhz),
                 "launch_ms": launch_ms, "launches": n}, extra
     if dom == "fitexp_cluster_kernel":
         trials = max(it.fit_trials, 1)
