@@ -166,18 +166,21 @@ __device__ __forceinline__ int bin_index(float d, float stepcl, float rcp) {
     return n;
 }
 
-// The IEEE square root without its range checks: one Newton step from the reciprocal square
-// root's approximation, the residual exact by the fused product.  Equal to __fsqrt_rn for zero and
-// for every float from 2^-60 to 2^4 (tests/test_pair_math_gpu.py compares all of them); squared
-// distances in box units lie there.
-__device__ __forceinline__ float sqrt_unit_from(float x, float y) {
+// The correctly rounded square root of zero and of every float from 2^-100 to 2^4, where squared
+// distances in box units lie.  PTX's sqrt.approx gives a float s within one unit in the last place of the
+// root, and Tuckerman's test (R. C. Agarwal, J. W. Cooley, F. G. Gustavson, J. B. Shearer, G. Slishman,
+// B. Tuckerman, "New scalar and vector elementary functions for the IBM System/370", IBM J. Res. Dev.
+// 30 (1986) 126-144) chooses between s and the floats before and after it: with t the next float and u = t - s,
+// the middle of the two squared is s t + u^2 / 4, and no float x of that size lies between s t and there, so
+// the root is nearer to t exactly when x > s t; the float before likewise.  The fused product's one rounding
+// keeps the sign of the difference.  tests/test_pair_math_gpu.py compares all of these floats with __fsqrt_rn.
+__device__ __forceinline__ float sqrt_unit(float x) {
     float s;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(s) : "f"(y));
-    const float d = __fmul_rn(x, s);
-    return __fmaf_rn(__fmaf_rn(-d, d, x), __fmul_rn(0.5f, s), d);
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(s) : "f"(x));
+    const float after = __int_as_float(__float_as_int(s) + 1), before = __int_as_float(__float_as_int(s) - 1);
+    const float up = __fmaf_rn(-s, after, x), down = __fmaf_rn(-s, before, x);
+    return up > 0.0f ? after : (down <= 0.0f ? before : s);
 }
-__device__ __forceinline__ float sqrt_unit(float x) { return sqrt_unit_from(x, fmaxf(x, 1e-37f)); }
-__device__ __forceinline__ float sqrt_unit_nz(float x) { return sqrt_unit_from(x, x); }   // a NaN for 0
 
 // pair_energy for a cubic box in box units, bit for bit, with the branch-free root, wrap and
 // index above; rcp = step_rcp(T.stepcl, T.izcut)

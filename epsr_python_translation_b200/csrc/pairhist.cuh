@@ -4,7 +4,7 @@
 //
 // What bounds it: instruction issue, 53 instructions a pair of which many issue every other cycle (68%
 // of the issue slots filled), then the shared-memory adds (2.3 wavefronts a warp).  Distance and bin
-// therefore avoid the conversion unit, the division and the root's range checks (common.cuh), the pair
+// therefore avoid the conversion unit and the division, and the root is branch-free (common.cuh), the pair
 // type's row comes from shared memory, four targets are in flight, a tile that counts whole is run
 // without comparing molecules, and a pair's closest-contact test compares against the largest contact
 // distance before it looks its own up.  The histogram leaves room for few CTAs on an SM, so a CTA is as
@@ -94,7 +94,7 @@ __device__ __forceinline__ void hist_stage_tile(const PairHist &H, const float4 
 template <int U, bool CUBIC, bool STAGED, bool SOME>
 __device__ __forceinline__ void hist_group(const PairHist &H, float4 p1, int im, bool after, const float4 *tp,
                                            const int *tm, const int *cls, int &uses) {
-    float ds[U], d[U];
+    float d[U];
     int n[U], base[U];
     bool use[U], odd[U], any = false;
 #pragma unroll
@@ -110,8 +110,7 @@ __device__ __forceinline__ void hist_group(const PairHist &H, float4 p1, int im,
         base[u] = STAGED ? *(const int *)((const char *)cls + ty) : __ldg(cls + ty) * H.ld;
         // xx = x1 - x2 (ato_manipulation_rev4.py:3798); the square does not see the sign
         if (CUBIC) {
-            ds[u] = dsq_cubic(p2, p1);
-            d[u] = sqrt_unit_nz(ds[u]);   // a NaN for 0, which is odd
+            d[u] = sqrt_unit(dsq_cubic(p2, p1));
         } else {
             d[u] = dist_f(H.L, __fsub_rn(p1.x, p2.x), __fsub_rn(p1.y, p2.y), __fsub_rn(p1.z, p2.z));
         }
@@ -121,10 +120,7 @@ __device__ __forceinline__ void hist_group(const PairHist &H, float4 p1, int im,
     if (any) {
 #pragma unroll
         for (int u = 0; u < U; ++u)
-            if (odd[u]) {
-                if (CUBIC) d[u] = __fsqrt_rn(ds[u]);
-                n[u] = nint_i(__fdiv_rn(d[u], H.stepcl));
-            }
+            if (odd[u]) n[u] = nint_i(__fdiv_rn(d[u], H.stepcl));
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {

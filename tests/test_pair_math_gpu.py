@@ -25,6 +25,10 @@ def test_root_equals_ieee_for_every_float():
     assert _mismatches(0, (127 - 60) << 23, (127 + 4) << 23) == 0        # 2^-60 .. 2^4, all of them
 
 
+def test_root_of_the_smallest_distances():
+    assert _mismatches(0, (127 - 100) << 23, (127 - 60) << 23) == 0      # 2^-100 .. 2^-60, all of them
+
+
 @pytest.mark.parametrize("stepcl", [0.03 / 14.42, 0.03 / 31.7, 0.03 / 84.3, 0.01 / 33.3, 0.05 / 500.0])
 def test_table_index_equals_the_division(stepcl):
     import numpy as np
