@@ -289,11 +289,11 @@ __global__ void __launch_bounds__(FM_THREADS) fm_write_kernel(const int32_t *vis
 // barriers that longer rows take).
 constexpr int FM_RANK = 512;
 __global__ void fm_sort_kernel(int M, const int32_t *rowcnt, int32_t *nergpairm, int32_t *molergpair,
-                               int32_t *ergpairref, int cap_pow2) {
-    extern __shared__ int32_t sk[];  // keys [cap], vals [cap]
+                               int32_t *ergpairref, int cap) {
+    extern __shared__ __align__(16) int32_t sk[];  // keys [cap], vals [cap]; cap a power of two, at least max(M, 4)
     const int m = blockIdx.x;
     const int n = min(rowcnt[m], M);
-    int32_t *key = sk, *val = sk + cap_pow2;
+    int32_t *key = sk, *val = sk + cap;
     int np2 = 1;
     while (np2 < n) np2 <<= 1;
     for (int i = threadIdx.x; i < max(np2, 4); i += blockDim.x) {
@@ -589,9 +589,8 @@ extern "C" int epsr_fmolec1(const epsr_box_t *box, const epsr_cells_t *cells, co
                                                       store->molergpair, store->ergpairref);
     fm_write_kernel<<<nmol, FM_THREADS, 0, s>>>(cells->cell_mols, cells->molcellno, reg, nn, M, ebuf, off, nintra,
                                                 store->ergpair, rowcnt, store->molergpair, store->ergpairref, err);
-    int maxrow = M;
-    int cap = 1;
-    while (cap < maxrow) cap <<= 1;
+    int cap = 4;   // places for the keys of a row, and for its partners: read four at a time
+    while (cap < M) cap <<= 1;
     size_t shm = sizeof(int32_t) * 2 * (size_t)cap;
     if (shm > 200 * 1024) {
         epsr_set_error("epsr_fmolec1: nnbrefmax %d too large for the row sort", M);

@@ -91,3 +91,37 @@ def test_long_region_matches_fine_cells():
     assert pairs[0][3] == 9000 and pairs[1][3] < 9000
     assert np.array_equal(pairs[0][0], pairs[1][0]) and np.array_equal(pairs[0][1], pairs[1][1])
     assert_bits_equal(pairs[0][2], pairs[1][2], "energies")
+
+
+@pytest.mark.parametrize("zero", [False, True])
+@pytest.mark.parametrize("nmol,nmolcell,rmax", [(1, 10, None), (2, 10, None), (3, 10, None), (4, 10, None), (5, 10, None),
+                                                (16, 1, 0.0), (64, 1, 0.0), (200, 1, 0.0), (200, 2, 0.0)])
+def test_short_rows_match_oracle(nmol, nmolcell, rmax, zero):
+    """Rows of one to five entries, from small boxes and from cells that are their own region (two molecules
+    at most in the first three), with and without intramolecular entries; the mirror index pairs each entry
+    with the other one of its energy."""
+    from epsr_python_translation_b200.device import DeviceBox
+    box = BoxArrays.from_system(configs.c1_water(seed=nmol, nmol=nmol))
+    rmax = box.sepmax if rmax is None else f32(rmax)
+    eintra = np.zeros(nmol, f32) if zero else np.random.default_rng(nmol).standard_normal(nmol).astype(f32)
+    oc = oracle.cell_list(box, nmolcell, rmax)
+    ost = oracle.fmolec1(box, oc, eintra, capacity=nmol * (oc["nnbrefmax"] + 1))
+    d = DeviceBox(box)
+    d.cell_list(nmolcell, rmax)
+    d.fmolec1(eintra, strict=True)
+    st = d.download_store()
+    M, n = st["nnbrefmax"], st["nergpair"]
+    assert M == oc["nnbrefmax"] and n == ost["nergpair"]
+    assert_bits_equal(st["ergpair"], ost["ergpair"][:n], "ergpair")
+    assert np.array_equal(st["nergpairm"], ost["nergpairm"])
+    om, oref = ost["molergpair"].reshape(nmol, M), ost["ergpairref"].reshape(nmol, M)
+    mirror = d.s_mirror[:nmol * M].cpu().numpy()
+    for m in range(nmol):
+        k = int(st["nergpairm"][m])
+        assert np.array_equal(st["molergpair"][m, :k], om[m, :k]) and np.array_equal(st["ergpairref"][m, :k], oref[m, :k])
+        for s in range(k):
+            p = st["molergpair"][m, s]
+            if p != m:
+                e = int(mirror[m * M + s])
+                assert e // M == p and st["molergpair"][p, e % M] == m
+                assert st["ergpairref"][p, e % M] == st["ergpairref"][m, s]
