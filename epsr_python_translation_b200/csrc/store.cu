@@ -92,8 +92,11 @@ __global__ void region_build_kernel(const int32_t *start, const int32_t *mols, c
         carry += tot;
     }
     __syncthreads();
-    if (carry > M) {
-        if (threadIdx.x == 0) atomicExch(err, 1);
+    if (carry > M) {   // refused (epsr_fmolec1 reads err): the region is empty to the kernels that follow
+        if (threadIdx.x == 0) {
+            atomicExch(err, 1);
+            nn[c0] = 0;
+        }
         return;
     }
     if (threadIdx.x == 0) nn[c0] = carry;
@@ -355,9 +358,11 @@ __global__ void fm_sort_kernel(int M, const int32_t *rowcnt, int32_t *nergpairm,
     if (threadIdx.x == 0) nergpairm[m] = n;
 }
 
-// mirror index: the two entries that reference one energy slot point at each other
+// mirror index: the two entries that reference one energy slot point at each other (left alone when a
+// row overflowed: slots it never wrote hold anything)
 __global__ void mirror_claim_kernel(int nmol, int M, const int32_t *nergpairm, const int32_t *ergpairref,
-                                    int32_t *owners) {
+                                    int32_t *owners, const int32_t *err) {
+    if (*err) return;
     const int m = blockIdx.x;
     const int n = nergpairm[m];
     for (int s = threadIdx.x; s < n; s += blockDim.x) {
@@ -368,7 +373,8 @@ __global__ void mirror_claim_kernel(int nmol, int M, const int32_t *nergpairm, c
 }
 
 __global__ void mirror_set_kernel(int nmol, int M, const int32_t *nergpairm, const int32_t *ergpairref,
-                                  const int32_t *owners, int32_t *mirror) {
+                                  const int32_t *owners, int32_t *mirror, const int32_t *err) {
+    if (*err) return;
     const int m = blockIdx.x;
     const int n = nergpairm[m];
     for (int s = threadIdx.x; s < M; s += blockDim.x) {
@@ -611,8 +617,8 @@ extern "C" int epsr_fmolec1(const epsr_box_t *box, const epsr_cells_t *cells, co
             return EPSR_ERR_CAPACITY;
         }
         EPSR_CUDA(cudaMemsetAsync(owners, 0xff, sizeof(int32_t) * 2 * (size_t)ntot, s));
-        mirror_claim_kernel<<<nmol, 128, 0, s>>>(nmol, M, store->nergpairm, store->ergpairref, owners);
-        mirror_set_kernel<<<nmol, 128, 0, s>>>(nmol, M, store->nergpairm, store->ergpairref, owners, store->mirror);
+        mirror_claim_kernel<<<nmol, 128, 0, s>>>(nmol, M, store->nergpairm, store->ergpairref, owners, err);
+        mirror_set_kernel<<<nmol, 128, 0, s>>>(nmol, M, store->nergpairm, store->ergpairref, owners, store->mirror, err);
     }
     EPSR_CUDA(cudaGetLastError());
     int32_t herr[1];

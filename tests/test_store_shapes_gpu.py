@@ -125,3 +125,38 @@ def test_short_rows_match_oracle(nmol, nmolcell, rmax, zero):
                 e = int(mirror[m * M + s])
                 assert e // M == p and st["molergpair"][p, e % M] == m
                 assert st["ergpairref"][p, e % M] == st["ergpairref"][m, s]
+
+
+@pytest.mark.parametrize("nmol,nmolcell,rmax,M", [(100, 10, None, 1), (100, 10, None, 90), (200, 1, 0.1, 15),
+                                                  (200, 1, 0.1, 21)])
+def test_too_few_slots_are_refused(nmol, nmolcell, rmax, M):
+    """Regions of more molecules than the store has slots (all of them, some, the largest): refused with the
+    capacity error whatever the scratch held, and the box's next store, with the slots it needs, is the
+    oracle's."""
+    import torch
+
+    from epsr_python_translation_b200 import _lib
+    from epsr_python_translation_b200.device import DeviceBox
+    box = BoxArrays.from_system(configs.c1_water(seed=5, nmol=nmol))
+    rmax = box.sepmax if rmax is None else f32(rmax)
+    eintra = np.ones(nmol, f32)
+    oc = oracle.cell_list(box, nmolcell, rmax)
+    ost = oracle.fmolec1(box, oc, eintra, capacity=nmol * nmol)
+    d = DeviceBox(box)
+    d.cell_list(nmolcell, rmax)
+    need = d.nnbrefmax
+    assert need > M
+    nb = d.lib.epsr_fmolec1_scratch_bytes(nmol, d.cells.ncell, need)
+    d.scratch("fmolec1", nb).fill_(0x7f)
+    for name in ("_s_mol", "_s_ref"):
+        d._buf(name, nmol * need, torch.int32).fill_(0x7f7f7f7f)
+    d.nnbrefmax = M
+    with pytest.raises(_lib.EpsrGpuError) as e:
+        d.fmolec1(eintra, strict=True)
+    assert e.value.code == 3
+    d.nnbrefmax = need
+    d.fmolec1(eintra, strict=True)
+    st = d.download_store()
+    n = st["nergpair"]
+    assert n == ost["nergpair"] and np.array_equal(st["nergpairm"], ost["nergpairm"])
+    assert_bits_equal(st["ergpair"], ost["ergpair"][:n], "ergpair")
