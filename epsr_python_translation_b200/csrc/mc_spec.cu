@@ -949,7 +949,10 @@ struct WalkShared {
 };
 
 // Per move: each partner's visit position (-1: visited later) and the two stored energies its new
-// energy is compared with, {as the cycle began, after the partner's own move}.
+// energy is compared with, {as the cycle began, after the partner's own move}.  The exact cycles are open to
+// a store whose mirror index is stale (rows rewritten since it was built; the drop-in asks for a strict cycle
+// then), so every entry's mirror is checked to be its energy's entry in the partner's row: where one is
+// not, the sequential kernel, which needs none, runs the cycle.
 __global__ void __launch_bounds__(128) spec_terms_kernel(SpecDev S) {
     if (S.flags[0]) return;
     const int k = blockIdx.x;
@@ -958,13 +961,12 @@ __global__ void __launch_bounds__(128) spec_terms_kernel(SpecDev S) {
     const size_t row = (size_t)m * S.M, krow = (size_t)k * S.M;
     for (int s = 1 + threadIdx.x; s < nn; s += blockDim.x) {
         const size_t e = row + s;
-        const int kp = S.vpos[S.molergpair[e]];
-        const float sv = S.ergpair[S.ergpairref[e] - 1];
+        const int p = S.molergpair[e], kp = S.vpos[p], ref = S.ergpairref[e];
+        const float sv = S.ergpair[ref - 1];
         float after = sv;
-        if (kp < k) {
-            const int e2 = S.mirror[e];
-            if (e2 % S.M >= 1) after = S.A[e2];
-        }
+        const long long s2 = (long long)S.mirror[e] - (long long)p * S.M;   // the slot in the partner's row
+        if (s2 < 0 || s2 >= S.nergpairm[p] || S.ergpairref[(size_t)p * S.M + s2] != ref) atomicExch(S.flags, 1);
+        else if (kp < k && s2 >= 1) after = S.A[(size_t)p * S.M + s2];
         S.farkp[krow + s - 1] = kp < k ? kp : -1;
         S.fart[krow + s - 1] = make_float2(sv, after);
     }
