@@ -435,7 +435,8 @@ __global__ void __launch_bounds__(MC_THREADS, 1) molfit_seq_kernel(McDev D) {
             }
         }
         __syncthreads();
-        if (sh_rot) {
+        const bool turned = sh_rot != 0;   // the molecule's groups were
+        if (turned) {
             const int im = sh_im, n = sh_n;
             const size_t row = (size_t)im * D.M;
             const float fdiff = en_change_mv(im, n, true, true);
@@ -475,7 +476,10 @@ __global__ void __launch_bounds__(MC_THREADS, 1) molfit_seq_kernel(McDev D) {
             }
             __syncthreads();
         }
-        if (D.shake) continue;   // the intramolecular cycle moves no molecule whole (uniform branch)
+        if (D.shake) {   // the intramolecular cycle moves no molecule whole (uniform branches)
+            if (!turned) __syncthreads();   // every warp has read sh_rot before warp 0 writes the next molecule's
+            continue;
+        }
         // ---- whole-molecule rotation and translation (molfit.py:362-448)
         if (wid == 0) {
             const int im = sh_im;
