@@ -210,11 +210,15 @@ __global__ void __launch_bounds__(1024) press_sum_fast_kernel(PressDev P, int nm
     __shared__ double r0[32], r1[32];
     double a = 0.0, b = 0.0;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-    if (P.M >= 2)   // a row of one slot holds no other molecule
-        for (int im = threadIdx.x; im < nmol - 1; im += blockDim.x) {
+    for (int im = threadIdx.x; im < nmol - 1; im += blockDim.x) {
+        if (P.M >= 2) {
             a += get_double(P.ergold + (size_t)im * P.M);
             b += get_double(P.ergnew + (size_t)im * P.M);
+        } else if (P.nergpairm[im] > 0) {   // a row of one slot has no room for a sum, and is its sum
+            a += (double)P.ergold[im];
+            b += (double)P.ergnew[im];
         }
+    }
     a = warp_sum_d(a);
     b = warp_sum_d(b);
     if (lane == 0) {
