@@ -163,9 +163,10 @@ __global__ void __launch_bounds__(PR_THREADS) press_pairs_kernel(PressDev P, int
         P.ergnew[row + s] = en;
     }
     if (!fast) return;
-    // the molecule's sums, by slot, so that they don't depend on the lists' order
-    __shared__ double r0[PR_THREADS / 32], r1[PR_THREADS / 32];
+    // the molecule's sums, by slot, so that they don't depend on the lists' order; the warps' parts lie where
+    // the atoms were, since the list may take all the shared memory that is left
     __syncthreads();
+    double *r0 = (double *)sa, *r1 = r0 + PR_THREADS / 32;
     double se = 0.0, sp = 0.0;
     for (int s = threadIdx.x; s < nn; s += blockDim.x) {
         se += (double)P.ergold[row + s];

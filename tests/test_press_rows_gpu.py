@@ -1,5 +1,5 @@
-"""press on stores a caller laid out itself, with rows of one slot and more.  The two molecules' pair is the
-only term, so the fast sums are the strict ones."""
+"""press on stores a caller laid out itself, with rows of one slot and more, up to as many as the kernel's
+shared memory lists.  The two molecules' pair is the only term, so the fast sums are the strict ones."""
 
 import numpy as np
 import pytest
@@ -11,7 +11,7 @@ from epsr_python_translation_b200.box import BoxArrays
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("M", [1, 2, 3])
+@pytest.mark.parametrize("M", [1, 2, 3, 57788])
 def test_fast_press_of_one_pair(M):
     from epsr_python_translation_b200.device import DeviceBox
     box = BoxArrays.from_system(configs.c1_water(seed=2, nmol=2))
