@@ -737,8 +737,10 @@ static inline size_t al256f(size_t x) { return (x + 255) & ~(size_t)255; }
 // two CTAs with the stream's warp among their own, 3,240 now), up to seven beside
 // the generator's CTA, the portable cluster size; more only for rows that need the memory.  Rows
 // and terms for 256 threads: barriers of half the warps, and registers for the whole row.
+// A CTA's rows have what the static arrays leave of the 227 KB a CTA may have.
 static int fx_workers(int npt, int nterms, int ncoef, int *rpc_out, int *threads_out) {
-    const size_t budget = 200 * 1024;
+    constexpr size_t fixed = 10 * 1024, budget = 227 * 1024 - fixed;
+    static_assert(sizeof(FxGen) + sizeof(FxShared) <= fixed, "the static arrays are beside the rows");
     const int want = std::min((npt + FX_ROWS - 1) / FX_ROWS, FX_MAXW - 1);
     for (int c = std::max(want, 1); c <= FX_MAXW; ++c) {
         const int rpc = (npt + c - 1) / c;

@@ -20,6 +20,16 @@ f32 = np.float32
     (5, 3, 1, -7), (160, 16, 1, -8), (161, 17, 2, -9), (320, 128, 1, -10), (321, 129, 3, -11), (1120, 24, 1, -12),
     (1121, 20, 1, -13), (2100, 12, 1, -14), (150, 300, 1, -15), (90, 21, 1, -2147483647)])
 def test_fit_shapes_match_oracle(npt, nterms, ncfirst, seed):
+    _compare(npt, nterms, ncfirst, seed)
+
+
+@pytest.mark.parametrize("npt,nterms,seed", [(1464, 300, -16), (2432, 200, -17), (3072, 168, -18)])
+def test_largest_rows_match_oracle(npt, nterms, seed):
+    """Shapes whose rows take nearly all the shared memory of the largest cluster."""
+    _compare(npt, nterms, 1, seed)
+
+
+def _compare(npt, nterms, ncfirst, seed):
     from epsr_python_translation_b200 import transforms
     rng = np.random.default_rng(npt)
     expr = configs.ep_basis(configs.qgrid(npt, 0.05), nterms)
