@@ -89,8 +89,21 @@ __device__ __forceinline__ void st_async_f64(uint32_t a, double v, uint32_t bar)
 __device__ __forceinline__ void st_cl_s64(uint32_t a, long long v) {
     asm volatile("st.shared::cluster.b64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
 }
+__device__ __forceinline__ void st_relaxed_cl_s64(uint32_t a, long long v) {
+    asm volatile("st.relaxed.cluster.shared::cluster.b64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
+}
 __device__ __forceinline__ void st_release_cl_s32(uint32_t a, int v) {
     asm volatile("st.release.cluster.shared::cluster.b32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ long long ld_relaxed_s64(const long long *p) {
+    long long v;
+    asm volatile("ld.relaxed.cluster.shared::cta.b64 %0, [%1];" : "=l"(v) : "r"(smem_addr(p)) : "memory");
+    return v;
+}
+__device__ __forceinline__ int ld_acquire_s32(const int *p) {
+    int v;
+    asm volatile("ld.acquire.cluster.shared::cta.b32 %0, [%1];" : "=r"(v) : "r"(smem_addr(p)) : "memory");
+    return v;
 }
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory");
@@ -176,7 +189,6 @@ __device__ void fx_generate(const FxDev &F, FxGen &G, FxShared &S, unsigned long
         else r1_make(G.pair, *(volatile int *)&G.idum, h.mul, 0x7fffffff);
         return;
     }
-    volatile FxShared *vs = &S;
     Ran1Warp g;
     g.load(F.ran1);
     const int32_t mcall0 = F.ran1[2];
@@ -205,13 +217,18 @@ __device__ void fx_generate(const FxDev &F, FxGen &G, FxShared &S, unsigned long
             }
         }
     };
-    // room for a batch in every ring; false when the workers are done (or gave up: 2 s without room)
+    // room for a batch in every ring; false when the workers are done (or gave up: 2 s without room).  The
+    // values before the workers' cursor have been read, as the trial they decide depends on them, so
+    // no fence stands between the cursor and a slot's next value (a releasing store a trial: 3% of a fit).
+    long long limit = FX_RING;
     auto room = [&]() -> bool {
         unsigned long long t0 = 0;
         while (true) {
             __syncwarp();
-            if (vs->done) return false;
-            if (vs->cons + FX_RING - pos >= 32) return true;
+            if (*(volatile int *)&S.done) return false;
+            if (limit - pos >= 32) return true;
+            limit = ld_relaxed_s64(&S.cons) + FX_RING;
+            if (limit - pos >= 32) return true;
             int give_up = 0;
             if (lane == 0) {
                 const unsigned long long t = now_ns();
@@ -264,8 +281,8 @@ __device__ void fx_generate(const FxDev &F, FxGen &G, FxShared &S, unsigned long
     // the state after exactly the values taken, from the last checkpoint at or before it (or from
     // the launch's state when none is left)
     __syncwarp();
-    if (lane == 0 && vs->done == 1) {
-        const long long cursor = vs->cons;
+    if (lane == 0 && ld_acquire_s32(&S.done) == 1) {
+        const long long cursor = S.cons;   // stored before done
         int best = -1;
         for (int k = 0; k < FX_CK; ++k)
             if (G.ckpos[k] >= 0 && G.ckpos[k] <= cursor && (best < 0 || G.ckpos[k] > G.ckpos[best])) best = k;
@@ -663,7 +680,7 @@ __global__ void __launch_bounds__(T, 1) fitexp_cluster_kernel(FxDev F) {
                     const bool acc = metropolis(chisqnew, u, draw);
                     // every worker has taken the values before `cursor` (its part of chi^2 is here),
                     // but the draw at `cursor` perhaps not yet
-                    if (rank == 0 && tid == 0) st_cl_s64(gen_cons, cursor);
+                    if (rank == 0 && tid == 0) st_relaxed_cl_s64(gen_cons, cursor);
                     cursor += draw;
                     if (acc) {
                         wo = wn;
@@ -719,7 +736,7 @@ __global__ void __launch_bounds__(T, 1) fitexp_cluster_kernel(FxDev F) {
     // the generator leaves, and writes the state after the values taken unless a wait gave up
     block_sync();
     if (rank == 0 && tid == 0) {
-        st_cl_s64(gen_cons, cursor);
+        st_relaxed_cl_s64(gen_cons, cursor);
         st_release_cl_s32(gen_done, vs->abort ? 2 : 1);
     }
     __syncwarp();
