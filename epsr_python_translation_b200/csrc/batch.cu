@@ -79,16 +79,33 @@ __global__ void bmc_begin_kernel(epsr_bmc_t B) {
     X.colour_off = (int)(r.w % (uint32_t)ncol);
 }
 
+// The place of a box's extent, the largest distance of an atom from its molecule's centre: the word of
+// the bin cursors that no cell has.
+__device__ __forceinline__ int32_t *box_extent(const epsr_bmc_t &B, const epsr_bmc_box_t &X, int b) {
+    return B.mol_cell + B.nmol + X.cell0 + b + X.ncell * X.ncell * X.ncell;
+}
+
 __global__ void bmc_count_kernel(epsr_bmc_t B) {
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= B.nmol) return;
     const int b = B.mol_box[m];
     const epsr_bmc_box_t &X = B.box[b];
     const int n = X.ncell;
-    const int c = (cell_coord(B.xadd[m], X.shift[0], n) * n + cell_coord(B.yadd[m], X.shift[1], n)) * n +
-                  cell_coord(B.zadd[m], X.shift[2], n);
+    const float4 centre = make_float4(B.xadd[m], B.yadd[m], B.zadd[m], 0.0f);
+    const int c = (cell_coord(centre.x, X.shift[0], n) * n + cell_coord(centre.y, X.shift[1], n)) * n +
+                  cell_coord(centre.z, X.shift[2], n);
     B.mol_cell[m] = c;
     atomicAdd(B.cell_start + X.cell0 + b + c + 1, 1);
+    const float4 *p = (const float4 *)B.pos + B.naf[m];
+    float r2 = 0.0f;
+    for (int q = 0; q < B.nato[m]; ++q) {
+        const float d = dsq_cubic(centre, p[q]);
+        if (!(d <= r2) && r2 == r2) r2 = d;     // a NaN stays, and makes the extent infinite
+    }
+    const int mine = r2 >= 0.0f ? __float_as_int(sqrtf(r2)) : 0x7f800000;   // distances order as their bits
+    const unsigned same = __match_any_sync(__activemask(), b);
+    const int most = __reduce_max_sync(same, mine);
+    if ((int)(threadIdx.x & 31) == __ffs(same) - 1) atomicMax(box_extent(B, X, b), most);
 }
 
 // one CTA per box: inclusive scan of the counts into starts
@@ -252,8 +269,8 @@ __device__ __forceinline__ float4 atom_pos(const epsr_bmc_t &B, int a) { return 
 // an atom of the moved molecule that can interact: of the cells within `nr` of the move's cell
 // (each cell once, wrapped) the molecules other than the moved one whose centre is within sqrt(r2)
 // of its centre, and of those the atoms a whose old or new position is within sqrt(ra2) of the
-// partner's centre (ra: the range plus a molecule's extent, so every atom pair in range belongs
-// to an item).  process(partner, atoms, a) is called once per item, partners of more than four
+// partner's centre (ra: the range plus the largest extent of the box's molecules, so every atom pair in
+// range belongs to an item, whatever r2 the caller gave).  process(partner, atoms, a) is called once per item, partners of more than four
 // atoms first, so that the lanes of a warp loop over atom counts that are alike.  Returns the
 // molecules of the cells, the same in every thread.
 //
@@ -467,7 +484,7 @@ __device__ __forceinline__ int near_items(const epsr_bmc_t &B, const epsr_bmc_bo
                         const int e = (int)(((float)i + 0.5f) * inv_na), a = i - e * P.na;
                         const NearMol m = Q.mol[Q.near_[e]];
                         const float4 c = make_float4(m.x, m.y, m.z, 0.0f);
-                        in = dsq_cubic(P.p_old[a], c) <= P.ra2 || dsq_cubic(P.p_new[a], c) <= P.ra2;
+                        in = !(dsq_cubic(P.p_old[a], c) > P.ra2 && dsq_cubic(P.p_new[a], c) > P.ra2);
                         big = (m.mol & 127u) > 4u;
                     }
                     const unsigned k0 = __ballot_sync(0xffffffffu, in && !big), k1 = __ballot_sync(0xffffffffu, in && big);
@@ -508,10 +525,11 @@ __device__ __forceinline__ int near_items(const epsr_bmc_t &B, const epsr_bmc_bo
 using WideSearch = Search<2048, 4096>;     // CTAs of more than 256 threads (and every feature search)
 using NarrowSearch = Search<1024, 2048>;
 
-// The largest distance of an atom from its molecule's centre, from a range that was made as
-// range + 2 extents + the largest displacement of a centre (BatchBoxes' rint and rfeat_c).
-__device__ __forceinline__ float extent_of(float reach, float range, float transmax) {
-    return fmaxf(0.5f * (reach - range - 1.7320508f * transmax), 0.0f);
+// The distance from a partner's centre within which an atom can be in `range` of its atoms, squared: the
+// box's extent as the binning found it (a molecule keeps its shape but for roundings), with slack for those.
+__device__ __forceinline__ float item_range2(const epsr_bmc_t &B, const epsr_bmc_box_t &X, int b, float range) {
+    const float r = range + __int_as_float(*box_extent(B, X, b)) + 1e-6f;
+    return r * r * 1.00001f;
 }
 
 // ----------------------------------------------------------------- propose
@@ -625,9 +643,8 @@ __global__ void __launch_bounds__(BMC_MAXT) bmc_propose_kernel(epsr_bmc_t B, int
     // the distances of every item's atom before and after the move to the partner's atoms, binned
     // (no atom of a partner whose centre is beyond rfeat_c is within 8 A of the moved molecule)
     const int a00 = B.naf[mol];
-    const float ra = rf + extent_of(X.rfeat_c, rf, X.transmax) + 1e-6f;
     const Near P{ix, iy, iz, X.nrange_feat, na_, mol_word(B, X, mol), B.xadd[mol], B.yadd[mol], B.zadd[mol],
-                 __fmul_rn(X.rfeat_c, X.rfeat_c), ra * ra * 1.00001f, p_old, p_new};
+                 __fmul_rn(X.rfeat_c, X.rfeat_c), item_range2(B, X, b, rf), p_old, p_new};
     const int scanned = near_items(B, X, b, P, *(WideSearch *)bmc_smem, [&](int b0, int nb, int a) {
         const int ca = B.fclass[a00 + a];
         const float4 po = p_old[a], pn = p_new[a];
@@ -860,9 +877,8 @@ __global__ void __launch_bounds__(MAXT, 1024 / MAXT) bmc_decide_kernel(epsr_bmc_
     // molecules' extents and the largest displacement)
     int ix, iy, iz;
     slot_cell(X, k, step, ix, iy, iz);
-    const float rc = (float)(X.izcut + 1) * X.stepcl, ra = rc + extent_of(X.rint, rc, X.transmax) + 1e-6f;
     const Near P{ix, iy, iz, X.nrange, na_, mol_word(B, X, mol), B.xadd[mol], B.yadd[mol], B.zadd[mol],
-                 __fmul_rn(X.rint, X.rint), ra * ra * 1.00001f, p_old, p_new};
+                 __fmul_rn(X.rint, X.rint), item_range2(B, X, b, (float)(X.izcut + 1) * X.stepcl), p_old, p_new};
     double de = 0.0;
     bool here = !staged, late = false;   // the tables have arrived; they did not in time
     const int scanned = near_items(B, X, b, P, *(S *)bmc_smem, [&](int b0, int nb, int a) {

@@ -285,8 +285,11 @@ typedef struct {
     int32_t ncell, stride, cell0, slot0, nslot;  /* cells per side, colour stride, offsets, (ncell/stride)^3 */
     int32_t tab0, ld, izcut, npairref0, ntype, xstar0;   /* tables: float4 offset, ld, cutoff, pair map */
     int32_t nrange, nrange_feat;                 /* cells scanned on each side for energies / features */
-    float stepcl, beta, dmax, rint, rfeat;       /* rint, rfeat: box units */
-    float rfeat_c;                               /* centre distance beyond which no feature pair exists */
+    float stepcl, beta, dmax, rint, rfeat;       /* rint: the distance from the moved molecule's centre before
+                                                    its move within which a centre's atoms count (the range, the
+                                                    two extents and the displacement, or less where less will
+                                                    do); rfeat: the features' range; box units */
+    float rfeat_c;                               /* the same distance for features */
     float rotmax, transmax;                      /* radians, box units */
     uint32_t key0, key1;                         /* Philox key */
     float shift[3];                              /* written by each sweep's binning */
@@ -310,8 +313,8 @@ typedef struct {
     const int32_t *npairref;      /* packed type-pair maps */
     int32_t *cell_start;          /* [ncell + nbox] per box ncell^3+1 starts */
     int32_t *cell_mols;           /* [nmol] */
-    int32_t *mol_cell;            /* [nmol + 2*ncell + nbox] scratch: cell of each molecule, bin cursors,
-                                     then the box of each packed cell (host-written, after the cursors) */
+    int32_t *mol_cell;            /* [nmol + 2*ncell + nbox] scratch: cell of each molecule, bin cursors and
+                                     extents, then the box of each packed cell (host-written, after the cursors) */
     int32_t *slot_mol;            /* [nslot] molecule moved in the step, -1 none, -2 left its cell */
     float *slot_new;              /* [nslot*64*4] proposed absolute positions */
     float *slot_off;              /* [nslot*64*4] proposed offsets */
