@@ -631,12 +631,14 @@ __global__ void __launch_bounds__(SP_RT, 1) __cluster_dims__(2, 1, 1) spec_resol
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const uint32_t rank = blockIdx.x;
     const int nblk = (N + SP_BLK - 1) / SP_BLK;
-    for (int i = tid; i < SP_FR; i += blockDim.x) vfar[i] = 0ull;
     for (int i = tid; i < nblk; i += blockDim.x) vpub[i] = 0ull;
-    if (tid == 0) {
-        abort_flag = 0;
-        for (int i = 0; i < SP_NSLOT; ++i) umma::mbar_init(&bars[i], 1);
-        umma::fence_mbar_init();
+    if (tid == 0) abort_flag = 0;
+    if (rank == 0) {   // the second CTA's stages lie where these are
+        for (int i = tid; i < SP_FR; i += blockDim.x) vfar[i] = 0ull;
+        if (tid == 0) {
+            for (int i = 0; i < SP_NSLOT; ++i) umma::mbar_init(&bars[i], 1);
+            umma::fence_mbar_init();
+        }
     }
     cluster_sync_all();
     const float temp = __fdiv_rn(1.0f, S.simt);
