@@ -490,6 +490,13 @@ int check_net(const epsr_mlp_t *net, const char *who) {
     }
     return EPSR_OK;
 }
+
+// the activations in the work area are stored, and read by TMA, 16 bytes at a time
+bool work_aligned(const void *work, const char *who) {
+    if (((uintptr_t)work & 15) == 0) return true;
+    epsr_set_error("%s: work %p must be 16-byte aligned", who, work);
+    return false;
+}
 }  // namespace
 
 extern "C" int epsr_mlp_sync_weights(const epsr_mlp_t *net, void *stream) {
@@ -511,6 +518,7 @@ extern "C" int epsr_mlp_forward(const epsr_mlp_t *net, const void *x, int32_t ro
         epsr_set_error("epsr_mlp_forward: null pointer or no rows");
         return EPSR_ERR_ARG;
     }
+    if (!work_aligned(work, "epsr_mlp_forward")) return EPSR_ERR_ARG;
     if (work_bytes < epsr_mlp_work_bytes(rows)) {
         epsr_set_error("epsr_mlp_forward: work needs %lld bytes", (long long)epsr_mlp_work_bytes(rows));
         return EPSR_ERR_CAPACITY;
@@ -544,6 +552,7 @@ extern "C" int epsr_mlp_train_step(const epsr_mlp_t *net, const void *x, const v
         epsr_set_error("epsr_mlp_train_step: null pointer, or rows/row0 not multiples of 128, or ldxt too small");
         return EPSR_ERR_ARG;
     }
+    if (!work_aligned(work, "epsr_mlp_train_step")) return EPSR_ERR_ARG;
     if (work_bytes < epsr_mlp_work_bytes(rows)) {
         epsr_set_error("epsr_mlp_train_step: work needs %lld bytes", (long long)epsr_mlp_work_bytes(rows));
         return EPSR_ERR_CAPACITY;
