@@ -553,6 +553,10 @@ extern "C" int epsr_fmolec1(const epsr_box_t *box, const epsr_cells_t *cells, co
     float *sums = (float *)take(sizeof(float) * 2);
     const size_t own_n = 2 * ((size_t)nmol + (size_t)nmol * M / 2 + 16);
     int32_t *owners = (int32_t *)take(sizeof(int32_t) * own_n);
+    // centres, then partial sums, lie where the mirror's owners come later, on a 16-byte boundary of their own
+    // (the scratch may have four bytes'; the owners' last 16 pairs are spare); rows of one slot have no room
+    // for the centres, and no entry to look at
+    float4 *ctr = (float4 *)(((uintptr_t)owners + 15) & ~(uintptr_t)15);
     float *ebuf = (float *)take(sizeof(float) * (size_t)nmol * M);
     EPSR_CUDA(cudaMemsetAsync(err, 0, sizeof(int32_t) * 8, s));
 
@@ -560,13 +564,13 @@ extern "C" int epsr_fmolec1(const epsr_box_t *box, const epsr_cells_t *cells, co
     Prefilter P;
     P.on = box->cubic ? 1 : 0;
     P.cut = (float)((double)(B.T.izcut - 1) * (double)box->stepcl * 1.00001 + 1.0e-6);
-    P.ctr = (const float4 *)owners;   // of later; rows of one slot have no room, and no entry to look at
+    P.ctr = ctr;
     const int noff = cells->ncellneighb;
     positions_kernel<<<nmol, 32, 0, s>>>(box->naf, box->nato, box->itype, box->xa, box->ya, box->za, box->xadd,
                                          box->yadd, box->zadd, nmol, (float4 *)box->pos);
     if (P.on && M >= 2)
         mol_centre_kernel<<<(nmol + 127) / 128, 128, 0, s>>>(box->naf, box->nato, box->xa, box->ya, box->za, box->xadd,
-                                                             box->yadd, box->zadd, nmol, (float4 *)owners);
+                                                             box->yadd, box->zadd, nmol, ctr);
     region_build_kernel<<<ncell, 256, sizeof(int32_t) * 2 * (size_t)noff, s>>>(
         cells->cell_start, cells->cell_mols, cells->offsets, noff, cells->ncelldiva, cells->ncelldivb,
         cells->ncelldivc, M, reg, nn, err);
@@ -604,10 +608,10 @@ extern "C" int epsr_fmolec1(const epsr_box_t *box, const epsr_cells_t *cells, co
     }
     if (shm > 48 * 1024) EPSR_SMEM_OPTIN(fm_sort_kernel);
     fm_sort_kernel<<<nmol, 256, shm, s>>>(M, rowcnt, store->nergpairm, store->molergpair, store->ergpairref, cap);
-    // the parts lie where the mirror's owners come later (8 bytes an entry, 16 a part)
+    // 16 bytes a part, where an entry has 8
     const int64_t nsum = ntot > nmol ? ntot : nmol;
     const int nparts = strict || nsum <= FM_SUM ? 1 : (int)(nsum < 256 * FM_SUM ? (nsum + FM_SUM - 1) / FM_SUM : 256);
-    double *part = (double *)owners;
+    double *part = (double *)ctr;
     fm_sums_kernel<<<nparts, strict ? 32 : 1024, 0, s>>>(store->ergpair, nintra, (int)ntot, eintra, nmol, strict,
                                                                     sums, part);
     if (nparts > 1) fm_parts_kernel<<<1, 256, 0, s>>>(part, nparts, nmol, sums);

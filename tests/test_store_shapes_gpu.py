@@ -160,3 +160,28 @@ def test_too_few_slots_are_refused(nmol, nmolcell, rmax, M):
     n = st["nergpair"]
     assert n == ost["nergpair"] and np.array_equal(st["nergpairm"], ost["nergpairm"])
     assert_bits_equal(st["ergpair"], ost["ergpair"][:n], "ergpair")
+
+
+@pytest.mark.parametrize("off", [4, 8, 12])
+def test_scratch_on_a_four_byte_boundary(off):
+    """The store needs four-byte alignment of its scratch, no more."""
+    import torch
+
+    from epsr_python_translation_b200.device import DeviceBox
+    box = BoxArrays.from_system(configs.c2_mixture(seed=4, ndmso=41, nwater=83))
+    eintra = np.random.default_rng(1).standard_normal(box.nmol).astype(f32)
+    out = []
+    for shift in (0, off):
+        d = DeviceBox(box)
+        d.cell_list(7, box.sepmax)
+        buf = torch.zeros(d.lib.epsr_fmolec1_scratch_bytes(box.nmol, d.cells.ncell, d.nnbrefmax) + 16, dtype=torch.uint8,
+                          device="cuda")
+        d.scratch = lambda name, nb, buf=buf, shift=shift: buf[shift:shift + nb]
+        sums = d.fmolec1(eintra, strict=True), d.fmolec1(eintra, strict=False)
+        st = d.download_store()
+        out.append((sums, st, d.s_mirror[:box.nmol * d.nnbrefmax].cpu().numpy()))
+        assert not buf[:shift].any()
+    (s0, a, m0), (s1, b, m1) = out
+    assert s0 == s1 and np.array_equal(m0, m1) and a["nergpair"] == b["nergpair"]
+    assert all(np.array_equal(a[k], b[k]) for k in ("nergpairm", "molergpair", "ergpairref"))
+    assert_bits_equal(a["ergpair"], b["ergpair"], "ergpair")
