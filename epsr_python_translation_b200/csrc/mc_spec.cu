@@ -1560,9 +1560,10 @@ int epsr_molfit_spec(const epsr_box_t *box, const epsr_cells_t *cells, epsr_stor
 }
 
 // Whether the walk takes a cycle of this box: its decisions fit, the store has its mirror index
-// and the scratch is the fast path's (a caller of the strict cycle may have given none).
+// and the scratch is the fast path's, on the 16-byte boundary its positions need (a caller of the
+// strict cycle may have given none, or one for the sequential kernel's words).
 bool epsr_molfit_walk_fits(const epsr_box_t *box, const epsr_store_t *store, const void *scratch, int64_t scratch_bytes) {
-    return box->nmol <= WK_MAXN && store->mirror && scratch && box->maxat <= SP_MAXAT &&
+    return box->nmol <= WK_MAXN && store->mirror && scratch && ((uintptr_t)scratch & 15) == 0 && box->maxat <= SP_MAXAT &&
            (int64_t)spec_bytes(box->nmol, box->natom, store->nnbrefmax, box->nmoltype) <= scratch_bytes &&
            sizeof(float) * 2 * (size_t)store->nnbrefmax <= 160 * 1024;
 }

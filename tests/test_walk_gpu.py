@@ -93,3 +93,21 @@ def test_stale_mirror_goes_to_the_sequential_kernel(name, groups):
         ca, cb = a.download_coords(), b.download_coords()
         assert all(np.array_equal(ca[k].view(np.uint32), cb[k].view(np.uint32)) for k in ca)
         assert np.array_equal(a.download_store()["ergpair"], b.download_store()["ergpair"])
+
+
+@pytest.mark.parametrize("off", [4, 8])
+def test_scratch_on_a_four_byte_boundary(off):
+    """A scratch that only the sequential kernel can use: the same strict cycles as on any other."""
+    s = SYSTEMS["mixture_45"]()
+    a, b = _box(s, False), _box(s, False)
+    nb = b.lib.epsr_molfit_scratch_bytes(s.nmol, s.natom, b.nnbrefmax)
+    buf = torch.zeros(nb + 16, dtype=torch.uint8, device="cuda")
+    b.scratch = lambda name, n: buf[off:off + n]
+    for _ in range(2):
+        for d in (a, b):
+            d.molfit(strict=True)
+            d.check_status()
+        x, y = a.download_mc(), b.download_mc()
+        assert np.array_equal(x["acc"], y["acc"]) and np.array_equal(x["den"].view(np.uint32), y["den"].view(np.uint32))
+        assert np.array_equal(a.download_store()["ergpair"], b.download_store()["ergpair"])
+    assert not buf.any()
