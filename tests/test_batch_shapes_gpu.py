@@ -68,3 +68,23 @@ def test_cell_members_ascend(natom):
     for c in range(nc0):
         assert np.all(np.diff(mols[s[c]:s[c + 1]]) > 0)
     assert np.array_equal(np.sort(mols[:m0]), np.arange(m0))
+
+
+def test_feature_rows_on_a_two_byte_boundary():
+    """Recorded features may lie at any element of the caller's array."""
+    from epsr_python_translation_b200.batch import FEAT_IN, BatchBoxes
+    out = []
+    for off in (0, 1, 3):
+        bb = BatchBoxes([configs.c1_water(seed=21, nmol=40)], rot_deg=20.0, trans_A=0.6, seed=9)
+        per = bb.steps_per_sweep * bb.nslot
+        flat = torch.zeros(2 * per * FEAT_IN + 4, dtype=torch.bfloat16, device="cuda")
+        rec = {"x": flat[off:off + 2 * per * FEAT_IN].view(2 * per, FEAT_IN),
+               "t": torch.zeros(per, dtype=torch.float32, device="cuda"), "n": 0}
+        assert rec["x"].data_ptr() % 4 == 2 * (off % 2)
+        bb.sweep("record", record=rec)
+        bb.check_status()
+        out.append((rec["x"].contiguous().view(torch.int16).cpu().numpy(), rec["t"].cpu().numpy()))
+        assert not flat[:off].any() and not flat[off + 2 * per * FEAT_IN:].any()
+    for x, t in out[1:]:
+        assert np.array_equal(x, out[0][0]) and x.any()
+        assert np.array_equal(t.view(np.uint32), out[0][1].view(np.uint32))
