@@ -141,11 +141,14 @@ namespace epsr {
 // the floats of bit patterns lo .. hi - 1
 __global__ void check_pair_math_kernel(int what, uint32_t lo, uint32_t hi, float par, unsigned long long *bad) {
     unsigned long long n = 0;
-    const float rcp = step_rcp(par, 4000);
+    const float rcp = step_rcp(par, 4000), wide = step_half(16384);
     for (uint64_t i = lo + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < hi; i += (uint64_t)gridDim.x * blockDim.x) {
         const float x = __uint_as_float((uint32_t)i);
         if (what == 0) n += __float_as_uint(sqrt_unit(x)) != __float_as_uint(__fsqrt_rn(x));
-        else if (what == 1) n += bin_index(x, par, rcp) != ifix(__fdiv_rn(x, par));
+        else if (what == 1) {
+            const int iz = ifix(__fdiv_rn(x, par));
+            n += (iz <= 4000 && bin_index(x, par, rcp) != iz) || bin_index(x, par, rcp, wide) != iz;
+        }
         else n += __float_as_uint(wrap_sq_small(x)) != __float_as_uint(wrap_sq(x));
     }
     if (n) atomicAdd(bad, n);

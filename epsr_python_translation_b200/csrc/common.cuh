@@ -154,15 +154,18 @@ __device__ __forceinline__ float dsq_cubic(float4 a, float4 b) {
 // 7.3e-4 of the rounded quotient while that is at most 4096, so its integer part is the index
 // unless it lies within 1e-3 of an integer; there (and for a NaN) the division decides.
 // rcp = step_rcp(stepcl, largest index asked for) is NaN, which always divides, beyond 4000.
-__host__ __device__ inline float step_rcp(float stepcl, int izmax) {
-    return izmax <= 4000 ? 1.0f / stepcl : nanf("");
+// With `half` = step_half of the largest index, the same up to 16,384 (2.93e-3, of 4e-3).
+constexpr float STEP_HALF = 0.499f;
+__host__ __device__ inline float step_half(int izmax) { return izmax <= 4000 ? STEP_HALF : 0.496f; }
+__host__ __device__ inline float step_rcp(float stepcl, int izmax, int limit = 4000) {
+    return izmax <= limit ? 1.0f / stepcl : nanf("");
 }
-__device__ __forceinline__ int bin_index(float d, float stepcl, float rcp) {
+__device__ __forceinline__ int bin_index(float d, float stepcl, float rcp, float half = STEP_HALF) {
     const float q = __fmul_rn(d, rcp);
     const float big = __fadd_rz(q, 8388608.0f);          // 2^23 + trunc(q), 0 <= q < 2^23
     const float fr = __fsub_rn(q, __fsub_rn(big, 8388608.0f));
     int n = __float_as_int(big) - 0x4b000000;
-    if (!(fabsf(__fsub_rn(fr, 0.5f)) < 0.499f)) n = ifix(__fdiv_rn(d, stepcl));
+    if (!(fabsf(__fsub_rn(fr, 0.5f)) < half)) n = ifix(__fdiv_rn(d, stepcl));
     return n;
 }
 
@@ -183,10 +186,11 @@ __device__ __forceinline__ float sqrt_unit(float x) {
 }
 
 // pair_energy for a cubic box in box units, bit for bit, with the branch-free root, wrap and
-// index above; rcp = step_rcp(T.stepcl, T.izcut)
-__device__ __forceinline__ float pair_energy_unit(const Tables &T, float rcp, float4 p1, float4 p2, int icref) {
+// index above; rcp = step_rcp(T.stepcl, T.izcut), half as bin_index's
+__device__ __forceinline__ float pair_energy_unit(const Tables &T, float rcp, float4 p1, float4 p2, int icref,
+                                                  float half = STEP_HALF) {
     const float d = sqrt_unit(dsq_cubic(p1, p2));
-    const int iz = bin_index(d, T.stepcl, rcp) + 2;
+    const int iz = bin_index(d, T.stepcl, rcp, half) + 2;
     const int izc = min(max(iz, 2), T.izcut);
     const float4 t = __ldg(T.tab + (size_t)icref * T.ld + izc);
     const float dt = __fsub_rn(d, __ldg(T.xstar + izc));

@@ -94,7 +94,7 @@ struct SpecDev {
     int32_t *acc;                          // [N] by visit position
     float *fdiff;                          // [N] by visit position
     double *fadd_acc;                      // [1]
-    float rcp;                             // step_rcp of the tables
+    float rcp, half;                       // step_rcp and step_half of the tables
     int ev;                                // the energy pass's staged values per chunk (>= 2 maxat^2)
     const int32_t *ngrot;                  // [N] rotational groups of each molecule, or NULL
     int32_t *ninter;                       // [2*nmoltype] zeroed by a cycle without internal rotations, or NULL
@@ -450,9 +450,9 @@ __global__ void __launch_bounds__(SP_ET, SP_EN_MINB) spec_energy_kernel(SpecDev 
                           c2 = col[__float_as_int(q2.w) * ntype];
                 float e0, e1, e2;
                 if (CUBIC) {
-                    e0 = pair_energy_unit(T, S.rcp, q0, p2, c0);
-                    e1 = pair_energy_unit(T, S.rcp, q1, p2, c1);
-                    e2 = pair_energy_unit(T, S.rcp, q2, p2, c2);
+                    e0 = pair_energy_unit(T, S.rcp, q0, p2, c0, S.half);
+                    e1 = pair_energy_unit(T, S.rcp, q1, p2, c1, S.half);
+                    e2 = pair_energy_unit(T, S.rcp, q2, p2, c2, S.half);
                 } else {
                     e0 = pair_energy(L, T, q0, p2, c0);
                     e1 = pair_energy(L, T, q1, p2, c1);
@@ -1480,7 +1480,8 @@ int epsr_molfit_spec(const epsr_box_t *box, const epsr_cells_t *cells, epsr_stor
     S.acc = (int32_t *)take(sizeof(int32_t) * N);
     S.fdiff = (float *)take(sizeof(float) * N);
     S.fadd_acc = (double *)take(sizeof(double));
-    S.rcp = step_rcp(S.T.stepcl, S.T.izcut);
+    S.rcp = step_rcp(S.T.stepcl, S.T.izcut, 16384);
+    S.half = step_half(S.T.izcut);
 
     // draws ahead: only with a buffer that holds a whole cycle's values (at most 7 a move)
     const bool ahead = mc->ahead && mc->ahead_cap >= (int64_t)N * 7;

@@ -37,6 +37,12 @@ def test_table_index_equals_the_division(stepcl):
     assert _mismatches(1, 0, 1, stepcl) == 0
 
 
+@pytest.mark.parametrize("stepcl", [0.002 / 31.7, 0.001 / 84.3, 0.87 / 16384])
+def test_table_index_of_fine_grids(stepcl):
+    import numpy as np
+    assert _mismatches(1, 0x20000000, int(np.float32(16384.0 * stepcl).view(np.uint32)), stepcl) == 0
+
+
 def test_minimum_image_square():
     import numpy as np
     top = int(np.float32(4.0).view(np.uint32))
