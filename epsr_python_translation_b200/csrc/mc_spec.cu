@@ -324,38 +324,13 @@ __global__ void spec_propose_kernel(SpecDev S) {
 }
 
 // ----------------------------------------------------------------- energies
-// E(a, b): a's atoms in shared memory (sa), b's absolute positions in global memory (read
-// through the L1 cache for every atom of a, which keeps registers -- and so resident warps --
-// free for latency hiding).
-// Both energies of one partner in one pass over its atoms: A against its cycle-start
-// position (pa), B against its proposed position (pn) when has_b; each summed ia outer, ja
-// inner as en_change, so each is the reference's value.
-__device__ __forceinline__ void mol_energy_ab(const Lattice &L, const Tables &T, const float4 *sa, int na,
-                                              const float4 *__restrict__ pa, const float4 *__restrict__ pn, int nb,
-                                              bool has_b, const int *spr, int ntype, float &ea, float &eb) {
-    float xa = 0.0f, xb = 0.0f;
-    for (int ia = 0; ia < na; ++ia) {
-        const float4 p1 = sa[ia];
-        const int *row = spr + __float_as_int(p1.w) * ntype;
-#pragma unroll 2
-        for (int j = 0; j < nb; ++j) {
-            const float4 p2 = __ldg(pa + j);
-            const int ic = row[__float_as_int(p2.w)];
-            xa = __fadd_rn(xa, pair_energy(L, T, p1, p2, ic));
-            if (has_b) xb = __fadd_rn(xb, pair_energy(L, T, p1, __ldg(pn + j), ic));
-        }
-    }
-    ea = xa;
-    eb = xb;
-}
-
 // One CTA per move.  The stored partners are taken in chunks of at most one per thread whose
 // pair values fit the staging area; a chunk is spread over the CTA as items (partner, partner
 // atom ja, which position: cycle start or proposed), each item evaluating its atom against
 // every atom ia of the moved molecule into the staging area at [ia][ja], and then one thread
 // per partner sums its values in the reference's order (ia outer, ja inner, from +0).  Every
-// pair value is pair_energy of the same operands as en_change, so A and B are the values of
-// mol_energy_ab bit for bit; the items keep a partner's nine (water) or more pair evaluations
+// pair value is pair_energy of the same operands as en_change, so A and B are the reference's
+// values; the items keep a partner's nine (water) or more pair evaluations
 // independent of each other instead of one thread's dependent chain of table loads.
 
 __device__ __forceinline__ int warp_incl_scan(int v, int lane) {

@@ -74,10 +74,6 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, i
         "l"((uint64_t)map), "r"(x), "r"(y), "r"(smem_u32(bar))
         : "memory");
 }
-__device__ __forceinline__ void prefetch_tmap(const CUtensorMap *map) {
-    asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)map) : "memory");
-}
-// generic-proxy shared-memory writes made visible to the async proxy (the MMA's operand reads)
 // One contiguous copy global -> this CTA's shared memory by the bulk-copy engine, completing
 // `bytes` of transaction on the mbarrier (both addresses 16-byte aligned, bytes a multiple of 16).
 __device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
@@ -86,6 +82,8 @@ __device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t b
                  "l"(src), "r"(bytes), "r"(smem_u32(bar))
                  : "memory");
 }
+// generic-proxy accesses of shared memory ordered before the async proxy's that follow (a copy into a slot that
+// was read)
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 // ----------------------------------------------------------------- tcgen05
