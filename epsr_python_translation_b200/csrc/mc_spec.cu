@@ -1330,6 +1330,17 @@ static size_t spec_bytes(int N, int natom, int M, int nmt) {
     return b;
 }
 
+// the energy pass's staged values per chunk (two positions of the largest pair of molecules at least), and its
+// shared memory: those, their items and the type pairs
+static int spec_staged_values(const epsr_box_t *box) {
+    const int ma = box->maxat > 0 && box->maxat <= SP_MAXAT ? box->maxat : SP_MAXAT;
+    return max(2 * ma * ma, 4096);
+}
+static size_t spec_energy_bytes(const epsr_box_t *box) {
+    const size_t ev = (size_t)spec_staged_values(box);
+    return sizeof(float) * ev + sizeof(uint16_t) * ((ev + 1) & ~(size_t)1) + sizeof(int) * (size_t)box->ntype * box->ntype;
+}
+
 extern "C" int64_t epsr_molfit_spec_scratch_bytes(int32_t nmol, int32_t natom, int32_t M, int32_t nmoltype) {
     return (int64_t)spec_bytes(nmol, natom, M, nmoltype);
 }
@@ -1457,6 +1468,7 @@ int epsr_molfit_spec(const epsr_box_t *box, const epsr_cells_t *cells, epsr_stor
     S.fadd_acc = (double *)take(sizeof(double));
     S.rcp = step_rcp(S.T.stepcl, S.T.izcut, 16384);
     S.half = step_half(S.T.izcut);
+    S.ev = spec_staged_values(box);
 
     // draws ahead: only with a buffer that holds a whole cycle's values (at most 7 a move)
     const bool ahead = mc->ahead && mc->ahead_cap >= (int64_t)N * 7;
@@ -1486,12 +1498,7 @@ int epsr_molfit_spec(const epsr_box_t *box, const epsr_cells_t *cells, epsr_stor
         EPSR_CUDA(cudaEventRecord(as->join, as->st));
     }
     EPSR_TIMED("spec_propose_kernel", s, spec_propose_kernel<<<(N + 127) / 128, 128, 0, s>>>(S));
-    {
-        const int ma = box->maxat > 0 && box->maxat <= SP_MAXAT ? box->maxat : SP_MAXAT;
-        S.ev = max(2 * ma * ma, 4096);
-    }
-    const size_t en_bytes = sizeof(float) * (size_t)S.ev + sizeof(uint16_t) * (size_t)((S.ev + 1) & ~1) +
-                            sizeof(int) * (size_t)box->ntype * box->ntype;
+    const size_t en_bytes = spec_energy_bytes(box);
     if (S.L.cubic) {
         EPSR_SMEM_OPTIN(spec_energy_kernel<true>);
         EPSR_TIMED("spec_energy_kernel", s, spec_energy_kernel<true><<<N, SP_ET, en_bytes, s>>>(S));
@@ -1535,11 +1542,12 @@ int epsr_molfit_spec(const epsr_box_t *box, const epsr_cells_t *cells, epsr_stor
     return molfit_seq_launch(box, cells, store, mc, nullptr, 0, s, S.flags, mode == 1);
 }
 
-// Whether the walk takes a cycle of this box: its decisions fit, the store has its mirror index
-// and the scratch is the fast path's, on the 16-byte boundary its positions need (a caller of the
-// strict cycle may have given none, or one for the sequential kernel's words).
+// Whether the walk takes a cycle of this box: its decisions fit, and its atom types' pairs the energy pass's
+// shared memory (which 220 or so types use up); the store has its mirror index; and the scratch is the fast
+// path's, on the 16-byte boundary its positions need (a caller of the strict cycle may have given none, or one
+// for the sequential kernel's words).
 bool epsr_molfit_walk_fits(const epsr_box_t *box, const epsr_store_t *store, const void *scratch, int64_t scratch_bytes) {
     return box->nmol <= WK_MAXN && store->mirror && scratch && ((uintptr_t)scratch & 15) == 0 && box->maxat <= SP_MAXAT &&
            (int64_t)spec_bytes(box->nmol, box->natom, store->nnbrefmax, box->nmoltype) <= scratch_bytes &&
-           sizeof(float) * 2 * (size_t)store->nnbrefmax <= 160 * 1024;
+           sizeof(float) * 2 * (size_t)store->nnbrefmax <= 160 * 1024 && spec_energy_bytes(box) <= 200 * 1024;
 }

@@ -111,3 +111,27 @@ def test_scratch_on_a_four_byte_boundary(off):
         assert np.array_equal(x["acc"], y["acc"]) and np.array_equal(x["den"].view(np.uint32), y["den"].view(np.uint32))
         assert np.array_equal(a.download_store()["ergpair"], b.download_store()["ergpair"])
     assert not buf.any()
+
+
+def _same(a, b):
+    for d in (a, b):
+        d.molfit(strict=True)
+        d.check_status()
+    x, y = a.download_mc(), b.download_mc()
+    assert np.array_equal(x["acc"], y["acc"]) and np.array_equal(x["den"].view(np.uint32), y["den"].view(np.uint32))
+    assert np.array_equal(x["ran1"].as_array(), y["ran1"].as_array())
+    assert np.array_equal(a.download_store()["ergpair"], b.download_store()["ergpair"])
+
+
+@pytest.mark.parametrize("ntype", [190, 240])
+def test_strict_cycles_of_boxes_with_many_atom_types(ntype):
+    """The type pairs of 240 types do not fit the energy pass's shared memory; the sequential kernel reads them
+    where they are."""
+    s = SYSTEMS["mixture_45"]()
+    a, b = _box(s, False), _box(s, False)
+    n = s.ntype
+    ref = torch.zeros(ntype, ntype, dtype=torch.int32, device="cuda")
+    ref[:n, :n] = a.npairref.reshape(n, n)
+    a.cbox.ntype, a.cbox.npairref = ntype, ref.data_ptr()
+    for _ in range(2):
+        _same(a, b)
