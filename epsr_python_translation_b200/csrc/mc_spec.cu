@@ -266,7 +266,9 @@ __global__ void spec_propose_kernel(SpecDev S) {
     const float pi = 3.14159265358979323846f;
     const int m = S.visit[k];
     const int n = S.nato[m];
-    if (n > SP_MAXAT) {   // beyond this path's per-molecule arrays: the sequential kernel refuses the cycle
+    // beyond this path's per-molecule arrays, which the sequential kernel refuses, or beyond what box->maxat
+    // says, on which the staging of the energy pass rests: that kernel needs none and runs the cycle
+    if (n > SP_MAXAT || 2 * n * n > S.ev) {
         atomicExch(S.flags, 1);
         return;
     }

@@ -113,6 +113,13 @@ def test_scratch_on_a_four_byte_boundary(off):
     assert not buf.any()
 
 
+def _chains(seed=9):
+    """Molecules of 64 atoms (the largest the kernels take), of 46 and of three."""
+    grid = np.stack(np.meshgrid(*[np.arange(4)] * 3, indexing="ij"), -1).reshape(-1, 3) * 1.6
+    big, mid = (configs.MolTemplate(k, ["C"] * n, grid[:n] - grid[:n].mean(axis=0)) for k, n in (("big", 64), ("mid", 46)))
+    return configs.build_system("chains", [big, mid, configs.water_template()], [2, 2, 6], 30.0, seed=seed)
+
+
 def _same(a, b):
     for d in (a, b):
         d.molfit(strict=True)
@@ -121,6 +128,19 @@ def _same(a, b):
     assert np.array_equal(x["acc"], y["acc"]) and np.array_equal(x["den"].view(np.uint32), y["den"].view(np.uint32))
     assert np.array_equal(x["ran1"].as_array(), y["ran1"].as_array())
     assert np.array_equal(a.download_store()["ergpair"], b.download_store()["ergpair"])
+
+
+@pytest.mark.parametrize("maxat", [0, 64, 45, 3])
+def test_largest_molecules_and_a_box_that_understates_them(maxat):
+    """The sequential kernel never read the box's maxat; where it is less than the molecules have, their strict
+    cycles go there."""
+    s = _chains()
+    a, b = _box(s, False), _box(s, False)
+    assert np.count_nonzero(a.s_nergpairm.cpu().numpy() > 1) >= 4
+    a.cbox.maxat = maxat
+    b.store.mirror = None
+    for _ in range(2):
+        _same(a, b)
 
 
 @pytest.mark.parametrize("ntype", [190, 240])
