@@ -205,7 +205,7 @@ __global__ void spec_plan_kernel(SpecDev S) {
     __syncthreads();   // off[N], the cycle's draw count
     // the cycle's ran1 values, from a copy of the state (a discarded cycle leaves the real state
     // untouched): the draws ahead when the previous cycle left them for exactly this state and
-    // count, else walked here by the first two warps
+    // count, else walked here by the first three warps
     const int lane = tid & 31;
     const int32_t count = S.off[S.N];
     bool ok = false;

@@ -2,8 +2,8 @@
 // distances by pair type in shared memory (the intermolecular pass of atogen,
 // ato_manipulation_rev4.py:3780-3850).
 //
-// What bounds it: instruction issue, 53 instructions a pair of which many issue every other cycle (68%
-// of the issue slots filled), then the shared-memory adds (2.3 wavefronts a warp).  Distance and bin
+// What bounds it: instruction issue, 55 instructions a pair of which many issue every other cycle (85%
+// of the issue slots of active cycles filled), then the shared-memory adds (2.3 wavefronts a warp).  Distance and bin
 // therefore avoid the conversion unit and the division, and the root is branch-free (common.cuh), the pair
 // type's row comes from shared memory, four targets are in flight, a tile that counts whole is run
 // without comparing molecules, and a pair's closest-contact test compares against the largest contact

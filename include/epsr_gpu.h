@@ -145,17 +145,22 @@ typedef struct {
                                        device cosine (test hook for bit-identity) */
     float *trace_den;               /* NULL or [nmol]: en_change value per move */
     int32_t *trace_acc;             /* NULL or [nmol]: 1 accepted, 0 rejected */
-    int32_t strict;                 /* 1: the sequential kernel, en_change summed in list
-                                       order (bit-identical); 0: the fast path -- every
-                                       proposal and pair energy of the cycle computed in
-                                       parallel, decisions resolved in visit order, each
-                                       move's change summed in double */
+    int32_t strict;                 /* 1: en_change summed in list order (bit-identical);
+                                       0: each move's change summed in double.  Either way
+                                       the proposals and pair energies of the cycle are
+                                       computed in parallel and the decisions resolved in
+                                       visit order, except by the sequential kernel: cycles
+                                       with internal rotations, and strict cycles without
+                                       what the parallel form needs (a mirror index that
+                                       fits the rows, scratch of
+                                       epsr_molfit_spec_scratch_bytes on 16 bytes, at most
+                                       65,536 molecules and about 220 atom types) */
     int32_t *status;                /* [1] device: 0 ok, 1 a molecule exceeds 64 atoms,
                                        2 the fast path's resolver timed out (cycle not applied) */
     /* Internal rotations of rotational groups before each molecule's whole-molecule move
      * (molfit.py:295-360, rotati :589): set intra (NULL: none).  Groups of type ROT or DIH; the
      * dihedral terms of DIH groups (en_mole_dihedral :1353) come from the dihedral block of the
-     * epsr_intra_t.  With intra set, every cycle runs the sequential kernel. */
+     * epsr_intra_t.  A cycle with rotations runs the sequential kernel. */
     const void *intra;              /* host pointer to the epsr_intra_t of the intramolecular model (its ngrot) */
     const int32_t *rot_nrf, *rot_nrl;   /* [nmol] first and last group of each molecule (0-based) */
     const int32_t *rot_axis;        /* [ngroups*2] axis atoms (0-based); the rotation is about the first */
@@ -165,7 +170,7 @@ typedef struct {
     int32_t rotcycle;               /* nonzero in a cycle where nisum is a multiple of rotfreq */
     int32_t *ninter;                /* [2*nmoltype] device: internal-rotation tries then rejections */
     float *faddbs;                  /* [1] device or NULL: faddbs += sum(accepted intra changes)/nmol */
-    /* Draws ahead (fast path only): NULL, or device int32 [80 + ahead_cap].  While a cycle runs,
+    /* Draws ahead (not by the sequential kernel): NULL, or device int32 [80 + ahead_cap].  While a cycle runs,
      * a second stream walks the ran1 stream on from where the cycle's draws end and keeps the
      * values here with the states they start from and lead to; the next cycle takes them when
      * it starts from exactly that state, and walks the stream itself otherwise -- the values
