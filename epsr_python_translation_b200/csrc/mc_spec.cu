@@ -916,6 +916,9 @@ constexpr int WK_W = 5;            // moves whose outcomes the lanes enumerate
 constexpr int WK_NW = 12;          // warps (moves in flight, most of them waiting or loading)
 constexpr int WK_CH = 256;         // partners resolved at a time
 constexpr int WK_MAXN = 65536;     // molecules whose decisions fit beside the staging
+// Fewer molecules than this are left to the sequential kernel's one launch: strict cycles of 3, 6, 9 and 16 water
+// molecules take 25, 39, 58 and 94 us there, and 47 to 52 us in the walk's nine launches.
+constexpr int WK_MINN = 8;
 
 struct WalkShared {
     float2 t[WK_NW][WK_CH];        // {new, old} energy of each partner of the chunk
@@ -1544,12 +1547,13 @@ int epsr_molfit_spec(const epsr_box_t *box, const epsr_cells_t *cells, epsr_stor
     return molfit_seq_launch(box, cells, store, mc, nullptr, 0, s, S.flags, mode == 1);
 }
 
-// Whether the walk takes a cycle of this box: its decisions fit, and its atom types' pairs the energy pass's
-// shared memory (which 220 or so types use up); the store has its mirror index; and the scratch is the fast
-// path's, on the 16-byte boundary its positions need (a caller of the strict cycle may have given none, or one
-// for the sequential kernel's words).
+// Whether the walk takes a cycle of this box: it has molecules enough, their decisions fit, and its atom types'
+// pairs the energy pass's shared memory (which 220 or so types use up); the store has its mirror index; and the
+// scratch is the fast path's, on the 16-byte boundary its positions need (a caller of the strict cycle may have
+// given none, or one for the sequential kernel's words).
 bool epsr_molfit_walk_fits(const epsr_box_t *box, const epsr_store_t *store, const void *scratch, int64_t scratch_bytes) {
-    return box->nmol <= WK_MAXN && store->mirror && scratch && ((uintptr_t)scratch & 15) == 0 && box->maxat <= SP_MAXAT &&
+    return box->nmol >= WK_MINN && box->nmol <= WK_MAXN && store->mirror && scratch && ((uintptr_t)scratch & 15) == 0 &&
+           box->maxat <= SP_MAXAT &&
            (int64_t)spec_bytes(box->nmol, box->natom, store->nnbrefmax, box->nmoltype) <= scratch_bytes &&
            sizeof(float) * 2 * (size_t)store->nnbrefmax <= 160 * 1024 && spec_energy_bytes(box) <= 200 * 1024;
 }

@@ -153,8 +153,8 @@ typedef struct {
                                        with internal rotations, and strict cycles without
                                        what the parallel form needs (a mirror index that
                                        fits the rows, scratch of
-                                       epsr_molfit_spec_scratch_bytes on 16 bytes, at most
-                                       65,536 molecules and about 220 atom types) */
+                                       epsr_molfit_spec_scratch_bytes on 16 bytes, 8 to
+                                       65,536 molecules, at most about 220 atom types) */
     int32_t *status;                /* [1] device: 0 ok, 1 a molecule exceeds 64 atoms,
                                        2 the fast path's resolver timed out (cycle not applied) */
     /* Internal rotations of rotational groups before each molecule's whole-molecule move

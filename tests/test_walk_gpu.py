@@ -155,3 +155,26 @@ def test_strict_cycles_of_boxes_with_many_atom_types(ntype):
     a.cbox.ntype, a.cbox.npairref = ntype, ref.data_ptr()
     for _ in range(2):
         _same(a, b)
+
+
+@pytest.mark.parametrize("nmol,walks", [(2, 0), (7, 0), (8, 1)])
+def test_few_molecules_stay_on_the_sequential_kernel(nmol, walks):
+    """One launch against nine: below eight molecules the sequential kernel is the faster one."""
+    import ctypes as C
+    s = configs.c1_water(seed=3, nmol=nmol)
+    a, b = _box(s, False), _box(s, False)
+    b.store.mirror = None
+    ms, n = C.c_double(), C.c_int64()
+    a.lib.epsr_timing_enable(1)
+    try:
+        a.molfit(strict=True)
+        torch.cuda.synchronize()
+        a.lib.epsr_timing_read(b"spec_walk_kernel", C.byref(ms), C.byref(n))
+    finally:
+        a.lib.epsr_timing_enable(0)
+    assert n.value == walks
+    b.molfit(strict=True)
+    x, y = a.download_mc(), b.download_mc()
+    assert np.array_equal(x["den"].view(np.uint32), y["den"].view(np.uint32))
+    for _ in range(2):
+        _same(a, b)
