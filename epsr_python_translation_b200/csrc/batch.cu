@@ -31,7 +31,8 @@
 namespace epsr {
 
 constexpr int BMC_THREADS = 256;
-constexpr int BMC_MAXT = 1024;            // most threads of a CTA that works on a move
+constexpr int BMC_MAXT = 1024;            // most threads of a CTA that works on a move: features,
+constexpr int BMC_MAXD = 512;             // decisions
 constexpr int BMC_MAXAT = 64;
 constexpr int BMC_LIST = 6144;            // partner molecules scanned per move
 constexpr int FEAT_BINS = 64, FEAT_CLASSES = 10, FEAT_HALF = FEAT_BINS * FEAT_CLASSES, FEAT_IN = 2 * FEAT_HALF;
@@ -1106,10 +1107,13 @@ epsr_bmc_t plain_bmc(const epsr_bmc_t *b) {
 
 // Threads of a moved molecule's CTA.  A step is one wave whose time is its slowest move's, and the
 // kernels' registers let 1,024 threads share an SM: the caller's count, doubled while every move's
-// CTA is still resident, so a few moves run wide and many narrow.
-int move_threads(const epsr_bmc_t *b) {
+// CTA is still resident, so a few moves run wide and many narrow.  A decision's items don't fill 1,024 threads,
+// whose barriers then cost more than they bring (plain sweeps of 48 boxes of 300 atoms 5.74 ms, at 512 threads 4.83;
+// of 16 boxes of 1,200 24.5 and 22.2; of one of 30,000 4.38 and 4.22), and the features' searches reach further
+// (learned sweeps of four boxes of 1,500 molecules 12.6 ms, at 512 threads 13.3).
+int move_threads(const epsr_bmc_t *b, int most) {
     int t = b->threads;
-    while (t < BMC_MAXT && 2ll * t * b->nslot <= 148ll * 1024) t *= 2;
+    while (t < most && 2ll * t * b->nslot <= 148ll * 1024) t *= 2;
     return t;
 }
 template <bool ODD>
@@ -1121,9 +1125,9 @@ int launch_features(const epsr_bmc_t *b, int t, int step, void *x, cudaStream_t 
 }
 template <int T>
 int launch_decide(const epsr_bmc_t *b, int t, int step, int mode, const float *y, float *target, cudaStream_t s) {
-    // an SM's shared memory over the CTAs of T threads that its registers hold: what the search
-    // leaves holds tables
-    const int bytes = (220 * 1024) / (1024 / T), table = bytes - (int)(T > BMC_THREADS ? sizeof(WideSearch) : sizeof(NarrowSearch)) - 4096;
+    // an SM's shared memory over the CTAs that share it, one each where there are SMs for all, else as many of T
+    // threads as its registers hold: what the search leaves holds tables
+    const int bytes = (220 * 1024) / (b->nslot <= 148 ? 1 : 1024 / T), table = bytes - (int)(T > BMC_THREADS ? sizeof(WideSearch) : sizeof(NarrowSearch)) - 4096;
     EPSR_SMEM_OPTIN(bmc_decide_kernel<T>);
     EPSR_TIMED("bmc_decide_kernel", s, bmc_decide_kernel<T><<<b->nslot, t, bytes - 4096, s>>>(*b, step, mode, y, target, table));
     return EPSR_OK;
@@ -1163,7 +1167,7 @@ extern "C" int epsr_bmc_propose(const epsr_bmc_t *b, int32_t step, void *x, void
     if (!x) {   // proposals alone: one warp a slot
         EPSR_TIMED("bmc_propose_kernel", s, bmc_propose_kernel<false><<<b->nslot, 32, 0, s>>>(B, step, nullptr));
     } else {
-        const int t = move_threads(&B);
+        const int t = move_threads(&B, BMC_MAXT);
         rc = ((uintptr_t)x & 3) ? launch_features<true>(&B, t, step, x, s) : launch_features<false>(&B, t, step, x, s);
         if (rc) return rc;
     }
@@ -1181,10 +1185,9 @@ extern "C" int epsr_bmc_decide(const epsr_bmc_t *b, int32_t step, int32_t mode, 
     }
     cudaStream_t s = (cudaStream_t)stream;
     const epsr_bmc_t B = plain_bmc(b);
-    const int t = move_threads(&B);
+    const int t = move_threads(&B, BMC_MAXD);
     rc = t <= BMC_THREADS ? launch_decide<BMC_THREADS>(&B, t, step, mode, y, target, s)
-         : t == 512       ? launch_decide<512>(&B, t, step, mode, y, target, s)
-                          : launch_decide<BMC_MAXT>(&B, t, step, mode, y, target, s);
+                          : launch_decide<BMC_MAXD>(&B, t, step, mode, y, target, s);
     if (rc) return rc;
     EPSR_CUDA(cudaGetLastError());
     return EPSR_OK;
