@@ -134,7 +134,11 @@ __global__ void ag_intra_kernel(AgDev A, const int32_t *itype, unsigned long lon
             float zz = __fmul_rn(__fsub_rn(A.za[ia], A.za[ja]), A.sizefactor);
             const float d = dist_f(A.L, xx, yy, zz);
             const int iz1 = nint_i(__fdiv_rn(d, A.stepcl)) + 2;
-            if (iz1 > 1 && iz1 <= A.npt1) add_count(counts + (size_t)icref * A.ldw + iz1);
+            if (iz1 > 1 && iz1 <= A.npt1) {
+                unsigned long long *c = counts + (size_t)icref * A.ldw + iz1;
+                if (A.L.cubic) add_count(c);
+                else atomicAdd(c, 1ull);
+            }
             ++np;
         }
     }
@@ -189,7 +193,7 @@ __global__ void __launch_bounds__(1024) ag_inter_kernel(AgDev A, const int2 *oat
     H.ntype = A.ntype;
     H.nlim = max(A.npt1 - 1, 0);
     H.stepcl = A.stepcl;
-    H.rcp = CUBIC ? hist_rcp(A.stepcl) : nanf("");
+    H.rcp = hist_rcp(A.stepcl);
     H.dmax = A.dmax;
     H.rmax = hist_rmax(A.rminex, A.npairs);
     H.L = A.L;
@@ -374,8 +378,7 @@ extern "C" int epsr_atogen(const epsr_box_t *box, int32_t npt1, float sizefactor
 
     const size_t nbins = (size_t)box->npairs * ldw;
     EPSR_CUDA(cudaMemsetAsync(counts, 0, sizeof(unsigned long long) * (2 * nbins + box->npairs), s));
-    EPSR_CUDA(cudaMemsetAsync(pairc, 0, sizeof(long long) * 2, s));
-    EPSR_CUDA(cudaMemsetAsync(csampled, 0, sizeof(int32_t) * (box->ntype + 1), s));
+    EPSR_CUDA(cudaMemsetAsync(csampled, 0, (size_t)((char *)(pairc + 2) - (char *)csampled), s));   // to pairc's end
     int rc = epsr_box_positions(box, stream);
     if (rc) return rc;
     const int ncand = im2 - im1 + 1;
@@ -403,7 +406,10 @@ extern "C" int epsr_atogen(const epsr_box_t *box, int32_t npt1, float sizefactor
     }
     if (noatoms > 0) {
         const int threads = hist_threads(shm);
-        const dim3 grid(ag_splits(ychunks, (natom + tile - 1) / tile, tile, nbins, 148 * (1024 / threads)), ychunks);
+        // in a cell that is not cubic a target costs so much more than a bin that every tile has a CTA of its own
+        // (5,000 water: 629 us, and 712 us by ag_splits)
+        const int ntiles = (natom + tile - 1) / tile;
+        const dim3 grid(box->cubic ? ag_splits(ychunks, ntiles, tile, nbins, 148 * (1024 / threads)) : ntiles, ychunks);
         if (box->cubic) {
             if (shm > 48 * 1024) EPSR_SMEM_OPTIN(ag_inter_kernel<true>);
             EPSR_TIMED("ag_inter_kernel", s, ag_inter_kernel<true><<<grid, threads, shm, s>>>(A, oatoms, misc + 1, molof, tile, counts, counts + 2 * nbins));

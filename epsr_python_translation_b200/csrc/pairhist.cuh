@@ -91,7 +91,7 @@ __device__ __forceinline__ void hist_stage_tile(const PairHist &H, const float4 
 }
 
 // SOME: the group may hold targets that don't count
-template <int U, bool CUBIC, bool STAGED, bool SOME>
+template <int U, bool STAGED, bool SOME>
 __device__ __forceinline__ void hist_group(const PairHist &H, float4 p1, int im, bool after, const float4 *tp,
                                            const int *tm, const int *cls, int &uses) {
     float d[U];
@@ -109,11 +109,7 @@ __device__ __forceinline__ void hist_group(const PairHist &H, float4 p1, int im,
         }
         base[u] = STAGED ? *(const int *)((const char *)cls + ty) : __ldg(cls + ty) * H.ld;
         // xx = x1 - x2 (ato_manipulation_rev4.py:3798); the square does not see the sign
-        if (CUBIC) {
-            d[u] = sqrt_unit(dsq_cubic(p2, p1));
-        } else {
-            d[u] = dist_f(H.L, __fsub_rn(p1.x, p2.x), __fsub_rn(p1.y, p2.y), __fsub_rn(p1.z, p2.z));
-        }
+        d[u] = sqrt_unit(dsq_cubic(p2, p1));
         n[u] = nint_index(d[u], H.rcp, odd[u]);
         any |= odd[u];
     }
@@ -133,13 +129,41 @@ __device__ __forceinline__ void hist_group(const PairHist &H, float4 p1, int im,
     }
 }
 
-template <bool CUBIC, bool STAGED, bool SOME>
+template <bool STAGED, bool SOME>
 __device__ __forceinline__ int hist_part(const PairHist &H, float4 p1, int im, bool after, const float4 *tp,
                                          const int *tm, int q0, int q1, const int *cls) {
     int uses = 0, q = q0;
-    for (; q + 4 <= q1; q += 4) hist_group<4, CUBIC, STAGED, SOME>(H, p1, im, after, tp + q, tm + q, cls, uses);
-    for (; q < q1; ++q) hist_group<1, CUBIC, STAGED, SOME>(H, p1, im, after, tp + q, tm + q, cls, uses);
+    for (; q + 4 <= q1; q += 4) hist_group<4, STAGED, SOME>(H, p1, im, after, tp + q, tm + q, cls, uses);
+    for (; q < q1; ++q) hist_group<1, STAGED, SOME>(H, p1, im, after, tp + q, tm + q, cls, uses);
     return SOME ? uses : max(q1 - q0, 0);
+}
+
+// Cells that are not cubic: one target at a time, by the general distance and the division, and none for a target
+// that does not count.  There the latency of three divisions and a root a pair bounds a thread, so that groups of four,
+// a second loop for the lanes whose tile counts whole, and distances to targets that don't count all cost time (the
+// cubic form with the general distance: sheared boxes of 200 DMSO + 400 water and 5,000 water, whole passes of 298
+// and 741 us; 227 and 517 so, with a CTA for every tile).
+template <bool STAGED>
+__device__ __forceinline__ int hist_any_cell(const PairHist &H, float4 p1, int im, bool after, const float4 *tp,
+                                             const int *tm, int q0, int q1, const int *cls) {
+    int uses = 0;
+    for (int q = q0; q < q1; ++q) {
+        const int jm = tm[q];
+        if (after ? jm <= im : jm == im) continue;
+        ++uses;
+        const float4 p2 = tp[q];
+        const int ty = __float_as_int(p2.w);
+        const int base = STAGED ? *(const int *)((const char *)cls + ty) : __ldg(cls + ty) * H.ld;
+        const float d = dist_f(H.L, __fsub_rn(p1.x, p2.x), __fsub_rn(p1.y, p2.y), __fsub_rn(p1.z, p2.z));
+        const int n = nint_i(__fdiv_rn(d, H.stepcl));
+        if ((unsigned)n < (unsigned)H.nlim) atomicAdd(H.hist + base + 2 + n, 1u);
+        const float dd = __fmul_rn(d, H.dmax);
+        if (dd < H.rmax) {
+            const int icref = base / H.ld;
+            if (dd < fabsf(__ldg(H.rminex + icref))) atomicAdd(H.hpot + icref, 1u);
+        }
+    }
+    return uses;
 }
 
 // Targets q0..q1-1 of a tile (its first and last molecule in `mols`) against origin p1 of molecule im:
@@ -150,9 +174,10 @@ __device__ __forceinline__ int hist_tile(const PairHist &H, float4 p1, int im, b
                                          const int *tm, int q0, int q1, const int *mols, const int *cls_sm) {
     const int it = __float_as_int(p1.w);
     const int *cls = STAGED ? cls_sm + it : H.npairref + it * H.ntype;
+    if (!CUBIC) return hist_any_cell<STAGED>(H, p1, im, after, tp, tm, q0, q1, cls);
     if (mols[0] > im || (!after && mols[1] < im))
-        return hist_part<CUBIC, STAGED, false>(H, p1, im, after, tp, tm, q0, q1, cls);
-    return hist_part<CUBIC, STAGED, true>(H, p1, im, after, tp, tm, q0, q1, cls);
+        return hist_part<STAGED, false>(H, p1, im, after, tp, tm, q0, q1, cls);
+    return hist_part<STAGED, true>(H, p1, im, after, tp, tm, q0, q1, cls);
 }
 
 // Threads of a CTA with `shm` bytes of shared memory: 64 registers a thread let 1,024 share an SM.

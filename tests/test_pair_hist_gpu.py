@@ -161,3 +161,34 @@ def test_stog_sums_match_sequential(nr, nq, npairs):
             ref = xwt[ic] + np.where(r > 0, v / r, v)
             tol = 2.0 ** -21 * (np.abs(xwt[ic]) + sfac * mag / np.where(r > 0, r, 1))
         assert np.all(np.abs(out[ic, 1:] - ref[1:]) <= tol[1:])
+
+
+def _sheared(box):
+    box.cubic = False
+    box.lat6 = np.array([1.0, 0.2, -0.1, 0.9, 0.15, 0.95], f32)
+    return box
+
+
+SHEARED = {"one": lambda: _grid_box(1), "halves_43": lambda: _grid_box(43), "halves_86": lambda: _grid_box(86),
+           "water_1201": lambda: _grid_box(1201, spread=False), "types_16": lambda: _many_types(60, 16),
+           "types_17": lambda: _many_types(60, 17), "mixture": lambda: BoxArrays.from_system(configs.c2_mixture(seed=5, ndmso=60, nwater=90))}
+
+
+@pytest.mark.parametrize("ngr", [0, 7])
+@pytest.mark.parametrize("name", list(SHEARED))
+def test_sheared_cells_match_oracle(name, ngr):
+    """The general cell's own loop: one and several origin chunks and tiles, origins all or sampled, few and many types."""
+    from epsr_python_translation_b200.device import DeviceBox
+    box = _sheared(SHEARED[name]())
+    d = DeviceBox(box)
+    st = Ran1State(idum=-8)
+    rmx = np.full(box.npairs, f32(-2.0), f32)
+    rmx[::2] = f32(3.5)
+    t = d.ran1_tensor(st)
+    got = d.atogen(ngr, t, rmx)
+    wav, potex, ref, after = oracle.atogen(box, ngr, st, rmx)
+    assert got == ref
+    mine, mp = d.download_wav()
+    assert_bits_equal(mine[:, :, 1:box.npt1 + 1], wav[:, :, 1:box.npt1 + 1], "wav")
+    assert_bits_equal(mp, potex, "potex")
+    assert np.array_equal(t.cpu().numpy(), after.as_array())
