@@ -31,8 +31,8 @@
 namespace epsr {
 
 constexpr int BMC_THREADS = 256;
-constexpr int BMC_MAXT = 1024;            // most threads of a CTA that works on a move: features,
-constexpr int BMC_MAXD = 512;             // decisions
+constexpr int BMC_MAXT = 1024;            // most threads of a CTA that works on a move
+constexpr int BMC_MAXD = 512;             // and of one that decides on a molecule of a few atoms
 constexpr int BMC_MAXAT = 64;
 constexpr int BMC_LIST = 6144;            // partner molecules scanned per move
 constexpr int FEAT_BINS = 64, FEAT_CLASSES = 10, FEAT_HALF = FEAT_BINS * FEAT_CLASSES, FEAT_IN = 2 * FEAT_HALF;
@@ -1107,10 +1107,7 @@ epsr_bmc_t plain_bmc(const epsr_bmc_t *b) {
 
 // Threads of a moved molecule's CTA.  A step is one wave whose time is its slowest move's, and the
 // kernels' registers let 1,024 threads share an SM: the caller's count, doubled while every move's
-// CTA is still resident, so a few moves run wide and many narrow.  A decision's items don't fill 1,024 threads,
-// whose barriers then cost more than they bring (plain sweeps of 48 boxes of 300 atoms 5.74 ms, at 512 threads 4.83;
-// of 16 boxes of 1,200 24.5 and 22.2; of one of 30,000 4.38 and 4.22), and the features' searches reach further
-// (learned sweeps of four boxes of 1,500 molecules 12.6 ms, at 512 threads 13.3).
+// CTA is still resident, so a few moves run wide and many narrow.
 int move_threads(const epsr_bmc_t *b, int most) {
     int t = b->threads;
     while (t < most && 2ll * t * b->nslot <= 148ll * 1024) t *= 2;
@@ -1185,9 +1182,15 @@ extern "C" int epsr_bmc_decide(const epsr_bmc_t *b, int32_t step, int32_t mode, 
     }
     cudaStream_t s = (cudaStream_t)stream;
     const epsr_bmc_t B = plain_bmc(b);
-    const int t = move_threads(&B, BMC_MAXD);
+    // The decisions of molecules of a few atoms don't fill 1,024 threads, whose barriers then cost more than they
+    // bring: plain sweeps of 48 boxes of 300 atoms of water and silica take 5.74 ms so, and 4.83 at 512 threads, of 16
+    // of 1,200 24.5 and 22.2, of one of 30,000 4.38 and 4.22; of four of 2,700 DMSO + 5,300 water (5.4 atoms a
+    // molecule) 11.05 and 11.15.  The features' searches reach further: learned sweeps of four boxes of 500 DMSO +
+    // 1,000 water take 12.6 ms, and 13.3 with features by 512 threads.
+    const int t = move_threads(&B, B.natom > 4ll * B.nmol ? BMC_MAXT : BMC_MAXD);
     rc = t <= BMC_THREADS ? launch_decide<BMC_THREADS>(&B, t, step, mode, y, target, s)
-                          : launch_decide<BMC_MAXD>(&B, t, step, mode, y, target, s);
+         : t <= BMC_MAXD  ? launch_decide<BMC_MAXD>(&B, t, step, mode, y, target, s)
+                          : launch_decide<BMC_MAXT>(&B, t, step, mode, y, target, s);
     if (rc) return rc;
     EPSR_CUDA(cudaGetLastError());
     return EPSR_OK;
